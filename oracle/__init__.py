@@ -346,5 +346,9 @@ def lm_steps(J, r, b, sig, damping):
     out = []
     for d0, d1 in _f64(damping).reshape(-1, 2):
         A = JJ + d0 * np.diag(np.diag(JJ)) + d1 * np.diag(1.0 / _f64(sig) ** 2)
-        out.append(_f64(b) + np.linalg.inv(A) @ g)
+        try:
+            inv = np.linalg.inv(A)
+        except np.linalg.LinAlgError:  # the reference's inv returns zeros (zmath.cpp:134)
+            inv = np.zeros_like(A)
+        out.append(_f64(b) + inv @ g)
     return np.array(out), JJ

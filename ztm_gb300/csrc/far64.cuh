@@ -1,0 +1,324 @@
+// far64.cuh - the prism far field at double accuracy on the FP32 pipe.
+//
+// GB300 issues FP64 at 1/64 of FP32, so the plain double mesh kernels spent
+// about 180 FP64 issue slots (90 clocks of an SM) on every corner function.
+// Beyond FAR64_Q half-diagonals the corner form is not even the accurate one:
+// its eight terms cancel like (R/a)^3.  There the moment expansion of
+// prism_common.cuh, taken to twelfth order and evaluated in pairs of floats
+// (value = hi + lo, 48 bits, every product and sum error-free to its low part),
+// is closer to the exact field than the corner form in double: truncation
+// 2e-15 of V/r^2 at 8 half-diagonals, rounding about 2e-14 a pair with random
+// sign, and nothing cancels.  A pair costs about 70 FP32 operations.
+//
+//   gz = G rho V Z/r^3 (1 + T),  T = u (C1 + u (C2 + ... + u C12)),  u = 1/r^2,
+//   C_k = sum over orders n of c[n][k-n](X^2, Y^2),
+// c[n][j] homogeneous of degree j, Z^2 eliminated by r^2 - X^2 - Y^2.
+//
+// Three forms by horizontal distance (half-diagonals), voted per warp:
+//   below 20    orders 2..12 (n <= 6), C1..C4's second- and fourth-order parts
+//               in float pairs (the fourth-order term is 4e-4 there)
+//   20 .. 128   orders 2..8, C1 and C2 in float pairs
+//   above 128   orders 2..6, T (below 1e-4) in float but for C1's low part
+// (order 12 reaches 2e-15 at 8, order 8 3e-15 at 20, order 6 1e-18 at 128).
+#pragma once
+#include <cuda_runtime.h>
+
+#include "prism_common.cuh"
+#include "ztm_internal.cuh"
+
+constexpr double FAR64_Q = 8.0;      // closed form in double nearer than this
+constexpr double FAR64_Q_B = 20.0;   // the middle form from here on
+constexpr double FAR64_Q_C = 128.0;  // the far form from here on
+
+// Coefficients c[n][j][i] of x^i y^(j-i) u^(n+j), x = X^2, y = Y^2 (lengths in
+// units of the largest cell edge): n = 1..6, packed by far64_at.
+constexpr int FAR64_N = 6;
+__host__ __device__ constexpr int far64_at(int n, int j, int i) {
+  // offset of order n: sum over m < n of (m+1)(m+2)/2
+  int o = 0;
+  for (int m = 1; m < n; m++) o += (m + 1) * (m + 2) / 2;
+  return o + j * (j + 1) / 2 + i;
+}
+constexpr int FAR64_COEFS = 83;
+
+struct Far64Coef {
+  float c[FAR64_COEFS];     // float values
+  float lo[9];              // low parts of the orders n = 1, 2 (far64_at < 9)
+  float dxh, dxl, dyh, dyl, dzh, dzl;  // cell edges / L0
+  float rh_b, rh_c;         // squared horizontal distances of the forms
+};
+
+// The coefficients of a cell of edges dx, dy, dz (units of L0), in double.
+void far64_coefs(double dx, double dy, double dz, double* c);
+Far64Coef far64_make(const MeshDesc& m, double L0);
+
+// What both double mesh kernels prepare (prism64.cu).
+struct Far64Mesh {
+  MeshConst k;    // near radius FAR64_Q
+  Far64Coef fc;
+};
+
+#ifdef __CUDACC__
+namespace far64 {
+
+// ---- packed operations (two lanes) -----------------------------------------
+__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+// a - b in one operation (b times -1 is exact)
+__device__ __forceinline__ float2 sub(float2 a, float2 b) {
+  return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+}
+// sign flip on the integer pipe, beside the FMA pipe's work
+__device__ __forceinline__ float2 neg(float2 a) {
+  return make_float2(__int_as_float(__float_as_int(a.x) ^ 0x80000000),
+                     __int_as_float(__float_as_int(a.y) ^ 0x80000000));
+}
+// error of s = a + b, any order (Knuth)
+__device__ __forceinline__ float2 sum_err(float2 a, float2 b, float2 s) {
+  const float2 bb = sub(s, a);
+  return add(sub(a, sub(s, bb)), sub(b, bb));
+}
+// a pair of floats (hi, lo)
+struct D2 {
+  float2 h, l;
+};
+// hi + lo renormalised
+__device__ __forceinline__ D2 quick(float2 h, float2 l) {
+  D2 r;
+  r.h = add(h, l);
+  r.l = sub(l, sub(r.h, h));
+  return r;
+}
+__device__ __forceinline__ D2 dd_mul(D2 a, D2 b) {
+  D2 r;
+  r.h = mul(a.h, b.h);
+  r.l = fma(a.h, b.h, neg(r.h));
+  r.l = fma(a.h, b.l, r.l);
+  r.l = fma(a.l, b.h, r.l);
+  return r;
+}
+__device__ __forceinline__ D2 dd_sq(D2 a) {
+  D2 r;
+  r.h = mul(a.h, a.h);
+  r.l = fma(a.h, a.h, neg(r.h));
+  r.l = fma(a.l, add(add(a.h, a.h), a.l), r.l);
+  return r;
+}
+__device__ __forceinline__ D2 dd_add(D2 a, D2 b) {
+  D2 r;
+  r.h = add(a.h, b.h);
+  r.l = add(sum_err(a.h, b.h, r.h), add(a.l, b.l));
+  return r;
+}
+__device__ __forceinline__ D2 dd_dup(float h, float l) { return D2{dup(h), dup(l)}; }
+
+// n d + e for an integer n (exact in float below 2^24) and pairs d, e with
+// |e| <= |d| / 2 unless n is huge: renormalised pair
+__device__ __forceinline__ D2 offset(float2 n, float dh, float dl, float2 eh, float2 el) {
+  const float2 p = mul(n, dup(dh));
+  const float2 pe = fma(n, dup(dl), fma(n, dup(dh), neg(p)));
+  const float2 s = add(p, eh);
+  return quick(s, add(sum_err(p, eh, s), add(pe, el)));
+}
+
+// Z and Z^2 of one station at layer n (n = l - home layer) as pairs, scalar:
+// |e| <= d / 2, so n d + e needs no ordering test (n = 0 adds to zero).
+__device__ __forceinline__ void layer_z(float n, const Far64Coef& f, float eh, float el, float* zh,
+                                        float* zl, float* qh, float* ql) {
+  const float p = __fmul_rn(n, f.dzh);  // (no contraction with the sum below)
+  const float pe = fmaf(n, f.dzl, fmaf(n, f.dzh, -p));
+  const float s = __fadd_rn(p, eh);
+  const float l = (eh - (s - p)) + (pe + el);
+  const float q = __fmul_rn(s, s);
+  *zh = s;
+  *zl = l;
+  *qh = q;
+  *ql = fmaf(l, (s + s) + l, fmaf(s, s, -q));
+}
+
+// ---- one lane pair's column state ------------------------------------------
+struct Col {
+  D2 R;        // X^2 + Y^2
+  D2 C2, C3, C4;  // C3.l, C4.l used by form 0 only
+  float2 c[8];    // C5 .. C12 (form 0), C5 .. C8 (form 1), C5, C6 (form 2)
+};
+
+template <int FORM>
+__device__ __forceinline__ float2 coef_sum(const Far64Coef& f, int kk, const float2* xp,
+                                           const float2* yp) {
+  // sum over n of c[n][kk-n], n from (skip parts kept in pairs) to the form's order
+  constexpr int NM = FORM == 0 ? 6 : FORM == 1 ? 4 : 3;
+  float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int n = 1; n <= NM; n++) {
+    const int j = kk - n;
+    if (j < 0 || j > n) continue;
+    if (n == 1 || (n == 2 && (FORM == 0 || kk == 2))) continue;  // in pairs
+#pragma unroll
+    for (int i = 0; i <= j; i++) {
+      const float2 mono = i == 0 ? yp[j] : i == j ? xp[j] : mul(xp[i], yp[j - i]);
+      s = fma(dup(f.c[far64_at(n, j, i)]), mono, s);
+    }
+  }
+  return s;
+}
+
+// Column state from the horizontal offsets X, Y (units of L0).
+template <int FORM>
+__device__ __forceinline__ Col make_col(const Far64Coef& f, D2 X, D2 Y) {
+  Col o;
+  const D2 x = dd_sq(X), y = dd_sq(Y);
+  {
+    const D2 r = dd_add(x, y);
+    o.R = quick(r.h, r.l);
+  }
+  constexpr int DEG = FORM == 0 ? 6 : FORM == 1 ? 4 : 3;
+  float2 xp[DEG + 1], yp[DEG + 1];
+  xp[0] = yp[0] = make_float2(1.f, 1.f);
+#pragma unroll
+  for (int i = 1; i <= DEG; i++) {
+    xp[i] = mul(xp[i - 1], x.h);
+    yp[i] = mul(yp[i - 1], y.h);
+  }
+  auto C = [&](int at) { return dd_dup(f.c[at], f.lo[at]); };
+  // order 2 (n = 1) and the constant of order 4 (n = 2) in pairs
+  D2 c2 = dd_add(dd_mul(C(far64_at(1, 1, 1)), x), dd_mul(C(far64_at(1, 1, 0)), y));
+  c2 = dd_add(c2, C(far64_at(2, 0, 0)));
+  o.C2 = quick(c2.h, c2.l);
+  if (FORM == 0) {
+    const D2 c3 = dd_add(dd_mul(C(far64_at(2, 1, 1)), x), dd_mul(C(far64_at(2, 1, 0)), y));
+    o.C3 = quick(c3.h, add(c3.l, coef_sum<FORM>(f, 3, xp, yp)));
+    const D2 xx = dd_sq(x), xy = dd_mul(x, y), yy = dd_sq(y);
+    D2 c4 = dd_add(dd_mul(C(far64_at(2, 2, 2)), xx), dd_mul(C(far64_at(2, 2, 1)), xy));
+    c4 = dd_add(c4, dd_mul(C(far64_at(2, 2, 0)), yy));
+    // the higher orders' part of C4 may exceed c4's: an exact sum
+    const float2 h4 = coef_sum<FORM>(f, 4, xp, yp);
+    const float2 s4 = add(c4.h, h4);
+    o.C4 = quick(s4, add(c4.l, sum_err(c4.h, h4, s4)));
+  } else {
+    o.C3 = D2{coef_sum<FORM>(f, 3, xp, yp), make_float2(0.f, 0.f)};
+    o.C4 = D2{coef_sum<FORM>(f, 4, xp, yp), make_float2(0.f, 0.f)};
+  }
+#pragma unroll
+  for (int kk = 5; kk <= (FORM == 0 ? 12 : FORM == 1 ? 8 : 6); kk++)
+    o.c[kk - 5] = coef_sum<FORM>(f, kk, xp, yp);
+  if (FORM != 0) {
+    // a lane far beyond the form's range (its warp's nearest lane decides):
+    // the powers of X^2 + Y^2 would overflow, and orders above 4 vanish there
+    const bool fx = o.R.h.x > 1.0e8f, fy = o.R.h.y > 1.0e8f;
+#pragma unroll
+    for (int q = 0; q < (FORM == 1 ? 4 : 2); q++) {
+      if (fx) o.c[q].x = 0.f;
+      if (fy) o.c[q].y = 0.f;
+    }
+  } else {
+    const bool fx = o.R.h.x > 1.0e5f, fy = o.R.h.y > 1.0e5f;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      if (fx) o.c[q].x = 0.f;
+      if (fy) o.c[q].y = 0.f;
+    }
+  }
+  return o;
+}
+
+// s u + c for pairs (one Horner step)
+__device__ __forceinline__ D2 horner(D2 s, float2 uh, float2 ul, D2 c) {
+  const float2 p = mul(s.h, uh);
+  float2 pe = fma(s.h, uh, neg(p));
+  pe = fma(s.h, ul, pe);
+  pe = fma(s.l, uh, pe);
+  D2 r;
+  r.h = add(p, c.h);
+  r.l = add(sum_err(p, c.h, r.h), add(pe, c.l));
+  return r;
+}
+
+// Z/r^3 (1 + T) for the two lanes: pair (v, ve).  Z, Z^2 as pairs.
+template <int FORM>
+__device__ __forceinline__ D2 value(const Far64Coef& f, const Col& o, D2 Z, D2 Q) {
+  // r^2 = R + Q, both >= 0: the larger operand by min / max on the integer pipe
+  const float2 hi = make_float2(fmaxf(o.R.h.x, Q.h.x), fmaxf(o.R.h.y, Q.h.y));
+  const float2 lo = make_float2(fminf(o.R.h.x, Q.h.x), fminf(o.R.h.y, Q.h.y));
+  const float2 s = add(o.R.h, Q.h);
+  const float2 sl = add(sub(lo, sub(s, hi)), add(o.R.l, Q.l));
+  const float2 y = make_float2(rsqrt_ftz(s.x), rsqrt_ftz(s.y));
+  const float2 p = mul(y, y), np = neg(p);
+  const float2 npe = fma(neg(y), y, p);  // p - y^2
+  // g = 1 - r^2 y^2 (about 1e-7), r^-3 = y^3 (1 + 1.5 g + 1.875 g^2)
+  float2 g = fma(s, np, make_float2(1.f, 1.f));
+  g = fma(sl, np, g);
+  g = fma(s, npe, g);
+  const float2 c = mul(g, fma(dup(1.875f), g, dup(1.5f)));
+  const float2 pe = neg(npe);
+  const float2 a = mul(Z.h, y);
+  float2 ae = fma(Z.h, y, neg(a));
+  ae = fma(Z.l, y, ae);
+  D2 v;
+  v.h = mul(a, p);
+  v.l = fma(a, p, neg(v.h));
+  v.l = fma(ae, p, v.l);
+  v.l = fma(a, pe, v.l);
+  v.l = fma(v.h, c, v.l);
+  const float c1h = f.c[0], c1l = f.lo[0];
+  if (FORM == 2) {
+    float2 t = fma(o.c[1], p, o.c[0]);
+    t = fma(t, p, o.C4.h);
+    t = fma(t, p, o.C3.h);
+    t = fma(t, p, o.C2.h);
+    t = add(fma(t, p, dup(c1l)), dup(c1h));
+    t = mul(t, p);
+    v.l = fma(v.h, t, fma(v.l, t, v.l));
+    return v;
+  }
+  const float2 ul = fma(p, g, pe);  // 1/r^2 = p + ul
+  D2 t;
+  if (FORM == 0) {
+    float2 w = fma(o.c[7], p, o.c[6]);
+#pragma unroll
+    for (int q = 5; q >= 0; q--) w = fma(w, p, o.c[q]);
+    t = horner(D2{w, make_float2(0.f, 0.f)}, p, ul, o.C4);
+    t = horner(t, p, ul, o.C3);
+    t = horner(t, p, ul, o.C2);
+  } else {
+    float2 w = fma(o.c[3], p, o.c[2]);
+    w = fma(w, p, o.c[1]);
+    w = fma(w, p, o.c[0]);
+    w = fma(w, p, o.C4.h);
+    w = fma(w, p, o.C3.h);
+    t.h = o.C2.h;
+    t.l = fma(w, p, o.C2.l);
+  }
+  t = horner(t, p, ul, dd_dup(c1h, c1l));
+  // T = t u, then v (1 + T)
+  const float2 Th = mul(t.h, p);
+  float2 te = fma(t.h, p, neg(Th));
+  te = fma(t.h, ul, te);
+  te = fma(t.l, p, te);
+  const float2 vt = mul(v.h, Th);
+  float2 vte = fma(v.h, Th, neg(vt));
+  vte = fma(v.h, te, vte);
+  vte = fma(v.l, Th, vte);
+  D2 r;
+  r.h = add(v.h, vt);
+  r.l = add(sub(vt, sub(r.h, v.h)), add(v.l, vte));
+  return r;
+}
+
+// acc += w x (w, x pairs), to the accumulator's low part
+__device__ __forceinline__ void mac(D2& acc, float2 wh, float2 wl, D2 x, bool mx, bool my) {
+  float2 m = mul(wh, x.h);
+  float2 me = fma(wh, x.h, neg(m));
+  me = fma(wl, x.h, me);
+  me = fma(wh, x.l, me);
+  if (mx) m.x = me.x = 0.f;  // select: also drops a NaN
+  if (my) m.y = me.y = 0.f;
+  const float2 s = add(acc.h, m);
+  acc.l = add(acc.l, add(sum_err(acc.h, m, s), me));
+  acc.h = s;
+}
+
+}  // namespace far64
+#endif

@@ -39,7 +39,6 @@ namespace {
 
 constexpr int FAR_TS = 128;   // stations per block in the far kernel
 constexpr int F64_TS = 64;    // stations per block in the plain double kernel
-constexpr int FAR_NEAR_ST = 32;  // stations per near item of the far kernel's queue
 
 // ---------------------------------------------------------------------------
 __global__ void station_prep_kernel(MeshDesc m, double L0, int ns,
@@ -156,13 +155,15 @@ struct FarArgs {
   int chunk_cols;     // columns per item
   int sc;             // columns per shared-memory stage
   int* counter;       // next work item (zeroed before the launch)
-  int n_near;         // near items (FAR_NEAR_ST stations each), spread through the queue
+  int n_near;         // near items, spread through the queue
+  int near_units;     // (station, part) units per near item, a warp each
+  int nparts;         // parts of a station's near vertices (near_parts)
   bool near_f64;      // near region in double (mixed) or float (FP32 method)
   MeshDesc m;
   const double* sxyz;
   const double* rho;  // caller's double density (near region)
   const int2* lr;     // per-station near layer range
-  double* near;       // [ns] near-region sums
+  double* near;       // [nparts][ns] near-region sums
   const float4* sf;
   const int4* si;
   const short2* iv;  // near-region intervals [station][box column]
@@ -190,8 +191,8 @@ __device__ __forceinline__ float far_pair(float rho, float Z, float rh, float a0
 
 // Persistent kernel of the mixed forward.  The work is tiles x chunks far
 // items (a tile of FAR_TS stations against a chunk of chunk_cols columns) and
-// n_near near items (the double near regions of FAR_NEAR_ST stations, one
-// warp per station), spread evenly through one queue so that while some
+// n_near near items (the double near regions of near_units units, one warp per
+// station or part of one), spread evenly through one queue so that while some
 // blocks of an SM sum near regions on the FP64 pipe the others sum far
 // fields on the FMA pipe.  The grid is the number of blocks resident at once;
 // each block takes items from a counter until none are left.  Each far item
@@ -273,16 +274,17 @@ __global__ void __launch_bounds__(FAR_TS, 6) far_kernel(FarArgs a) {
         if (threadIdx.x == 0) issue(far_index(nxt), 0, seq);
         issued = seq + 1;
       }
-      const int s0 = near_before(item) * FAR_NEAR_ST;
-      for (int j = warp; j < FAR_NEAR_ST; j += FAR_TS / 32) {
-        const int s = s0 + j;
+      const int u0 = near_before(item) * a.near_units;
+      for (int j = warp; j < a.near_units; j += FAR_TS / 32) {
+        const int s = (u0 + j) / a.nparts, part = (u0 + j) % a.nparts;
         if (s >= a.ns) break;
+        double* out = a.near + (size_t)part * a.ns;
         if (a.near_f64)
-          near_station<double>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho, a.near, lane,
-                               COUNT ? &nphi : nullptr);
+          near_station<double>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho, out, lane,
+                               COUNT ? &nphi : nullptr, part, a.nparts);
         else
-          near_station<float>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho, a.near, lane,
-                              COUNT ? &nphi : nullptr);
+          near_station<float>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho, out, lane,
+                              COUNT ? &nphi : nullptr, part, a.nparts);
       }
       if (threadIdx.x == 0) s_item[par] = nxt < n_items ? atomicAdd(a.counter, 1) : n_items;
       __syncthreads();
@@ -382,16 +384,20 @@ __global__ void __launch_bounds__(FAR_TS, 6) far_kernel(FarArgs a) {
   }
 }
 
-// gz[s] = G5 * (far_scale * sum_c partial[c][s] + near[s])
+// gz[s] = G5 * (far_scale * sum_c partial[c][s] + sum_q near[q][s])
 __global__ void finalize_kernel(int ns, int nchunks, const double* __restrict__ partial,
-                                double far_scale, const double* __restrict__ near,
+                                double far_scale, const double* __restrict__ near, int nparts,
                                 double G5, double* __restrict__ gz) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= ns) return;
   double f = 0.0;
   for (int c = 0; c < nchunks; c++) f += partial[(size_t)c * ns + s];
   double g = far_scale * f;
-  if (near) g += near[s];
+  if (near) {
+    double n = near[s];
+    for (int q = 1; q < nparts; q++) n += near[(size_t)q * ns + s];
+    g += n;
+  }
   gz[s] = G5 * g;
 }
 
@@ -620,6 +626,17 @@ FarShape far_shape(const MeshConst& k, int ns, int num_sms, const ztm_opts* o, i
   return f;
 }
 
+// Near work of the far kernel's queue.  A station's near vertices (a few
+// hundred to two thousand double corner functions) take one warp 100 us and
+// more, so few stations leave most of the chip idle: up to sixteen warps per SM
+// each take a part of a station (9x7 stations over 33x29x14 prisms: a call
+// 726 us with 32 whole stations per item).  From 16384 stations on an item is
+// 32 whole stations, as its count alone fills the queue; below, fewer.
+int near_parts(int ns, int num_sms) {
+  return std::max(1, std::min(16, (int)((16LL * std::max(num_sms, 1) + ns - 1) / ns)));
+}
+int near_units(int ns) { return std::max(4, std::min(32, ns / 2048 * 4)); }
+
 std::vector<long long> tune_key(const MeshConst& k, int ns) {
   return {1, k.nx, k.ny, k.nz, ns};
 }
@@ -683,6 +700,7 @@ void launch_mesh_near_iv(ztm_ctx* c, const MeshConst& k, const MeshDesc& m, int 
 }
 
 size_t ztm_prism_ws(const MeshDesc& m, int ns, int precision, int num_sms, const ztm_opts* o) {
+  if (precision == ZTM_PREC_FP64 && ztm_far64_use(m, ns)) return ztm_prism64_ws(m, ns, num_sms);
   if (precision == ZTM_PREC_FP64) {
     const long long nv = (long long)(m.nx + 1) * (m.ny + 1) * (m.nz + 1);
     long long len;
@@ -698,7 +716,8 @@ size_t ztm_prism_ws(const MeshDesc& m, int ns, int precision, int num_sms, const
   return WsCarver::need(sizeof(int)) + WsCarver::need((size_t)k.ncols * k.nzp * 4) +
          WsCarver::need((size_t)ns * 16) * 2 + WsCarver::need((size_t)ns * 4) +
          ztm_station_order_ws(ns, m.nx, m.ny) +
-         WsCarver::need((size_t)ns * 8) + WsCarver::need((size_t)chunks * ns * 8) +
+         WsCarver::need((size_t)near_parts(ns, num_sms) * ns * 8) +
+         WsCarver::need((size_t)chunks * ns * 8) +
          WsCarver::need((size_t)ns * k.nslots * 4) + WsCarver::need((size_t)ns * 8);
 }
 
@@ -706,6 +725,8 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
                      const double* d_sxyz, double* d_gz, double G, int precision,
                      const ztm_opts* o, WsCarver& wc) {
   const double G5 = G * 1.0e5;
+  if (precision == ZTM_PREC_FP64 && ztm_far64_use(m, ns))
+    return ztm_launch_prism64(c, m, d_rho, ns, d_sxyz, d_gz, G, wc);
   if (precision == ZTM_PREC_FP64) {
     const long long nv = (long long)(m.nx + 1) * (m.ny + 1) * (m.nz + 1);
     if (nv > (1LL << 31) - 1) return ztm_fail(c, ZTM_ERR_RANGE, "mesh has more than 2^31-1 vertices");
@@ -721,7 +742,7 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
                                                                            partial);
     }
     finalize_kernel<<<(ns + 255) / 256, 256, 0, c->stream>>>(ns, (int)ch, partial, 1.0, nullptr,
-                                                             G5, d_gz);
+                                                             0, G5, d_gz);
     c->launches += 3;
     return ztm_after_launch(c, "prism FP64 kernels");
   }
@@ -743,7 +764,8 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
   float* rhoT = wc.take<float>((size_t)k.ncols * k.nzp);
   float4* sf = wc.take<float4>(ns);
   int4* si = wc.take<int4>(ns);
-  double* near = wc.take<double>(ns);
+  const int nparts = near_parts(ns, c->num_sms);
+  double* near = wc.take<double>((size_t)nparts * ns);
   int max_chunks = 0;
   for (const auto& sh : FAR_SHAPES)
     max_chunks = std::max(max_chunks, far_shape(k, ns, c->num_sms, o, sh[0], sh[1]).chunks);
@@ -762,7 +784,9 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
   a.perm = perm;
   a.err = c->d_err;
   a.counter = counter;
-  a.n_near = (ns + FAR_NEAR_ST - 1) / FAR_NEAR_ST;
+  a.nparts = nparts;
+  a.near_units = near_units(ns);
+  a.n_near = (int)(((long long)ns * nparts + a.near_units - 1) / a.near_units);
   a.near_f64 = precision == ZTM_PREC_MIXED;
   a.m = m;
   a.sxyz = d_sxyz;
@@ -815,7 +839,7 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
   }
   const double far_scale = k.L0 * (double)k.dxn * k.dyn * k.dzn;
   finalize_kernel<<<(ns + 255) / 256, 256, 0, c->stream>>>(ns, f.chunks, partial, far_scale, near,
-                                                           G5, d_gz);
+                                                           nparts, G5, d_gz);
   c->launches++;
   return ztm_after_launch(c, "prism mixed kernels");
 }
@@ -863,7 +887,7 @@ int ztm_launch_prism_list(ztm_ctx* c, long long np, const double* d_geom, const 
   } else {
     ch = 0;
   }
-  finalize_kernel<<<(ns + 255) / 256, 256, 0, c->stream>>>(ns, (int)ch, partial, 1.0, nullptr, G5,
+  finalize_kernel<<<(ns + 255) / 256, 256, 0, c->stream>>>(ns, (int)ch, partial, 1.0, nullptr, 0, G5,
                                                            d_gz);
   c->launches++;
   return ztm_after_launch(c, "prism list kernels");

@@ -1,0 +1,780 @@
+// prism64.cu - the double prism forward and adjoint on meshes larger than
+// their near regions: far field in float pairs (far64.cuh), near regions
+// (closer than FAR64_Q half-diagonals) by the closed form in double.
+//
+// The vertex kernels of prism.cu and adjoint.cu evaluate one double corner
+// function per (vertex, station) and run on the FP64 pipe alone: 51.6 ms for
+// 64x64x32 prisms under 32x32 stations, two FP64 results a clock per SM.  Here
+// the FP64 pipe only sees the near vertices (about 1,050 a station) and the
+// FMA pipe takes the other pairs at about 0.6 clocks each; both run at once,
+// as blocks of one launch.  What is left on the vertex kernels: meshes that
+// are mostly near region, and shapes outside far64_use's limits.
+//
+// Inputs are scaled by a power of two of their largest magnitude (found in the
+// preparation kernel) so that float pairs cannot overflow or lose low parts.
+#include <cuda_runtime.h>
+#include <math.h>
+
+#include <algorithm>
+
+#include "far64.cuh"
+#include "prism_common.cuh"
+#include "ztm_internal.cuh"
+
+// ---------------------------------------------------------------------------
+// coefficients
+namespace {
+
+// Integer table of one derivative: the coefficients of x^i y^(j-i) u^(n+j) in
+// d^2a/dX^2a d^2b/dY^2b of Z/r^3, relative to Z/r^3 (a + b = n), built by
+// differentiating polynomials over odd powers of r (all integers, exact in
+// double).  Independent of any input; made once.
+struct DerivTable {
+  double d[FAR64_N + 1][FAR64_N + 1][FAR64_N + 1][FAR64_N + 1];  // [n][a][j][i]
+  DerivTable() {
+    constexpr int DG = 2 * FAR64_N + 2;  // degrees 0 .. DG-1 per variable
+    auto at = [](int x, int y, int z) { return (x * DG + y) * DG + z; };
+    double binom[DG][DG] = {};
+    for (int p = 0; p < DG; p++) {
+      binom[p][0] = 1.0;
+      for (int q = 1; q <= p; q++) binom[p][q] = binom[p - 1][q - 1] + (q < p ? binom[p - 1][q] : 0.0);
+    }
+    for (auto& q : d)
+      for (auto& r : q)
+        for (auto& s : r)
+          for (double& v : s) v = 0.0;
+    std::vector<double> P(DG * DG * DG), Q(DG * DG * DG);
+    // P / r^(2m+1) differentiated along `axis`: Q / r^(2m+3)
+    auto derive = [&](int m, int axis) {
+      std::fill(Q.begin(), Q.end(), 0.0);
+      for (int x = 0; x < DG; x++)
+        for (int y = 0; y < DG; y++)
+          for (int z = 0; z < DG; z++) {
+            const double v = P[at(x, y, z)];
+            if (v == 0.0) continue;
+            int e[3] = {x, y, z};
+            const int p = e[axis];
+            if (p) {
+              int k[3] = {x, y, z};
+              k[axis]--;
+              for (int t = 0; t < 3; t++) {
+                int k2[3] = {k[0], k[1], k[2]};
+                k2[t] += 2;
+                Q[at(k2[0], k2[1], k2[2])] += p * v;
+              }
+            }
+            e[axis]++;
+            Q[at(e[0], e[1], e[2])] -= (2 * m + 1) * v;
+          }
+      P.swap(Q);
+    };
+    for (int n = 1; n <= FAR64_N; n++)
+      for (int a = 0; a <= n; a++) {
+        std::fill(P.begin(), P.end(), 0.0);
+        P[0] = 1.0;
+        int m = 0;
+        for (int q = 0; q < 2 * a; q++) derive(m++, 0);
+        for (int q = 0; q < 2 * (n - a); q++) derive(m++, 1);
+        derive(m++, 2);
+        for (int x = 0; x <= 2 * n; x += 2)
+          for (int y = 0; x + y <= 2 * n; y += 2) {
+            const int z = 2 * n - x - y;
+            const double v = P[at(x, y, z + 1)];
+            if (v == 0.0) continue;
+            const int A = x / 2, B = y / 2, C = z / 2;
+            // -P/Z with Z^2C = (r^2 - x - y)^C
+            for (int k = 0; k <= C; k++)
+              for (int l = 0; l <= k; l++)
+                d[n][a][A + B + k][A + l] +=
+                    -v * binom[C][k] * (k % 2 ? -1.0 : 1.0) * binom[k][l];
+          }
+      }
+  }
+};
+
+double factorial(int n) {
+  double f = 1.0;
+  for (int q = 2; q <= n; q++) f *= q;
+  return f;
+}
+
+}  // namespace
+
+void far64_coefs(double dx, double dy, double dz, double* c) {
+  static const DerivTable table;
+  const double ax = 0.25 * dx * dx, ay = 0.25 * dy * dy, az = 0.25 * dz * dz;
+  double binom[FAR64_N + 1][FAR64_N + 1] = {};
+  for (int p = 0; p <= FAR64_N; p++) {
+    binom[p][0] = 1.0;
+    for (int q = 1; q <= p; q++) binom[p][q] = binom[p - 1][q - 1] + (q < p ? binom[p - 1][q] : 0.0);
+  }
+  for (int q = 0; q < FAR64_COEFS; q++) c[q] = 0.0;
+  for (int n = 1; n <= FAR64_N; n++) {
+    // box moments over d^2i/dX d^2j/dY d^2k/dZ, with d^2/dZ^2 = -(d^2/dX^2 + d^2/dY^2)
+    double A[FAR64_N + 1] = {};
+    for (int i = 0; i <= n; i++)
+      for (int j = 0; i + j <= n; j++) {
+        const int k = n - i - j;
+        const double mom = pow(ax, i) * pow(ay, j) * pow(az, k) /
+                           (factorial(2 * i + 1) * factorial(2 * j + 1) * factorial(2 * k + 1));
+        for (int l = 0; l <= k; l++) A[i + l] += mom * (k % 2 ? -1.0 : 1.0) * binom[k][l];
+      }
+    for (int a = 0; a <= n; a++)
+      for (int j = 0; j <= n; j++)
+        for (int i = 0; i <= j; i++) c[far64_at(n, j, i)] += A[a] * table.d[n][a][j][i];
+  }
+}
+
+Far64Coef far64_make(const MeshDesc& m, double L0) {
+  Far64Coef f;
+  double c[FAR64_COEFS];
+  const double dx = m.dx / L0, dy = m.dy / L0, dz = m.dz / L0;
+  far64_coefs(dx, dy, dz, c);
+  for (int q = 0; q < FAR64_COEFS; q++) f.c[q] = (float)c[q];
+  for (int q = 0; q < 9; q++) f.lo[q] = (float)(c[q] - (double)f.c[q]);
+  f.dxh = (float)dx;
+  f.dxl = (float)(dx - (double)f.dxh);
+  f.dyh = (float)dy;
+  f.dyl = (float)(dy - (double)f.dyh);
+  f.dzh = (float)dz;
+  f.dzl = (float)(dz - (double)f.dzh);
+  const double ell = 0.5 * sqrt(dx * dx + dy * dy + dz * dz);
+  f.rh_b = (float)(FAR64_Q_B * FAR64_Q_B * ell * ell);
+  f.rh_c = (float)(FAR64_Q_C * FAR64_Q_C * ell * ell);
+  return f;
+}
+
+namespace {
+
+using far64::D2;
+
+constexpr int F64_T = 128;       // threads per block: stations (forward), columns (adjoint)
+constexpr int F64_STAGE = 1024;  // float4 per shared-memory stage of the forward (16 KB)
+constexpr int F64_LG = 8;        // layers per thread of the adjoint
+constexpr int F64_ST = 32;       // stations per shared-memory tile of the adjoint
+constexpr int F64_MAX_NZ = F64_STAGE;
+constexpr int F64_MAX_SLOTS = 1024;
+
+// Power-of-two scale of the input whose largest |value| has high word `hw`
+// (0 or not finite: 1): values * 2^-e lie below 2.
+__device__ __forceinline__ int scale_exp(unsigned hw) {
+  const int b = (int)(hw >> 20);
+  return (b == 0 || b >= 2047) ? 0 : min(b - 1023, 1022);
+}
+__device__ __forceinline__ double pow2(int e) {  // 2^e, |e| <= 1022
+  return __hiloint2double((1023 + e) << 20, 0);
+}
+
+// Station remainders and home cells (as station_prep_kernel, in pairs of
+// floats), and the largest |v| over nv values (its high word, by atomicMax on
+// *hw, zeroed before): the density (forward) or the residuals (adjoint).
+__global__ void f64_prep(MeshDesc m, double L0, int ns, const double* __restrict__ sxyz,
+                         float4* __restrict__ sxy, float2* __restrict__ sz, int4* __restrict__ si,
+                         long long nv, const double* __restrict__ v, unsigned* __restrict__ hw) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  unsigned w = 0;
+  for (long long q = t; q < nv; q += stride)
+    w = max(w, (unsigned)__double2hiint(v[q]) & 0x7fffffffu);
+  w = __reduce_max_sync(0xffffffffu, w);
+  if ((threadIdx.x & 31) == 0 && w) atomicMax(hw, w);
+  for (long long q = t; q < ns; q += stride) {
+    const int s = (int)q;
+    const double xs = sxyz[3 * s], ys = sxyz[3 * s + 1], zs = sxyz[3 * s + 2];
+    const double lim = 1.0e9;
+    const int ix = (int)fmin(fmax(floor((xs - m.x0) / m.dx), -lim), lim);
+    const int iy = (int)fmin(fmax(floor((ys - m.y0) / m.dy), -lim), lim);
+    const int iz = (int)fmin(fmax(floor((m.zt - zs) / m.dz), -lim), lim);
+    const double ex = ((xs - m.x0) - (ix + 0.5) * m.dx) / L0;
+    const double ey = ((ys - m.y0) - (iy + 0.5) * m.dy) / L0;
+    const double ez = (zs - (m.zt - (iz + 0.5) * m.dz)) / L0;
+    const float xh = (float)ex, yh = (float)ey, zh = (float)ez;
+    sxy[s] = make_float4(xh, (float)(ex - (double)xh), yh, (float)(ey - (double)yh));
+    sz[s] = make_float2(zh, (float)(ez - (double)zh));
+    si[s] = make_int4(ix, iy, iz, 0);
+  }
+}
+
+// Density in pairs of floats, two neighbouring columns per entry:
+// rp[cp*nz + l] = (hi A, hi B, lo A, lo B) of columns 2cp, 2cp+1 at layer l,
+// scaled by 2^-scale_exp; a column past the end is zero.  A block takes 32
+// column pairs x 32 layers through shared memory, so that both sides are
+// coalesced.
+__global__ void __launch_bounds__(256)
+    f64_split(int ncols, int nz, const double* __restrict__ rho, const unsigned* __restrict__ hw,
+              float4* __restrict__ rp) {
+  __shared__ float2 t[32][65];
+  const double sc = pow2(-scale_exp(*hw));
+  const int c0 = blockIdx.x * 64, l0 = blockIdx.y * 32;
+  for (int q = threadIdx.x; q < 32 * 64; q += 256) {
+    const int l = q >> 6, c = q & 63;
+    const double v = (l0 + l < nz && c0 + c < ncols) ? rho[(long long)(l0 + l) * ncols + c0 + c] * sc : 0.0;
+    const float h = (float)v;
+    t[l][c] = make_float2(h, (float)(v - (double)h));
+  }
+  __syncthreads();
+  const int npair = (ncols + 1) >> 1;
+  for (int q = threadIdx.x; q < 32 * 32; q += 256) {
+    const int cp = q >> 5, l = q & 31;
+    if (l0 + l < nz && (c0 >> 1) + cp < npair) {
+      const float2 a = t[l][2 * cp], b = t[l][2 * cp + 1];
+      rp[(size_t)((c0 >> 1) + cp) * nz + l0 + l] = make_float4(a.x, b.x, a.y, b.y);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// forward
+struct Fwd64Args {
+  Far64Coef fc;
+  MeshConst k;
+  MeshDesc m;
+  int ns, npair;
+  int near_blocks, nparts;     // near blocks: 4 warps, one (station, part) each
+  int tiles, chunk_pairs;      // far blocks: station tile x chunk of column pairs
+  const float4* sxy;
+  const float2* sz;
+  const int4* si;
+  const int* perm;
+  const short2* iv;
+  const int2* lr;
+  const double* sxyz;
+  const double* rho;
+  const float4* rp;
+  double* near;     // [nparts][ns]
+  double* partial;  // [chunk][ns]
+};
+
+// All layers of one column pair against this thread's station.
+template <int FORM, bool MASK>
+__device__ __forceinline__ void fwd_pair(const Far64Coef& f, const float4* col, int nz, D2 X, D2 Y,
+                                         float n0, float2 ez, int2 a, int2 b, D2& acc) {
+  const far64::Col o = far64::make_col<FORM>(f, X, Y);
+  float n = n0;
+  for (int l = 0; l < nz; l++, n += 1.f) {
+    float zh, zl, qh, ql;
+    far64::layer_z(n, f, ez.x, ez.y, &zh, &zl, &qh, &ql);
+    const D2 v = far64::value<FORM>(f, o, far64::dd_dup(zh, zl), far64::dd_dup(qh, ql));
+    const float4 w = col[l];
+    // near layers [a.x, a.y] of the first column, [b.x, b.y] of the second
+    far64::mac(acc, make_float2(w.x, w.y), make_float2(w.z, w.w), v,
+               MASK && (unsigned)(l - a.x) <= (unsigned)(a.y - a.x),
+               MASK && (unsigned)(l - b.x) <= (unsigned)(b.y - b.x));
+  }
+  acc = far64::quick(acc.h, acc.l);
+}
+
+__global__ void __launch_bounds__(F64_T, 4) f64_fwd_kernel(const __grid_constant__ Fwd64Args a) {
+  __shared__ float4 stage[F64_STAGE];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const MeshConst& k = a.k;
+  if ((int)blockIdx.x < a.near_blocks) {
+    // near regions first in the grid: their blocks start with the launch and
+    // use the FP64 pipe while the far blocks use the FMA pipe
+    const int w = blockIdx.x * (F64_T / 32) + warp;
+    const int s = w / a.nparts, part = w % a.nparts;
+    if (s < a.ns)
+      near_station<double>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho,
+                           a.near + (size_t)part * a.ns, lane, nullptr, part, a.nparts);
+    return;
+  }
+  const int item = blockIdx.x - a.near_blocks;
+  const int tile = item % a.tiles, chunk = item / a.tiles;
+  const int slot = tile * F64_T + threadIdx.x;
+  // threads past the last station repeat it (a finite value that is not stored)
+  const int s = a.perm[min(slot, a.ns - 1)];
+  const float4 e = a.sxy[s];
+  const float2 ez = a.sz[s];
+  const int4 h = a.si[s];
+  const NearBox nb = near_box(h, k);
+  const float n0 = -(float)h.z;
+  const int p0 = chunk * a.chunk_pairs, p1 = min(a.npair, p0 + a.chunk_pairs);
+  const int sp = F64_STAGE / k.nz;  // column pairs per stage
+  D2 acc = far64::dd_dup(0.f, 0.f);
+  double tot = 0.0;
+  for (int q0 = p0; q0 < p1; q0 += sp) {
+    const int q1 = min(p1, q0 + sp);
+    __syncthreads();
+    for (int t = threadIdx.x; t < (q1 - q0) * k.nz; t += F64_T)
+      stage[t] = a.rp[(size_t)q0 * k.nz + t];
+    __syncthreads();
+    for (int q = q0; q < q1; q++) {
+      const int ca = 2 * q, cb = ca + 1;
+      const int xa = ca % k.nx, ya = ca / k.nx, xb = cb % k.nx, yb = cb / k.nx;
+      const D2 X = far64::offset(make_float2((float)(h.x - xa), (float)(h.x - xb)), a.fc.dxh,
+                                 a.fc.dxl, far64::dup(e.x), far64::dup(e.y));
+      const D2 Y = far64::offset(make_float2((float)(h.y - ya), (float)(h.y - yb)), a.fc.dyh,
+                                 a.fc.dyl, far64::dup(e.z), far64::dup(e.w));
+      const float rh = fminf(fmaf(X.h.x, X.h.x, Y.h.x * Y.h.x), fmaf(X.h.y, X.h.y, Y.h.y * Y.h.y));
+      const bool na = xa >= nb.x0 && xa <= nb.x1 && ya >= nb.y0 && ya <= nb.y1;
+      const bool nbb = xb >= nb.x0 && xb <= nb.x1 && yb >= nb.y0 && yb <= nb.y1;
+      int2 ia = make_int2(1 << 20, 1 << 20), ib = ia;  // no layer
+      if (na) {
+        const short2 t = a.iv[(size_t)s * k.nslots + near_slot(nb, xa, ya)];
+        if (t.x <= t.y) ia = make_int2(t.x, t.y);
+      }
+      if (nbb) {
+        const short2 t = a.iv[(size_t)s * k.nslots + near_slot(nb, xb, yb)];
+        if (t.x <= t.y) ib = make_int2(t.x, t.y);
+      }
+      const bool pad = cb >= k.ncols;  // no second column: every layer of it masked
+      if (pad) ib = make_int2(0, k.nz);
+      const float4* col = stage + (q - q0) * k.nz;
+      // one form and one mask variant per warp
+      if (pad || __any_sync(0xffffffffu, na || nbb))
+        fwd_pair<0, true>(a.fc, col, k.nz, X, Y, n0, ez, ia, ib, acc);
+      else if (__all_sync(0xffffffffu, rh >= a.fc.rh_c))
+        fwd_pair<2, false>(a.fc, col, k.nz, X, Y, n0, ez, ia, ib, acc);
+      else if (__all_sync(0xffffffffu, rh >= a.fc.rh_b))
+        fwd_pair<1, false>(a.fc, col, k.nz, X, Y, n0, ez, ia, ib, acc);
+      else
+        fwd_pair<0, false>(a.fc, col, k.nz, X, Y, n0, ez, ia, ib, acc);
+    }
+    tot += ((double)acc.h.x + (double)acc.l.x) + ((double)acc.h.y + (double)acc.l.y);
+    acc = far64::dd_dup(0.f, 0.f);
+  }
+  if (slot < a.ns) a.partial[(size_t)chunk * a.ns + s] = tot;
+}
+
+// gz[s] = G5 (far_scale 2^e sum_chunks partial + sum_parts near): 32 stations
+// per block, 16 threads each over the chunks, summed in a fixed order.
+__global__ void __launch_bounds__(512)
+    f64_fwd_finalize(int ns, int nchunks, const double* __restrict__ partial, int nparts,
+                     const double* __restrict__ near, double far_scale,
+                     const unsigned* __restrict__ hw, double G5, double* __restrict__ gz) {
+  __shared__ double sm[16][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int s = blockIdx.x * 32 + x;
+  double f = 0.0;
+  if (s < ns)
+    for (int c = y; c < nchunks; c += 16) f += partial[(size_t)c * ns + s];
+  sm[y][x] = f;
+  __syncthreads();
+  if (y || s >= ns) return;
+  f = 0.0;
+#pragma unroll
+  for (int q = 0; q < 16; q++) f += sm[q][x];
+  double n = 0.0;
+  for (int q = 0; q < nparts; q++) n += near[(size_t)q * ns + s];
+  gz[s] = G5 * (far_scale * (f * pow2(scale_exp(*hw))) + n);
+}
+
+// ---------------------------------------------------------------------------
+// adjoint
+struct Adj64Args {
+  Far64Coef fc;
+  MeshConst k;
+  MeshDesc m;
+  int ns;
+  int near_blocks, cap;       // near blocks: 4 warps taking stations in turn
+  int ctiles, groups, slice;  // far blocks: column tile x layer group x station slice
+  int fix_exp;                // near sums in fixed point: value * 2^(fix_exp - scale_exp)
+  const float4* sxy;
+  const float2* sz;
+  const int4* si;
+  const int* perm;
+  const short2* iv;
+  const int2* lr;
+  const double* sxyz;
+  const double* res;
+  const unsigned* hw;         // high word of the largest |res|
+  double* phi;                // [near block][warp][cap] vertex values
+  unsigned long long* gnear;  // [np] fixed-point near sums, zeroed before
+  double* partial;            // [slice][np]
+};
+
+struct Adj64Smem {
+  float2 xh[F64_ST / 2], xl[F64_ST / 2], yh[F64_ST / 2], yl[F64_ST / 2];  // remainders
+  float2 hx[F64_ST / 2], hy[F64_ST / 2];                                  // home cells
+  float2 rh[F64_ST / 2], rl[F64_ST / 2];                                  // residuals
+  int4 box[F64_ST];                                                       // near box columns
+  int id[F64_ST];
+  float4 z[F64_ST / 2][F64_LG], q[F64_ST / 2][F64_LG];  // (hi, hi, lo, lo) of Z, Z^2
+};
+
+// One column's layers of the group against a station pair.
+template <int FORM, bool MASK>
+__device__ __forceinline__ void adj_pair(const Far64Coef& f, const Adj64Smem& sm, int q, D2 X, D2 Y,
+                                         int2 a, int2 b, D2 (&acc)[F64_LG]) {
+  const far64::Col o = far64::make_col<FORM>(f, X, Y);
+  const float2 rh = sm.rh[q], rl = sm.rl[q];
+#pragma unroll
+  for (int l = 0; l < F64_LG; l++) {
+    const float4 z = sm.z[q][l], zz = sm.q[q][l];
+    const D2 v = far64::value<FORM>(f, o, D2{make_float2(z.x, z.y), make_float2(z.z, z.w)},
+                                    D2{make_float2(zz.x, zz.y), make_float2(zz.z, zz.w)});
+    far64::mac(acc[l], rh, rl, v, MASK && (unsigned)(l - a.x) <= (unsigned)(a.y - a.x),
+               MASK && (unsigned)(l - b.x) <= (unsigned)(b.y - b.x));
+  }
+}
+
+// Near region of station s by one warp: Phi at the vertices of a near prism,
+// then the signed corner sums, added in fixed point (order-independent).
+__device__ void adj64_near(const Adj64Args& a, int s, double* phi, int lane) {
+  const MeshConst& k = a.k;
+  const MeshDesc& m = a.m;
+  const double r = a.res[s];
+  const unsigned hw = *a.hw;
+  if (r == 0.0 || (hw >> 20) >= 2047u) return;  // not finite: the finalize writes NaN
+  const int2 L = a.lr[s];
+  if (L.x > L.y) return;
+  const NearBox b = near_box(a.si[s], k);
+  const short2* ivs = a.iv + (size_t)s * k.nslots;
+  const double xs = a.sxyz[3 * s], ys = a.sxyz[3 * s + 1], zs = a.sxyz[3 * s + 2];
+  const int nvx = b.x1 - b.x0 + 2, nvy = b.y1 - b.y0 + 2, nvz = L.y - L.x + 2;
+  const int nv = nvx * nvy * nvz;
+  if (nv > a.cap) return;  // the host sizes cap for the largest box
+  for (int v = lane; v < nv; v += 32) {
+    const int ax = v % nvx, ay = (v / nvx) % nvy, cz = L.x + v / (nvx * nvy);
+    bool used = false;  // a corner of some near prism
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+      const int ix = b.x0 + ax - 1 + (d & 1), iy = b.y0 + ay - 1 + (d >> 1);
+      if (ix < b.x0 || ix > b.x1 || iy < b.y0 || iy > b.y1) continue;
+      const short2 t = ivs[near_slot(b, ix, iy)];
+      used |= t.x <= t.y && cz >= t.x && cz <= t.y + 1;
+    }
+    if (used)
+      phi[v] = ztm_phi<double>((m.x0 + (b.x0 + ax) * m.dx) - xs, (m.y0 + (b.y0 + ay) * m.dy) - ys,
+                               (m.zt - cz * m.dz) - zs);
+  }
+  __syncwarp();
+  const double sc = r * pow2(max(-1022, min(1022, a.fix_exp - scale_exp(hw))));
+  const int bx = nvx - 1, by = nvy - 1, nb = bx * by * (nvz - 1);
+  for (int q = lane; q < nb; q += 32) {
+    const int qx = q % bx, qy = (q / bx) % by, qz = q / (bx * by);
+    const short2 t = ivs[near_slot(b, b.x0 + qx, b.y0 + qy)];
+    const int l = L.x + qz;
+    if (l < t.x || l > t.y) continue;
+    auto P = [&](int dx, int dy, int dz) { return phi[(qx + dx) + nvx * ((qy + dy) + nvy * (qz + dz))]; };
+    const double u = P(1, 1, 0) - P(0, 1, 0) - P(1, 0, 0) + P(0, 0, 0) - P(1, 1, 1) + P(0, 1, 1) +
+                     P(1, 0, 1) - P(0, 0, 1);
+    const long long p = (b.x0 + qx) + (long long)m.nx * (b.y0 + qy) + (long long)k.ncols * l;
+    atomicAdd(&a.gnear[p], (unsigned long long)__double2ll_rn(sc * u));
+  }
+  __syncwarp();
+}
+
+__global__ void __launch_bounds__(F64_T, 4) f64_adj_kernel(const __grid_constant__ Adj64Args a) {
+  __shared__ __align__(16) Adj64Smem sm;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const MeshConst& k = a.k;
+  if ((int)blockIdx.x < a.near_blocks) {
+    const int w = blockIdx.x * (F64_T / 32) + warp;
+    for (int s = w; s < a.ns; s += a.near_blocks * (F64_T / 32))
+      adj64_near(a, s, a.phi + (size_t)w * a.cap, lane);
+    return;
+  }
+  int item = blockIdx.x - a.near_blocks;
+  const int ct = item % a.ctiles;
+  item /= a.ctiles;
+  const int lg = item % a.groups, sl = item / a.groups;
+  const int cc = ct * F64_T + threadIdx.x, c = min(cc, k.ncols - 1);
+  const int ix = c % k.nx, iy = c / k.nx, l0 = lg * F64_LG;
+  const float fix = (float)ix, fiy = (float)iy;
+  const double rsc = pow2(-scale_exp(*a.hw));
+  D2 acc[F64_LG];
+#pragma unroll
+  for (int l = 0; l < F64_LG; l++) acc[l] = far64::dd_dup(0.f, 0.f);
+  const int s0 = sl * a.slice, s1 = min(a.ns, s0 + a.slice);
+  for (int t0 = s0; t0 < s1; t0 += F64_ST) {
+    __syncthreads();
+    for (int q = threadIdx.x; q < F64_ST * F64_LG; q += F64_T) {
+      const int j = q / F64_LG, l = q % F64_LG, lane2 = j & 1;
+      const bool ok = t0 + j < s1;
+      const int s = a.perm[min(t0 + j, s1 - 1)];  // past the slice: repeated, zero residual
+      const int4 h = a.si[s];
+      float zh, zl, qh, ql;
+      const float2 ez = a.sz[s];
+      far64::layer_z((float)(l0 + l) - (float)h.z, a.fc, ez.x, ez.y, &zh, &zl, &qh, &ql);
+      float* z = reinterpret_cast<float*>(&sm.z[j >> 1][l]);
+      float* zz = reinterpret_cast<float*>(&sm.q[j >> 1][l]);
+      z[lane2] = zh;
+      z[2 + lane2] = zl;
+      zz[lane2] = qh;
+      zz[2 + lane2] = ql;
+      if (l == 0) {
+        const float4 e = a.sxy[s];
+        const double r = ok ? a.res[s] * rsc : 0.0;
+        const float r1 = (float)r;
+        const NearBox b = near_box(h, k);
+        auto put = [&](float2* d, float v) { reinterpret_cast<float*>(&d[j >> 1])[lane2] = v; };
+        put(sm.xh, e.x);
+        put(sm.xl, e.y);
+        put(sm.yh, e.z);
+        put(sm.yl, e.w);
+        put(sm.hx, (float)h.x);
+        put(sm.hy, (float)h.y);
+        put(sm.rh, r1);
+        put(sm.rl, (float)(r - (double)r1));
+        sm.box[j] = ok ? make_int4(b.x0, b.x1, b.y0, b.y1) : make_int4(1, 0, 1, 0);
+        sm.id[j] = s;
+      }
+    }
+    __syncthreads();
+    const int np = (min(F64_ST, s1 - t0) + 1) >> 1;
+    for (int q = 0; q < np; q++) {
+      const D2 X = far64::offset(far64::sub(sm.hx[q], far64::dup(fix)), a.fc.dxh, a.fc.dxl,
+                                 sm.xh[q], sm.xl[q]);
+      const D2 Y = far64::offset(far64::sub(sm.hy[q], far64::dup(fiy)), a.fc.dyh, a.fc.dyl,
+                                 sm.yh[q], sm.yl[q]);
+      const float rh = fminf(fmaf(X.h.x, X.h.x, Y.h.x * Y.h.x), fmaf(X.h.y, X.h.y, Y.h.y * Y.h.y));
+      int2 iv[2];
+      bool near = false;
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const int4 b = sm.box[2 * q + j];
+        iv[j] = make_int2(1 << 20, 1 << 20);
+        if (ix >= b.x && ix <= b.y && iy >= b.z && iy <= b.w) {
+          near = true;
+          const short2 t = a.iv[(size_t)sm.id[2 * q + j] * k.nslots + (ix - b.x) +
+                                (b.y - b.x + 1) * (iy - b.z)];
+          if (t.x <= t.y) iv[j] = make_int2(t.x - l0, t.y - l0);
+        }
+      }
+      // the repeated station of an odd count may sit on a prism centre: masked
+      const bool pad = t0 + 2 * q + 1 >= s1;
+      if (pad) iv[1] = make_int2(0, F64_LG);
+      if (pad || __any_sync(0xffffffffu, near))
+        adj_pair<0, true>(a.fc, sm, q, X, Y, iv[0], iv[1], acc);
+      else if (__all_sync(0xffffffffu, rh >= a.fc.rh_c))
+        adj_pair<2, false>(a.fc, sm, q, X, Y, iv[0], iv[1], acc);
+      else if (__all_sync(0xffffffffu, rh >= a.fc.rh_b))
+        adj_pair<1, false>(a.fc, sm, q, X, Y, iv[0], iv[1], acc);
+      else
+        adj_pair<0, false>(a.fc, sm, q, X, Y, iv[0], iv[1], acc);
+    }
+#pragma unroll
+    for (int l = 0; l < F64_LG; l++) acc[l] = far64::quick(acc[l].h, acc[l].l);
+  }
+  if (cc >= k.ncols) return;
+  double* out = a.partial + (size_t)sl * ((size_t)k.ncols * k.nz) + c;
+#pragma unroll
+  for (int l = 0; l < F64_LG; l++)
+    if (l0 + l < k.nz)
+      out[(size_t)(l0 + l) * k.ncols] = ((double)acc[l].h.x + (double)acc[l].l.x) +
+                                        ((double)acc[l].h.y + (double)acc[l].l.y);
+}
+
+__global__ void f64_adj_finalize(long long np, int slices, const double* __restrict__ partial,
+                                 const unsigned long long* __restrict__ gnear, double far_scale,
+                                 int fix_exp, const unsigned* __restrict__ hw, double G5,
+                                 double* __restrict__ g) {
+  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (p >= np) return;
+  const unsigned w = *hw;
+  if ((w >> 20) >= 2047u) {  // a residual that is not finite reaches every prism
+    g[p] = __longlong_as_double(0x7ff8000000000000ll);
+    return;
+  }
+  double f = 0.0;
+  for (int q = 0; q < slices; q++) f += partial[(size_t)q * np + p];
+  const int e = scale_exp(w);
+  const double n = (double)(long long)gnear[p] * pow2(max(-1022, min(1022, e - fix_exp)));
+  g[p] = G5 * (far_scale * (f * pow2(e)) + n);
+}
+
+// ---------------------------------------------------------------------------
+struct Fwd64Shape {
+  int tiles, npair, chunk_pairs, chunks, nparts, near_blocks;
+};
+
+// Far blocks of a station tile x a chunk of column pairs, about sixteen per
+// SM slot; a near warp per station, or per part of a station's vertices while
+// the stations alone would not give every SM sixteen warps.
+Fwd64Shape fwd64_shape(const MeshConst& k, int ns, int num_sms) {
+  Fwd64Shape f;
+  f.tiles = (ns + F64_T - 1) / F64_T;
+  f.npair = (k.ncols + 1) / 2;
+  const int sp = std::max(1, F64_STAGE / k.nz);
+  const long long want = std::max(1LL, (64LL * num_sms + f.tiles - 1) / f.tiles);
+  long long cp = std::max(1LL, (f.npair + want - 1) / want);
+  if (cp > sp) cp = (cp + sp - 1) / sp * sp;  // whole stages
+  f.chunk_pairs = (int)cp;
+  f.chunks = (f.npair + f.chunk_pairs - 1) / f.chunk_pairs;
+  f.nparts = (int)std::max(1LL, std::min(16LL, (16LL * num_sms + ns - 1) / ns));
+  f.near_blocks = (int)(((long long)ns * f.nparts + F64_T / 32 - 1) / (F64_T / 32));
+  return f;
+}
+
+struct Adj64Shape {
+  int ctiles, groups, slice, slices, near_blocks, cap;
+};
+
+int adj64_cap(const MeshConst& k) {
+  return (std::min(2 * k.wx + 1, k.nx) + 1) * (std::min(2 * k.wy + 1, k.ny) + 1) *
+         (std::min(2 * k.wl + 1, k.nz) + 1);
+}
+
+Adj64Shape adj64_shape(const MeshConst& k, int ns, int num_sms) {
+  Adj64Shape f;
+  f.ctiles = (k.ncols + F64_T - 1) / F64_T;
+  f.groups = (k.nz + F64_LG - 1) / F64_LG;
+  const long long per = (long long)f.ctiles * f.groups;
+  long long want = std::max(1LL, (64LL * num_sms + per - 1) / per);
+  want = std::min(want, 16LL);  // the slices' partial sums are np doubles each
+  long long sl = (ns + want - 1) / want;
+  sl = (sl + F64_ST - 1) / F64_ST * F64_ST;
+  f.slice = (int)sl;
+  f.slices = (ns + f.slice - 1) / f.slice;
+  // two near blocks per SM at most: each warp owns a box of vertex values
+  f.near_blocks = (int)std::min<long long>(((long long)ns + F64_T / 32 - 1) / (F64_T / 32), 2LL * num_sms);
+  f.cap = adj64_cap(k);
+  return f;
+}
+
+// Preparation shared by both directions.
+struct Prep64 {
+  unsigned* hw;
+  float4* sxy;
+  float2* sz;
+  int4* si;
+  int* perm;
+  short2* iv;
+  int2* lr;
+};
+
+size_t prep64_ws(const MeshConst& k, int ns) {
+  return WsCarver::need(4) + WsCarver::need((size_t)ns * 16) * 2 + WsCarver::need((size_t)ns * 8) +
+         WsCarver::need((size_t)ns * 4) + ztm_station_order_ws(ns, k.nx, k.ny) +
+         WsCarver::need((size_t)ns * k.nslots * 4) + WsCarver::need((size_t)ns * 8);
+}
+
+int prep64(ztm_ctx* c, const MeshDesc& m, const MeshConst& k, int ns, const double* d_sxyz,
+           long long nv, const double* d_v, WsCarver& wc, Prep64* o) {
+  o->hw = wc.take<unsigned>(1);
+  o->sxy = wc.take<float4>(ns);
+  o->sz = wc.take<float2>(ns);
+  o->si = wc.take<int4>(ns);
+  o->perm = wc.take<int>(ns);
+  o->iv = wc.take<short2>((size_t)ns * k.nslots);
+  o->lr = wc.take<int2>(ns);
+  cudaMemsetAsync(o->hw, 0, 4, c->stream);
+  const long long n = std::max((long long)ns, nv);
+  const int blocks = (int)std::max(1LL, std::min((n + 255) / 256, 8LL * std::max(c->num_sms, 1)));
+  f64_prep<<<blocks, 256, 0, c->stream>>>(m, k.L0, ns, d_sxyz, o->sxy, o->sz, o->si, nv, d_v, o->hw);
+  c->launches++;
+  if (int rc = ztm_station_order(c, c->stream, ns, reinterpret_cast<const int*>(o->si), 4, m.nx,
+                                 m.ny, o->perm, wc))
+    return rc;
+  launch_mesh_near_iv(c, k, m, ns, o->si, d_sxyz, o->iv, o->lr);
+  return ZTM_OK;
+}
+
+}  // namespace
+
+// Where the far field pays: a mesh with at least twice the vertices of the
+// largest near box (below that most of it is closed form either way), near
+// boxes of at most F64_MAX_SLOTS columns (flat cells have wide boxes), and
+// columns that fit a stage.
+bool ztm_far64_use(const MeshDesc& m, int ns) {
+  if (ns < 1 || m.nz > F64_MAX_NZ) return false;
+  const double emax = std::max(m.dx, std::max(m.dy, m.dz)), emin = std::min(m.dx, std::min(m.dy, m.dz));
+  if (!(emax / emin <= 32.0)) return false;  // wider boxes than F64_MAX_SLOTS; int-safe below
+  const MeshConst k = make_mesh_const(m, FAR64_Q);
+  if (k.nslots > F64_MAX_SLOTS || (long long)ns * k.nslots > (1LL << 29) || k.ncols > (1 << 30))
+    return false;
+  const long long nv = (long long)(m.nx + 1) * (m.ny + 1) * (m.nz + 1);
+  return nv >= 2LL * adj64_cap(k);
+}
+
+size_t ztm_prism64_ws(const MeshDesc& m, int ns, int num_sms) {
+  const MeshConst k = make_mesh_const(m, FAR64_Q);
+  const Fwd64Shape f = fwd64_shape(k, ns, std::max(num_sms, 1));
+  return prep64_ws(k, ns) + WsCarver::need((size_t)f.npair * k.nz * 16) +
+         WsCarver::need((size_t)f.nparts * ns * 8) + WsCarver::need((size_t)f.chunks * ns * 8);
+}
+
+int ztm_launch_prism64(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
+                       const double* d_sxyz, double* d_gz, double G, WsCarver& wc) {
+  Fwd64Args a;
+  a.k = make_mesh_const(m, FAR64_Q);
+  a.fc = far64_make(m, a.k.L0);
+  a.m = m;
+  a.ns = ns;
+  const Fwd64Shape f = fwd64_shape(a.k, ns, std::max(c->num_sms, 1));
+  Prep64 p;
+  if (int rc = prep64(c, m, a.k, ns, d_sxyz, (long long)a.k.ncols * a.k.nz, d_rho, wc, &p)) return rc;
+  float4* rp = wc.take<float4>((size_t)f.npair * a.k.nz);
+  a.near = wc.take<double>((size_t)f.nparts * ns);
+  a.partial = wc.take<double>((size_t)f.chunks * ns);
+  a.npair = f.npair;
+  a.near_blocks = f.near_blocks;
+  a.nparts = f.nparts;
+  a.tiles = f.tiles;
+  a.chunk_pairs = f.chunk_pairs;
+  a.sxy = p.sxy;
+  a.sz = p.sz;
+  a.si = p.si;
+  a.perm = p.perm;
+  a.iv = p.iv;
+  a.lr = p.lr;
+  a.sxyz = d_sxyz;
+  a.rho = d_rho;
+  a.rp = rp;
+  f64_split<<<dim3((a.k.ncols + 63) / 64, (a.k.nz + 31) / 32), 256, 0, c->stream>>>(
+      a.k.ncols, a.k.nz, d_rho, p.hw, rp);
+  {
+    ZtmProf prof_(c, "prism_f64");
+    f64_fwd_kernel<<<(unsigned)(f.near_blocks + f.tiles * f.chunks), F64_T, 0, c->stream>>>(a);
+  }
+  const double far_scale = m.dx / a.k.L0 * (m.dy / a.k.L0) * m.dz;
+  f64_fwd_finalize<<<(ns + 31) / 32, 512, 0, c->stream>>>(ns, f.chunks, a.partial, f.nparts, a.near,
+                                                          far_scale, p.hw, G * 1.0e5, d_gz);
+  c->launches += 3;
+  return ztm_after_launch(c, "prism FP64 kernels");
+}
+
+size_t ztm_adjoint64_ws(const MeshDesc& m, int ns, int num_sms) {
+  const MeshConst k = make_mesh_const(m, FAR64_Q);
+  const Adj64Shape f = adj64_shape(k, ns, std::max(num_sms, 1));
+  const size_t np = (size_t)k.ncols * k.nz;
+  return prep64_ws(k, ns) + WsCarver::need((size_t)f.near_blocks * (F64_T / 32) * f.cap * 8) +
+         WsCarver::need(np * 8) + WsCarver::need((size_t)f.slices * np * 8);
+}
+
+int ztm_launch_adjoint64(ztm_ctx* c, const MeshDesc& m, int ns, const double* d_sxyz,
+                         const double* d_res, double* d_g, double G, WsCarver& wc) {
+  Adj64Args a;
+  a.k = make_mesh_const(m, FAR64_Q);
+  a.fc = far64_make(m, a.k.L0);
+  a.m = m;
+  a.ns = ns;
+  const Adj64Shape f = adj64_shape(a.k, ns, std::max(c->num_sms, 1));
+  const size_t np = (size_t)a.k.ncols * a.k.nz;
+  Prep64 p;
+  if (int rc = prep64(c, m, a.k, ns, d_sxyz, ns, d_res, wc, &p)) return rc;
+  a.phi = wc.take<double>((size_t)f.near_blocks * (F64_T / 32) * f.cap);
+  a.gnear = wc.take<unsigned long long>(np);
+  a.partial = wc.take<double>((size_t)f.slices * np);
+  a.near_blocks = f.near_blocks;
+  a.cap = f.cap;
+  a.ctiles = f.ctiles;
+  a.groups = f.groups;
+  a.slice = f.slice;
+  // |r U| < 2^(e+1) 2 pi dz for a prism (no more than an infinite slab), summed
+  // over at most ns stations: below 2^62 in fixed point
+  int b = 0;
+  frexp(2.0 * 6.2831853071795865 * m.dz * ns, &b);
+  a.fix_exp = 61 - b;
+  a.sxy = p.sxy;
+  a.sz = p.sz;
+  a.si = p.si;
+  a.perm = p.perm;
+  a.iv = p.iv;
+  a.lr = p.lr;
+  a.sxyz = d_sxyz;
+  a.res = d_res;
+  a.hw = p.hw;
+  cudaMemsetAsync(a.gnear, 0, np * 8, c->stream);
+  {
+    ZtmProf prof_(c, "adjoint_f64");
+    f64_adj_kernel<<<(unsigned)(f.near_blocks + f.ctiles * f.groups * f.slices), F64_T, 0,
+                     c->stream>>>(a);
+  }
+  const double far_scale = m.dx / a.k.L0 * (m.dy / a.k.L0) * m.dz;
+  f64_adj_finalize<<<(unsigned)((np + 255) / 256), 256, 0, c->stream>>>(
+      (long long)np, f.slices, a.partial, a.gnear, far_scale, a.fix_exp, p.hw, G * 1.0e5, d_g);
+  c->launches += 2;
+  return ztm_after_launch(c, "adjoint FP64 kernels");
+}

@@ -225,7 +225,8 @@ __device__ __forceinline__ int near_slot(const NearBox& b, int ix, int iy) {
 // Near region of station s in T (double: the mixed method; float: the FP32
 // method), by one warp: Phi once per vertex of the region times the signed
 // triple difference of the region's densities around the vertex; lane 0
-// writes out[s].
+// writes out[s].  part of nparts: one of nparts equal ranges of the vertices
+// (the sums of the parts add up to the station's).
 template <typename T>
 __device__ __forceinline__ void near_station(const MeshConst& k, const MeshDesc& m, int s,
                                              const double* __restrict__ sxyz,
@@ -234,7 +235,8 @@ __device__ __forceinline__ void near_station(const MeshConst& k, const MeshDesc&
                                              const int2* __restrict__ lr,
                                              const double* __restrict__ rho,
                                              double* __restrict__ out, int lane,
-                                             unsigned* nphi = nullptr) {
+                                             unsigned* nphi = nullptr, int part = 0,
+                                             int nparts = 1) {
   const NearBox b = near_box(si[s], k);
   const int2 L = lr[s];
   if (L.x > L.y) {  // no near prism
@@ -247,7 +249,9 @@ __device__ __forceinline__ void near_station(const MeshConst& k, const MeshDesc&
   const int nv = nvx * nvy * nvz;
   const long long plane = (long long)m.nx * m.ny;
   T acc = T(0);
-  for (int v = lane; v < nv; v += 32) {
+  const int vb = (int)((long long)nv * part / nparts);
+  const int ve = (int)((long long)nv * (part + 1) / nparts);
+  for (int v = vb + lane; v < ve; v += 32) {
     const int a = b.x0 + v % nvx;
     const int bb = b.y0 + (v / nvx) % nvy;
     const int cz = L.x + v / (nvx * nvy);
