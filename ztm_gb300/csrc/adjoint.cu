@@ -229,16 +229,9 @@ __device__ __forceinline__ void adj_near_station(const AdjArgs& a, int s, T* phi
   const short2* ivs = a.iv + (size_t)s * k.nslots;
   const double xs = a.sxyz[3 * s], ys = a.sxyz[3 * s + 1], zs = a.sxyz[3 * s + 2];
   const int nvx = b.x1 - b.x0 + 2, nvy = b.y1 - b.y0 + 2, nvz = L.y - L.x + 2;
-  const int nv = nvx * nvy * nvz;
-  if (nv > a.cap) return;  // the host sizes cap for the largest box
-  for (int v = lane; v < nv; v += 32) {
-    const int ax = b.x0 + v % nvx;
-    const int ay = b.y0 + (v / nvx) % nvy;
-    const int cz = L.x + v / (nvx * nvy);
-    phi[v] = ztm_phi<T>((T)((m.x0 + ax * m.dx) - xs), (T)((m.y0 + ay * m.dy) - ys),
-                        (T)((m.zt - cz * m.dz) - zs));
-  }
-  __syncwarp();
+  if (nvx * nvy * nvz > a.cap) return;  // the host sizes cap for the largest box
+  near_corners<T>(k, m, b, L, ivs, xs, ys, zs, a.cap, phi, lane);
+  const double sc = sizeof(T) == 8 ? a.G5 * r * k.ninv : a.G5 * r;
   const int bx = nvx - 1, by = nvy - 1, bz = nvz - 1;
   const int nb = bx * by * bz;
   const long long plane = (long long)m.nx * m.ny;
@@ -255,7 +248,7 @@ __device__ __forceinline__ void adj_near_station(const AdjArgs& a, int s, T* phi
     T u = P(1, 1, 0) - P(0, 1, 0) - P(1, 0, 0) + P(0, 0, 0) - P(1, 1, 1) + P(0, 1, 1) + P(1, 0, 1) -
           P(0, 0, 1);
     const long long p = ix + (long long)m.nx * iy + plane * l;
-    atomicAdd(&a.g[p], a.G5 * r * (double)u);
+    atomicAdd(&a.g[p], sc * (double)u);
   }
   __syncwarp();  // the scratch is rewritten by the warp's next station
 }
@@ -399,7 +392,6 @@ int adj_grid_max(int num_sms) { return std::max(adj_grid(num_sms, true), adj_gri
 }  // namespace
 
 size_t ztm_adjoint_ws(const MeshDesc& m, int ns, int precision, int num_sms, double near_q) {
-  if (precision == ZTM_PREC_FP64 && ztm_far64_use(m, ns)) return ztm_adjoint64_ws(m, ns, num_sms);
   if (precision == ZTM_PREC_FP64) {
     const long long nv = (long long)(m.nx + 1) * (m.ny + 1) * (m.nz + 1);
     int len;
@@ -422,8 +414,6 @@ int ztm_launch_adjoint(ztm_ctx* c, const MeshDesc& m, int ns, const double* d_sx
     cudaMemsetAsync(d_g, 0, np * 8, c->stream);
     return ztm_after_launch(c, "adjoint (no stations)");
   }
-  if (precision == ZTM_PREC_FP64 && ztm_far64_use(m, ns))
-    return ztm_launch_adjoint64(c, m, ns, d_sxyz, d_res, d_g, G, wc);
   if (precision == ZTM_PREC_FP64) {
     const long long nv = (long long)(m.nx + 1) * (m.ny + 1) * (m.nz + 1);
     if (nv > (1LL << 31) - 1) return ztm_fail(c, ZTM_ERR_RANGE, "mesh has more than 2^31-1 vertices");

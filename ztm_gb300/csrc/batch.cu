@@ -225,7 +225,7 @@ __device__ void near_item(const BJob& J, int tile, double* phi_all, int phi_cap,
     const int s = J.perm[slot];
     if (J.nmodels == 1) {  // one model: the forward's vertex pass (Phi only where
                            // the region's signed density difference is not zero)
-      near_station<double>(J.k, m, s, J.sxyz, J.si, J.iv, J.lr, J.rho, J.near, lane);
+      near_station<double, false>(J.k, m, s, J.sxyz, J.si, J.iv, J.lr, J.rho, J.near, lane);
       continue;
     }
     const int2 L = J.lr[s];
@@ -237,35 +237,11 @@ __device__ void near_item(const BJob& J, int tile, double* phi_all, int phi_cap,
     const short2* ivs = J.iv + (size_t)s * J.k.nslots;
     const double xs = J.sxyz[3 * s], ys = J.sxyz[3 * s + 1], zs = J.sxyz[3 * s + 2];
     const int nvx = b.x1 - b.x0 + 2, nvy = b.y1 - b.y0 + 2, nvz = L.y - L.x + 2;
-    const int nv = min(nvx * nvy * nvz, J.nv_cap);
-    // is one of the (up to 8) prisms around vertex (a, bb, cz) in the region
-    auto touches = [&](int a, int bb, int cz) {
-#pragma unroll
-      for (int da = 0; da < 2; da++) {
-        const int ix = a - 1 + da;
-        if (ix < b.x0 || ix > b.x1) continue;
-#pragma unroll
-        for (int db = 0; db < 2; db++) {
-          const int iy = bb - 1 + db;
-          if (iy < b.y0 || iy > b.y1) continue;
-          const short2 t = ivs[near_slot(b, ix, iy)];
-          if (t.x <= t.y && t.x <= cz && cz - 1 <= t.y) return true;  // layer cz - 1 or cz
-        }
-      }
-      return false;
-    };
-    for (int v = lane; v < nv; v += 32) {
-      const int a = b.x0 + v % nvx, bb = b.y0 + (v / nvx) % nvy, cz = L.x + v / (nvx * nvy);
-      phi[v] = touches(a, bb, cz) ? ztm_phi<double>((m.x0 + a * m.dx) - xs,
-                                                    (m.y0 + bb * m.dy) - ys,
-                                                    (m.zt - cz * m.dz) - zs)
-                                  : 0.0;
-    }
-    __syncwarp();
+    near_corners<double>(J.k, m, b, L, ivs, xs, ys, zs, J.nv_cap, phi, lane);
     // unit responses: vertices x lower qx (-), upper qx+1 (+); z: layer top
     // index qz (+), bottom qz+1 (-); zero outside the region
     const int bx = nvx - 1, by = nvy - 1, bz = nvz - 1;
-    const int nbp = bx * by * bz;  // < nv
+    const int nbp = bx * by * bz;  // fewer than the vertices
     for (int q = lane; q < nbp; q += 32) {
       const int qx = q % bx, qy = (q / bx) % by, qz = q / (bx * by);
       const short2 t = ivs[near_slot(b, b.x0 + qx, b.y0 + qy)];
@@ -278,7 +254,7 @@ __device__ void near_item(const BJob& J, int tile, double* phi_all, int phi_cap,
         u = P(1, 1, 0) - P(0, 1, 0) - P(1, 0, 0) + P(0, 0, 0) - P(1, 1, 1) + P(0, 1, 1) +
             P(1, 0, 1) - P(0, 0, 1);
       }
-      U[q] = u;
+      U[q] = u * J.k.ninv;
     }
     __syncwarp();
     for (int md = 0; md < J.nmodels; md++) {

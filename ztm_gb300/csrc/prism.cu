@@ -280,10 +280,10 @@ __global__ void __launch_bounds__(FAR_TS, 6) far_kernel(FarArgs a) {
         if (s >= a.ns) break;
         double* out = a.near + (size_t)part * a.ns;
         if (a.near_f64)
-          near_station<double>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho, out, lane,
+          near_station<double, false>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho, out, lane,
                                COUNT ? &nphi : nullptr, part, a.nparts);
         else
-          near_station<float>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho, out, lane,
+          near_station<float, false>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho, out, lane,
                               COUNT ? &nphi : nullptr, part, a.nparts);
       }
       if (threadIdx.x == 0) s_item[par] = nxt < n_items ? atomicAdd(a.counter, 1) : n_items;
@@ -579,6 +579,17 @@ __global__ void __launch_bounds__(F64_TS)
 }
 
 // ---------------------------------------------------------------------------
+// Near work of the far kernel's queue.  A station's near vertices (a few
+// hundred to two thousand double corner functions) take one warp 100 us and
+// more, so few stations leave most of the chip idle: up to sixteen warps per SM
+// each take a part of a station (9x7 stations over 33x29x14 prisms: a call
+// 726 us with 32 whole stations per item).  From 16384 stations on an item is
+// 32 whole stations, as its count alone fills the queue; below, fewer.
+int near_parts(int ns, int num_sms) {
+  return std::max(1, std::min(16, (int)((16LL * std::max(num_sms, 1) + ns - 1) / ns)));
+}
+int near_units(int ns) { return std::max(4, std::min(32, ns / 2048 * 4)); }
+
 struct FarShape {
   int tiles, chunks, chunk_cols, sc, grid;
   size_t smem;
@@ -622,20 +633,11 @@ FarShape far_shape(const MeshConst& k, int ns, int num_sms, const ztm_opts* o, i
   cc = ((cc + sc - 1) / sc) * sc;
   f.chunk_cols = cc;
   f.chunks = (k.ncols + cc - 1) / cc;
-  f.grid = (int)std::min(resident, (long long)f.tiles * f.chunks);
+  const int nu = near_units(ns);
+  const long long n_near = ((long long)ns * near_parts(ns, num_sms) + nu - 1) / nu;
+  f.grid = (int)std::min(resident, (long long)f.tiles * f.chunks + n_near);
   return f;
 }
-
-// Near work of the far kernel's queue.  A station's near vertices (a few
-// hundred to two thousand double corner functions) take one warp 100 us and
-// more, so few stations leave most of the chip idle: up to sixteen warps per SM
-// each take a part of a station (9x7 stations over 33x29x14 prisms: a call
-// 726 us with 32 whole stations per item).  From 16384 stations on an item is
-// 32 whole stations, as its count alone fills the queue; below, fewer.
-int near_parts(int ns, int num_sms) {
-  return std::max(1, std::min(16, (int)((16LL * std::max(num_sms, 1) + ns - 1) / ns)));
-}
-int near_units(int ns) { return std::max(4, std::min(32, ns / 2048 * 4)); }
 
 std::vector<long long> tune_key(const MeshConst& k, int ns) {
   return {1, k.nx, k.ny, k.nz, ns};
@@ -674,6 +676,8 @@ MeshConst make_mesh_const(const MeshDesc& m, double near_q) {
   const double R = near_q * 0.5 * sqrt(m.dx * m.dx + m.dy * m.dy + m.dz * m.dz);
   k.R2 = R * R;
   k.nslots = (2 * k.wx + 1) * (2 * k.wy + 1);
+  k.nsc = ldexp(1.0, -ilogb(k.L0));
+  k.ninv = ldexp(1.0, ilogb(k.L0));
   return k;
 }
 
@@ -700,7 +704,6 @@ void launch_mesh_near_iv(ztm_ctx* c, const MeshConst& k, const MeshDesc& m, int 
 }
 
 size_t ztm_prism_ws(const MeshDesc& m, int ns, int precision, int num_sms, const ztm_opts* o) {
-  if (precision == ZTM_PREC_FP64 && ztm_far64_use(m, ns)) return ztm_prism64_ws(m, ns, num_sms);
   if (precision == ZTM_PREC_FP64) {
     const long long nv = (long long)(m.nx + 1) * (m.ny + 1) * (m.nz + 1);
     long long len;
@@ -725,8 +728,6 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
                      const double* d_sxyz, double* d_gz, double G, int precision,
                      const ztm_opts* o, WsCarver& wc) {
   const double G5 = G * 1.0e5;
-  if (precision == ZTM_PREC_FP64 && ztm_far64_use(m, ns))
-    return ztm_launch_prism64(c, m, d_rho, ns, d_sxyz, d_gz, G, wc);
   if (precision == ZTM_PREC_FP64) {
     const long long nv = (long long)(m.nx + 1) * (m.ny + 1) * (m.nz + 1);
     if (nv > (1LL << 31) - 1) return ztm_fail(c, ZTM_ERR_RANGE, "mesh has more than 2^31-1 vertices");

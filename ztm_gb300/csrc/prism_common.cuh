@@ -4,6 +4,9 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#ifdef __CUDACC__
+#include "phi64.cuh"
+#endif
 #include "ztm_internal.cuh"
 
 // Far-field expansion of one prism's attraction, relative to the point-mass
@@ -170,6 +173,8 @@ struct MeshConst {
   double L0;
   double dxm, dym, dzm;  // cell edges (m)
   double R2;             // (near_q * half diagonal)^2 (m^2)
+  double nsc, ninv;      // power of two near 1/L0 and its reciprocal: near
+                         // regions' corners are taken in those units
   int nslots;            // (2wx+1)(2wy+1): columns of a near box
   FarCoef fc;
 };
@@ -222,12 +227,82 @@ __device__ __forceinline__ int near_slot(const NearBox& b, int ix, int iy) {
   return (ix - b.x0) + (b.x1 - b.x0 + 1) * (iy - b.y0);
 }
 
+// Corner function of a near region's vertex (offsets in m): double in scaled
+// lengths by phi64.cuh (the result times ninv is the corner function up to
+// terms linear in x and y, which the signed corner sums drop), float by the
+// library functions in metres.
+template <typename T>
+__device__ __forceinline__ T near_phi(const MeshConst& k, double x, double y, double z);
+template <>
+__device__ __forceinline__ double near_phi<double>(const MeshConst& k, double x, double y,
+                                                   double z) {
+  return phi64::phi(x * k.nsc, y * k.nsc, z * k.nsc);
+}
+template <>
+__device__ __forceinline__ float near_phi<float>(const MeshConst&, double x, double y, double z) {
+  return ztm_phi<float>((float)x, (float)y, (float)z);
+}
+
+// A warp's queue of near vertices (index, and density difference where one is
+// used), one entry per lane, held in registers so that full warps evaluate.
+struct NearQueue {
+  int v, n;  // this lane's entry; entries held (lanes 0 .. n-1)
+  double d;
+  // position of the r-th set bit of m
+  static __device__ __forceinline__ int nth(unsigned m, int r) {
+    int p = 0;
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1) {
+      const int c = __popc(m & ((1u << h) - 1u));
+      if (r >= c) {
+        r -= c;
+        p += h;
+        m >>= h;
+      }
+    }
+    return p & 31;
+  }
+  // Adds the entries of the lanes with `use`; calls eval(v, d) on every lane
+  // when there are 32.
+  template <class F>
+  __device__ __forceinline__ void push(int lane, bool use, int nv, double nd, F&& eval) {
+    const unsigned bal = __ballot_sync(0xffffffffu, use);
+    const int cnt = __popc(bal);
+    const int sa = nth(bal, lane - n);  // (not used below lane n)
+    const int va = __shfl_sync(0xffffffffu, nv, sa);
+    const double da = __shfl_sync(0xffffffffu, nd, sa);
+    if (lane >= n) {
+      v = va;
+      d = da;
+    }
+    if (n + cnt >= 32) {
+      eval(v, d);
+      const int sb = nth(bal, 32 - n + lane);
+      v = __shfl_sync(0xffffffffu, nv, sb);
+      d = __shfl_sync(0xffffffffu, nd, sb);
+      n += cnt - 32;
+    } else {
+      n += cnt;
+    }
+  }
+  template <class F>
+  __device__ __forceinline__ void finish(int lane, F&& eval) {
+    if (lane < n) eval(v, d);
+  }
+};
+
 // Near region of station s in T (double: the mixed method; float: the FP32
 // method), by one warp: Phi once per vertex of the region times the signed
 // triple difference of the region's densities around the vertex; lane 0
 // writes out[s].  part of nparts: one of nparts equal ranges of the vertices
-// (the sums of the parts add up to the station's).
-template <typename T>
+// (the sums of the parts add up to the station's).  The vertices whose
+// difference is not zero are about 45% of the box around the region; QUEUED:
+// they go through the warp's queue so that every Phi is evaluated by a full
+// warp.  That pays where near regions bound the kernel (the double forward);
+// in the mixed far kernel, which hides them behind the FMA pipe, the queue's
+// registers cost the far loop 3% (22.2 against 21.5 ms, 256x256x64 prisms under
+// 128x128 stations), so it evaluates in place.
+template <typename T, bool QUEUED>
 __device__ __forceinline__ void near_station(const MeshConst& k, const MeshDesc& m, int s,
                                              const double* __restrict__ sxyz,
                                              const int4* __restrict__ si,
@@ -251,44 +326,92 @@ __device__ __forceinline__ void near_station(const MeshConst& k, const MeshDesc&
   T acc = T(0);
   const int vb = (int)((long long)nv * part / nparts);
   const int ve = (int)((long long)nv * (part + 1) / nparts);
-  for (int v = vb + lane; v < ve; v += 32) {
-    const int a = b.x0 + v % nvx;
-    const int bb = b.y0 + (v / nvx) % nvy;
-    const int cz = L.x + v / (nvx * nvy);
-    // signed triple difference of the region's density around vertex
-    // (a, bb, cz): prism ix = a-1 has the vertex as its upper x limit (+),
-    // ix = a lower (-); layer l = cz has it as its upper z limit (+), l = cz-1
-    // lower (-).
+  auto eval = [&](int v, double D) {
+    const int a = b.x0 + v % nvx, bb = b.y0 + (v / nvx) % nvy, cz = L.x + v / (nvx * nvy);
+    acc = fma((T)D, near_phi<T>(k, fma((double)a, m.dx, m.x0) - xs,
+                                fma((double)bb, m.dy, m.y0) - ys,
+                                fma(-(double)cz, m.dz, m.zt) - zs), acc);
+    if (nphi) ++*nphi;
+  };
+  NearQueue q;
+  q.n = 0;
+  for (int v0 = vb; v0 < ve; v0 += 32) {
+    const int v = v0 + lane;
     double D = 0.0;
+    if (v < ve) {
+      const int a = b.x0 + v % nvx;
+      const int bb = b.y0 + (v / nvx) % nvy;
+      const int cz = L.x + v / (nvx * nvy);
+      // signed triple difference of the region's density around vertex
+      // (a, bb, cz): prism ix = a-1 has the vertex as its upper x limit (+),
+      // ix = a lower (-); layer l = cz has it as its upper z limit (+), l = cz-1
+      // lower (-).
 #pragma unroll
-    for (int da = 0; da < 2; da++) {
-      const int ix = a - 1 + da;
-      if (ix < b.x0 || ix > b.x1) continue;
+      for (int da = 0; da < 2; da++) {
+        const int ix = a - 1 + da;
+        if (ix < b.x0 || ix > b.x1) continue;
 #pragma unroll
-      for (int db = 0; db < 2; db++) {
-        const int iy = bb - 1 + db;
-        if (iy < b.y0 || iy > b.y1) continue;
-        const short2 t = ivs[near_slot(b, ix, iy)];
+        for (int db = 0; db < 2; db++) {
+          const int iy = bb - 1 + db;
+          if (iy < b.y0 || iy > b.y1) continue;
+          const short2 t = ivs[near_slot(b, ix, iy)];
 #pragma unroll
-        for (int dc = 0; dc < 2; dc++) {
-          const int l = cz - 1 + dc;
-          if (l < t.x || l > t.y) continue;
-          const double r = rho[ix + (long long)m.nx * iy + plane * l];
-          const int neg = (da == 1) ^ (db == 1) ^ (dc == 0);
-          D += neg ? -r : r;
+          for (int dc = 0; dc < 2; dc++) {
+            const int l = cz - 1 + dc;
+            if (l < t.x || l > t.y) continue;
+            const double r = rho[ix + (long long)m.nx * iy + plane * l];
+            const int neg = (da == 1) ^ (db == 1) ^ (dc == 0);
+            D += neg ? -r : r;
+          }
         }
       }
     }
-    if (D != 0.0) {
-      const T x = (T)((m.x0 + a * m.dx) - xs);
-      const T y = (T)((m.y0 + bb * m.dy) - ys);
-      const T z = (T)((m.zt - cz * m.dz) - zs);
-      acc += (T)D * ztm_phi<T>(x, y, z);
-      if (nphi) ++*nphi;
-    }
+    if (QUEUED)
+      q.push(lane, D != 0.0, v, D, eval);
+    else if (D != 0.0)
+      eval(v, D);
   }
+  if (QUEUED) q.finish(lane, eval);
   double tot = warp_sum_d((double)acc);
-  if (lane == 0) out[s] = tot;
+  if (lane == 0) out[s] = sizeof(T) == 8 ? tot * k.ninv : tot;
+}
+
+// Corner functions of a near region's vertices, by one warp: phi[v] of every
+// vertex of the near box's layers L.x .. L.y + 1 (v = x + nvx (y + nvy z),
+// cap values at most) that is a corner of a near prism, the others untouched.
+// Full warps evaluate, through a queue as in near_station; double values
+// are in scaled lengths (times ninv: metres).
+template <typename T>
+__device__ __forceinline__ void near_corners(const MeshConst& k, const MeshDesc& m,
+                                             const NearBox& b, int2 L,
+                                             const short2* __restrict__ ivs, double xs, double ys,
+                                             double zs, int cap, T* __restrict__ phi, int lane) {
+  const int nvx = b.x1 - b.x0 + 2, nvy = b.y1 - b.y0 + 2, nvz = L.y - L.x + 2;
+  const int nv = min(nvx * nvy * nvz, cap);
+  auto eval = [&](int v, double) {
+    phi[v] = near_phi<T>(k, fma((double)(b.x0 + v % nvx), m.dx, m.x0) - xs,
+                         fma((double)(b.y0 + (v / nvx) % nvy), m.dy, m.y0) - ys,
+                         fma(-(double)(L.x + v / (nvx * nvy)), m.dz, m.zt) - zs);
+  };
+  NearQueue q;
+  q.n = 0;
+  for (int v0 = 0; v0 < nv; v0 += 32) {
+    const int v = v0 + lane;
+    bool used = false;
+    if (v < nv) {
+      const int ax = v % nvx, ay = (v / nvx) % nvy, cz = L.x + v / (nvx * nvy);
+#pragma unroll
+      for (int d = 0; d < 4; d++) {  // the (up to) four columns around the vertex
+        const int ix = b.x0 + ax - 1 + (d & 1), iy = b.y0 + ay - 1 + (d >> 1);
+        if (ix < b.x0 || ix > b.x1 || iy < b.y0 || iy > b.y1) continue;
+        const short2 t = ivs[near_slot(b, ix, iy)];
+        used |= t.x <= t.y && cz >= t.x && cz <= t.y + 1;
+      }
+    }
+    q.push(lane, used, v, 0.0, eval);
+  }
+  q.finish(lane, eval);
+  __syncwarp();
 }
 
 // ---- host launchers (prism.cu) ------------------------------------------
