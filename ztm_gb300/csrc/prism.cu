@@ -704,6 +704,7 @@ void launch_mesh_near_iv(ztm_ctx* c, const MeshConst& k, const MeshDesc& m, int 
 }
 
 size_t ztm_prism_ws(const MeshDesc& m, int ns, int precision, int num_sms, const ztm_opts* o) {
+  if (precision == ZTM_PREC_FP64 && ztm_far64_use(m, ns)) return ztm_prism64_ws(m, ns, num_sms);
   if (precision == ZTM_PREC_FP64) {
     const long long nv = (long long)(m.nx + 1) * (m.ny + 1) * (m.nz + 1);
     long long len;
@@ -728,6 +729,8 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
                      const double* d_sxyz, double* d_gz, double G, int precision,
                      const ztm_opts* o, WsCarver& wc) {
   const double G5 = G * 1.0e5;
+  if (precision == ZTM_PREC_FP64 && ztm_far64_use(m, ns))
+    return ztm_launch_prism64(c, m, d_rho, ns, d_sxyz, d_gz, G, wc);
   if (precision == ZTM_PREC_FP64) {
     const long long nv = (long long)(m.nx + 1) * (m.ny + 1) * (m.nz + 1);
     if (nv > (1LL << 31) - 1) return ztm_fail(c, ZTM_ERR_RANGE, "mesh has more than 2^31-1 vertices");

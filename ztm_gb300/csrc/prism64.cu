@@ -274,8 +274,9 @@ __global__ void __launch_bounds__(F64_T, 4) f64_fwd_kernel(const __grid_constant
     const int w = blockIdx.x * (F64_T / 32) + warp;
     const int s = w / a.nparts, part = w % a.nparts;
     if (s < a.ns)
-      near_station<double>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho,
-                           a.near + (size_t)part * a.ns, lane, nullptr, part, a.nparts);
+      near_station<double, true>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho,
+                           a.near + (size_t)part * a.ns, lane,
+                           nullptr, part, a.nparts);
     return;
   }
   const int item = blockIdx.x - a.near_blocks;
@@ -422,27 +423,12 @@ __device__ void adj64_near(const Adj64Args& a, int s, double* phi, int lane) {
   const short2* ivs = a.iv + (size_t)s * k.nslots;
   const double xs = a.sxyz[3 * s], ys = a.sxyz[3 * s + 1], zs = a.sxyz[3 * s + 2];
   const int nvx = b.x1 - b.x0 + 2, nvy = b.y1 - b.y0 + 2, nvz = L.y - L.x + 2;
-  const int nv = nvx * nvy * nvz;
-  if (nv > a.cap) return;  // the host sizes cap for the largest box
-  for (int v = lane; v < nv; v += 32) {
-    const int ax = v % nvx, ay = (v / nvx) % nvy, cz = L.x + v / (nvx * nvy);
-    bool used = false;  // a corner of some near prism
-#pragma unroll
-    for (int d = 0; d < 4; d++) {
-      const int ix = b.x0 + ax - 1 + (d & 1), iy = b.y0 + ay - 1 + (d >> 1);
-      if (ix < b.x0 || ix > b.x1 || iy < b.y0 || iy > b.y1) continue;
-      const short2 t = ivs[near_slot(b, ix, iy)];
-      used |= t.x <= t.y && cz >= t.x && cz <= t.y + 1;
-    }
-    if (used)
-      phi[v] = ztm_phi<double>((m.x0 + (b.x0 + ax) * m.dx) - xs, (m.y0 + (b.y0 + ay) * m.dy) - ys,
-                               (m.zt - cz * m.dz) - zs);
-  }
-  __syncwarp();
-  const double sc = r * pow2(max(-1022, min(1022, a.fix_exp - scale_exp(hw))));
+  if (nvx * nvy * nvz > a.cap) return;  // the host sizes cap for the largest box
+  near_corners<double>(k, m, b, L, ivs, xs, ys, zs, a.cap, phi, lane);
+  const double sc = r * k.ninv * pow2(max(-1022, min(1022, a.fix_exp - scale_exp(hw))));
   const int bx = nvx - 1, by = nvy - 1, nb = bx * by * (nvz - 1);
-  for (int q = lane; q < nb; q += 32) {
-    const int qx = q % bx, qy = (q / bx) % by, qz = q / (bx * by);
+  for (int w = lane; w < nb; w += 32) {
+    const int qx = w % bx, qy = (w / bx) % by, qz = w / (bx * by);
     const short2 t = ivs[near_slot(b, b.x0 + qx, b.y0 + qy)];
     const int l = L.x + qz;
     if (l < t.x || l > t.y) continue;
