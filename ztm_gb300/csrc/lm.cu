@@ -76,27 +76,56 @@ __host__ __device__ constexpr uint32_t oz_off(int digit, int k8, int i) {
 
 // Instruction descriptor (kind::f16): D F32 (bits 4-5 = 1), A and B BF16 (bits
 // 7-9, 10-12 = 1), both K-major, N >> 3 in bits 17-22, M >> 4 in bits 24-28.
-constexpr uint32_t OZ_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_N >> 3) << 17) |
-                              ((uint32_t)(OZ_M >> 4) << 24);
+__device__ __forceinline__ uint32_t oz_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
+         ((uint32_t)(OZ_M >> 4) << 24);
+}
 
 __device__ __forceinline__ void oz_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                       uint32_t accumulate) {
+                                       uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(OZ_IDESC), "r"(accumulate)
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
-// Levels read back after stage t of n: level l takes l + 1 products of 2^14 at
-// most per K, so it may hold 32/(l+1) stages of 32; all levels after the last.
+// (h 2^32 + l) 2^e rounded to nearest, in integer instructions: the FP64 pipe's
+// conversions and scalings (six slots an element) cost the trailing update more
+// than its products.  Below the normal range: zero.
+__device__ __forceinline__ double oz_double(long long h, unsigned l, int e) {
+  const bool neg = h < 0;
+  if (neg) {
+    l = 0u - l;
+    h = ~h + (l == 0u);
+  }
+  unsigned long long x;  // leading bits, bit 63 set
+  if (h) {
+    const int z = __clzll(h);
+    x = (unsigned long long)h << z;
+    x |= z >= 32 ? (unsigned long long)l << (z - 32) : (unsigned long long)(l >> (32 - z));
+    e += 95 - z;
+  } else {
+    if (!l) return 0.0;
+    const int z = __clz(l);
+    x = (unsigned long long)l << (z + 32);
+    e += 31 - z;
+  }
+  // round to 53 bits; the carry out of bit 63 moves into the exponent
+  const unsigned long long r = (x >> 11) + ((x >> 10) & 1u);
+  const int be = e + 1022;  // r's bit 52 adds one
+  if (be < 0) return 0.0;
+  if (be > 2045) return __longlong_as_double((neg ? 0xfff0000000000000ull : 0x7ff0000000000000ull));
+  return __longlong_as_double((neg ? 1ull << 63 : 0ull) | (((unsigned long long)be << 52) + r));
+}
+
+// Levels read back after stage t of n: bit 0 the low levels (p + q = 0 .. 3),
+// bit 1 the high ones (4 .. 6).  Level l takes l + 1 products of 2^14 at most per
+// K, so that its sums stay within 2^24: the low levels over 8 stages of 32 (4 x 256
+// x 2^14 = 2^24), the high ones over 4.
 __device__ __forceinline__ unsigned oz_flush(int t, int n) {
-  if (t + 1 == n) return (1u << OZ_S) - 1u;
-  unsigned m = 0;
-#pragma unroll
-  for (int l = 0; l < OZ_S; l++)
-    if ((t + 1) % (32 / (l + 1)) == 0) m |= 1u << l;
-  return m;
+  if (t + 1 == n) return 3u;
+  return ((t + 1) % 8 == 0 ? 1u : 0u) | ((t + 1) % 4 == 0 ? 2u : 0u);
 }
 
 struct OzArgs {
@@ -105,6 +134,7 @@ struct OzArgs {
   int n;                     // indices (rows and columns of the result)
   const int* exps;           // scale exponents of the indices
   int* err;
+  int tiles, work;           // tiles of one matrix; tiles of the launch
   // <0>: JJ partial sums, one matrix per row slice
   int tiles_j;               // column tiles
   int per;                   // chunks per slice
@@ -118,18 +148,44 @@ struct OzArgs {
   const int* bad;            // per pair: not positive definite
 };
 
+// Tile w of the launch: matrix (row slice or pair), row block, column tile.
+struct OzTile {
+  int z, ib, jt, c0, T;
+};
+template <int MODE>
+__device__ __forceinline__ OzTile oz_tile(const OzArgs& a, int w) {
+  OzTile t;
+  t.z = w / a.tiles;
+  int ib = 0, jt = w % a.tiles;
+  if (MODE == 0) {  // upper: column tiles from the diagonal on
+    while (jt >= a.tiles_j - 2 * ib) jt -= a.tiles_j - 2 * ib++;
+    jt += 2 * ib;
+  } else {  // lower: column tiles up to the diagonal
+    while (jt >= 2 * ib + 2) jt -= 2 * ib++ + 2;
+  }
+  t.ib = ib;
+  t.jt = jt;
+  t.c0 = MODE == 0 ? t.z * a.per : 0;
+  t.T = min(a.per, a.nkc - t.c0);
+  return t;
+}
+
 struct OzShared {
-  uint64_t full[2], empty[2], ready, flushed, fin;
+  uint64_t full[2], empty[2], ready, flushed[2], fin;
   uint32_t tmem;
   int fail;
 };
 
-// One 128 x 64 tile: 8 warps of read-back (thread: one row, 32 columns), a
-// thread that copies stages of operand digits (two, 84 KB each), a thread that
-// issues the 56 MMAs of a stage.  The digits of both operands stay in shared
-// memory for all 28 products, so a stage feeds 2,700 clocks of MMA from 84 KB.
-// After a read-back the levels it covers are issued last in the next stage,
-// so that the tensor core works on the others meanwhile.
+// 128 x 64 tiles, one block per SM taking them in turn: 8 warps of read-back
+// (thread: one row, 32 columns), a thread that copies stages of operand digits
+// (two, 84 KB each), a thread that issues the MMAs.  The digits of both operands
+// stay in shared memory for all 28 products.  Digit p of A meets neighbouring
+// digits of B in MMAs up to four digits (N = 256) wide: their levels are
+// neighbouring accumulators, and A is read from shared memory once for them
+// (with N = 64 alone, A's reads bound the MMAs: 82 against 32 clocks each).
+// The levels are issued and read back in two groups, 0 .. 3 and 4 .. 6, so that
+// the tensor core works on one group while the other is read; the conversion
+// and update of a finished tile run beside the next one's copies and MMAs.
 // MODE 0: result rows and columns are columns of J (upper tiles).
 // MODE 1: S -= L L^T over the panel's 64 columns (lower tiles).
 template <int MODE>
@@ -138,19 +194,6 @@ __global__ void __launch_bounds__(OZ_T, 1) oz_kernel(const __grid_constant__ OzA
   OzShared& sh = *reinterpret_cast<OzShared*>(oz_smem);
   unsigned char* stage = oz_smem + 1024;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pair = MODE == 1 ? blockIdx.y : 0;
-  if (MODE == 1 && a.bad[pair]) return;  // uniform: before any barrier or TMEM
-  // the tile's row block and column tile
-  int ib = 0, jt = blockIdx.x;
-  if (MODE == 0) {
-    while (jt >= a.tiles_j - 2 * ib) jt -= a.tiles_j - 2 * ib++;
-    jt += 2 * ib;
-  } else {
-    while (jt >= 2 * ib + 2) jt -= 2 * ib++ + 2;
-  }
-  const int c0 = MODE == 0 ? blockIdx.y * a.per : 0;
-  const int T = min(a.per, a.nkc - c0);
-  const unsigned char* dig = a.dig + pair * a.dig_stride;
   if (warp == 0) {
     tmem_alloc(&sh.tmem, OZ_COLS);
     tmem_relinquish();
@@ -161,7 +204,8 @@ __global__ void __launch_bounds__(OZ_T, 1) oz_kernel(const __grid_constant__ OzA
       mbar_init(&sh.empty[q], 1);
     }
     mbar_init(&sh.ready, 1);
-    mbar_init(&sh.flushed, 256);
+    mbar_init(&sh.flushed[0], 256);
+    mbar_init(&sh.flushed[1], 256);
     mbar_init(&sh.fin, 1);
     sh.fail = 0;
     fence_mbar_init();
@@ -171,96 +215,163 @@ __global__ void __launch_bounds__(OZ_T, 1) oz_kernel(const __grid_constant__ OzA
   tc_fence_after();
   const uint32_t tmem = sh.tmem;
   volatile int* fail = &sh.fail;
-  long long hi[32], lo[32];
+  auto skip = [&](const OzTile& t) { return MODE == 1 && a.bad[t.z] != 0; };
   if (warp < 8) {
-#pragma unroll
-    for (int j = 0; j < 32; j++) hi[j] = lo[j] = 0;
     int ph = 0;
-    for (int t = 0; t < T; t++) {
-      const unsigned m = oz_flush(t, T);
-      if (!m) continue;
-      // one verdict per warp: the TMEM reads below take whole warps
-      if (!__all_sync(0xffffffffu, mbar_wait(&sh.ready, ph & 1))) {
-        *fail = 1;
-        break;
-      }
-      ph++;
-      tc_fence_after();
+    for (int w = blockIdx.x; w < a.work; w += gridDim.x) {
+      const OzTile t = oz_tile<MODE>(a, w);
+      if (skip(t)) continue;
+      long long hi[32], lo[32];
 #pragma unroll
-      for (int l = 0; l < OZ_S; l++) {
-        if (!((m >> l) & 1u)) continue;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          uint32_t v[16];
-          tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 64 * l + 32 * (warp >> 2) + 16 * h, v);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 16; j++) {
-            const long long x = __float2int_rn(__uint_as_float(v[j]));
-            if (l < 3)
-              hi[16 * h + j] += x * (1ll << (l < 3 ? 8 * (2 - l) : 0));
-            else
-              lo[16 * h + j] += x * (1ll << (8 * (6 - l)));
-          }
-        }
-      }
-      tc_fence_before();
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sh.flushed)) : "memory");
-    }
-  } else if (warp == 8 && lane == 0) {
-    const unsigned char* A = dig + ((size_t)ib * a.nkc + c0) * OZ_CHUNK;
-    const unsigned char* B = dig + ((size_t)(jt >> 1) * a.nkc + c0) * OZ_CHUNK + (jt & 1) * 1024;
-    for (int t = 0; t < T; t++) {
-      const int b = t & 1;
-      if (t >= 2 && !mbar_wait(&sh.empty[b], ((t >> 1) - 1) & 1)) {
-        *fail = 1;
-        break;
-      }
-      unsigned char* d = stage + b * OZ_STAGE;
-      mbar_expect_tx(&sh.full[b], OZ_STAGE);
-      bulk_g2s(d, A + (size_t)t * OZ_CHUNK, OZ_CHUNK, &sh.full[b]);
-      for (int q = 0; q < 4 * OZ_S; q++)  // 64 of a chunk's 128 indices, per digit and k/8
-        bulk_g2s(d + OZ_CHUNK + q * 1024, B + (size_t)t * OZ_CHUNK + q * 2048, 1024, &sh.full[b]);
-    }
-  } else if (warp == 9 && lane == 0) {
-    unsigned fresh = (1u << OZ_S) - 1u, prev = 0;
-    int waits = 0;
-    for (int t = 0; t < T; t++) {
-      const int b = t & 1;
-      if (!mbar_wait(&sh.full[b], (t >> 1) & 1)) {
-        *fail = 1;
-        break;
-      }
-      tc_fence_after();
-      const uint32_t sa = smem_u32(stage + b * OZ_STAGE), sb = sa + OZ_CHUNK;
-      auto level = [&](int l) {
-        for (int ks = 0; ks < 2; ks++)
-          for (int p = 0; p <= l; p++) {
-            const uint64_t da = tc_smem_desc(sa + p * OZ_SLICE_A + ks * 4096, 2048, 128);
-            const uint64_t db = tc_smem_desc(sb + (l - p) * OZ_SLICE_B + ks * 2048, 1024, 128);
-            oz_mma(tmem + 64 * l, da, db, (fresh >> l) & 1u ? 0u : 1u);
-            fresh &= ~(1u << l);
-          }
-      };
-      for (int l = 0; l < OZ_S; l++)
-        if (!((prev >> l) & 1u)) level(l);
-      if (prev) {
-        if (!mbar_wait(&sh.flushed, waits & 1)) {
-          *fail = 1;
+      for (int j = 0; j < 32; j++) hi[j] = lo[j] = 0;
+      bool ok = true;
+      for (int k = 0; k < t.T; k++) {
+        const unsigned m = oz_flush(k, t.T);
+        if (!m) continue;
+        // one verdict per warp: the TMEM reads below take whole warps
+        if (!__all_sync(0xffffffffu, mbar_wait(&sh.ready, ph & 1))) {
+          ok = false;
           break;
         }
-        waits++;
+        ph++;
         tc_fence_after();
-        for (int l = 0; l < OZ_S; l++)
-          if ((prev >> l) & 1u) level(l);
+#pragma unroll
+        for (int l = 0; l < OZ_S; l++) {
+          if (l < 4 ? !(m & 1u) : !(m & 2u)) continue;
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            uint32_t v[16];
+            tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 64 * l + 32 * (warp >> 2) + 16 * h, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+              const long long x = __float2int_rn(__uint_as_float(v[j]));
+              if (l < 3)
+                hi[16 * h + j] += x * (1ll << (l < 3 ? 8 * (2 - l) : 0));
+              else
+                lo[16 * h + j] += x * (1ll << (8 * (6 - l)));
+            }
+          }
+          if (l == 3 || l == OZ_S - 1) {  // the group may be written again
+            tc_fence_before();
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sh.flushed[l > 3]))
+                         : "memory");
+          }
+        }
       }
-      tc_commit(&sh.empty[b]);
-      prev = oz_flush(t, T);
-      if (prev) {
-        tc_commit(&sh.ready);
-        fresh |= prev;
+      if (!ok) {
+        *fail = 1;
+        break;
+      }
+      // hi 2^32 + lo, scaled by 2^(e_i + e_j - 64)
+      const int i = t.ib * OZ_M + 32 * (warp & 3) + lane, j0 = t.jt * OZ_N + 32 * (warp >> 2);
+      if (i >= a.n) continue;
+      const int* ex = a.exps + (MODE == 1 ? t.z * a.exp_stride : 0);
+      const int ei = ex[i] - 64;
+      double* out = MODE == 0 ? a.out + ((size_t)t.z * a.n + i) * a.n + j0
+                              : a.S + t.z * a.s_stride + (size_t)(a.r0 + i) * a.ld + a.r0 + j0;
+      // columns of this thread's 32 that belong to the half it writes: [jb, je)
+      const int jb = MODE == 0 ? max(0, min(32, i - j0)) : 0;
+      const int je = MODE == 0 ? max(0, min(32, a.n - j0)) : max(0, min(32, i + 1 - j0));
+      // every load before the first store (eight columns at a time): loads and
+      // stores in turn took 20 us a tile, one memory latency per column
+#pragma unroll
+      for (int q = 0; q < 32; q += 8) {
+        double s[8];
+        int e[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const bool on = q + j >= jb && q + j < je;
+          s[j] = (MODE == 1 && on) ? out[q + j] : 0.0;
+          e[j] = on ? ex[j0 + q + j] : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const double v = oz_double(hi[q + j] + (lo[q + j] >> 32), (unsigned)lo[q + j], ei + e[j]);
+          if (q + j >= jb && q + j < je) out[q + j] = MODE == 1 ? s[j] - v : v;
+        }
       }
     }
+  } else if (warp == 8 && lane == 0) {
+    unsigned g = 0;  // stages of the block so far
+    bool ok = true;
+    for (int w = blockIdx.x; ok && w < a.work; w += gridDim.x) {
+      const OzTile t = oz_tile<MODE>(a, w);
+      if (skip(t)) continue;
+      const unsigned char* dig = a.dig + (MODE == 1 ? t.z * a.dig_stride : 0);
+      const unsigned char* A = dig + ((size_t)t.ib * a.nkc + t.c0) * OZ_CHUNK;
+      const unsigned char* B = dig + ((size_t)(t.jt >> 1) * a.nkc + t.c0) * OZ_CHUNK + (t.jt & 1) * 1024;
+      for (int k = 0; k < t.T; k++, g++) {
+        const unsigned b = g & 1u;
+        if (g >= 2 && !mbar_wait(&sh.empty[b], ((g >> 1) - 1u) & 1u)) {
+          ok = false;
+          break;
+        }
+        unsigned char* d = stage + b * OZ_STAGE;
+        mbar_expect_tx(&sh.full[b], OZ_STAGE);
+        bulk_g2s(d, A + (size_t)k * OZ_CHUNK, OZ_CHUNK, &sh.full[b]);
+        // 64 of a chunk's 128 indices per digit and k/8: [k/8][digit][index]
+        for (int q = 0; q < 4 * OZ_S; q++)
+          bulk_g2s(d + OZ_CHUNK + ((q & 3) * OZ_S + (q >> 2)) * 1024, B + (size_t)k * OZ_CHUNK + q * 2048,
+                   1024, &sh.full[b]);
+      }
+    }
+    if (!ok) *fail = 1;
+  } else if (warp == 9 && lane == 0) {
+    unsigned fresh = 3u, prev = 0, g = 0;  // groups: to be overwritten; being read back
+    unsigned waits[2] = {0u, 0u};
+    bool ok = true;
+    for (int w = blockIdx.x; ok && w < a.work; w += gridDim.x) {
+      const OzTile t = oz_tile<MODE>(a, w);
+      if (skip(t)) continue;
+      for (int k = 0; ok && k < t.T; k++, g++) {
+        const unsigned b = g & 1u;
+        if (!mbar_wait(&sh.full[b], (g >> 1) & 1u)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        // everything but the stage's base is a constant of the unrolled code: with
+        // descriptors and widths formed in loops the issuing thread, not the
+        // tensor core, set the pace (6.6 against 2.8 ms for 12000 x 2700)
+        const uint32_t sa = smem_u32(stage + b * OZ_STAGE);
+        const uint64_t da = tc_smem_desc(sa, 2048, 128);
+        const uint64_t db = tc_smem_desc(sa + OZ_CHUNK, OZ_S * 1024, 128);
+        // groups that were not read back first
+#pragma unroll
+        for (int o = 0; o < 4; o++) {
+          const int grp = o & 1;
+          if (((prev >> grp) & 1u) != (o >> 1)) continue;
+          if (o >> 1) {
+            if (!mbar_wait(&sh.flushed[grp], waits[grp] & 1u)) {
+              ok = false;
+              break;
+            }
+            waits[grp]++;
+            tc_fence_after();
+          }
+          const int l0 = grp ? 4 : 0, l1 = grp ? OZ_S : 4;
+#pragma unroll
+          for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+            for (int p = 0; p < l1; p++) {
+              const int l = p > l0 ? p : l0;  // levels l .. l1 - 1: digits l - p .. of B
+              oz_mma(tmem + 64 * l, da + (p * (OZ_SLICE_A / 16) + ks * 256),
+                     db + ((l - p) * 64 + ks * (2 * OZ_S * 64)), oz_idesc(64 * (l1 - l)),
+                     p == 0 && ks == 0 ? ((fresh >> grp) & 1u) ^ 1u : 1u);
+            }
+        }
+        if (!ok) break;
+        fresh = 0;
+        tc_commit(&sh.empty[b]);
+        prev = oz_flush(k, t.T);
+        if (prev) {
+          tc_commit(&sh.ready);
+          fresh = prev;
+        }
+      }
+    }
+    if (!ok) *fail = 1;
     // every MMA complete before the block frees TMEM and its stages
     tc_commit(&sh.fin);
     if (!mbar_wait(&sh.fin, 0)) *fail = 1;
@@ -279,29 +390,6 @@ __global__ void __launch_bounds__(OZ_T, 1) oz_kernel(const __grid_constant__ OzA
     __syncthreads();
   }
   if (warp == 0) tmem_dealloc(tmem, OZ_COLS);
-  if (warp >= 8 || *fail) return;
-  // hi 2^32 + lo, scaled by 2^(e_i + e_j - 64)
-  const int i = ib * OZ_M + 32 * (warp & 3) + lane, j0 = jt * OZ_N + 32 * (warp >> 2);
-  const int* ex = a.exps + pair * a.exp_stride;
-  if (i >= a.n) return;
-  const int ei = ex[i];
-  double* out = MODE == 0 ? a.out + ((size_t)blockIdx.y * a.n + i) * a.n
-                          : a.S + pair * a.s_stride + (size_t)(a.r0 + i) * a.ld + a.r0;
-#pragma unroll
-  for (int j = 0; j < 32; j++) {
-    const int jj = j0 + j;
-    if (MODE == 0 ? (jj < i || jj >= a.n) : (jj > i)) continue;
-    // integers to double by their bits: |h| < 2^51, 0 <= l < 2^32
-    const long long h = hi[j] + (lo[j] >> 32);
-    const double hd = __longlong_as_double(h + 0x4338000000000000ll) - 6755399441055744.0;
-    const double ld = __hiloint2double(0x43300000, (int)lo[j]) - 4503599627370496.0;
-    const int e = ei + ex[jj] - 64, e1 = e >> 1;
-    const double v = fma(hd, 4294967296.0, ld) * lm_pow2(e1) * lm_pow2(e - e1);
-    if (MODE == 0)
-      out[jj] = v;
-    else
-      out[jj] -= v;
-  }
 }
 
 // The seven digits of x scaled by 2^-e (|x| < 2^(e-1)): x 2^-e = sum of
@@ -362,13 +450,25 @@ __global__ void __launch_bounds__(128)
 __global__ void lm_colfinish(int ncols, int nb, const unsigned* __restrict__ pmax,
                              const double* __restrict__ pdot, int* __restrict__ ex,
                              int* __restrict__ odd, double* __restrict__ g) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ncols) return;
+  // 32 columns a block, eight threads each over the row blocks, in a fixed order
+  __shared__ unsigned sm[8][32];
+  __shared__ double ss[8][32];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, i = blockIdx.x * 32 + x;
   unsigned m = 0;
   double s = 0.0;
-  for (int q = 0; q < nb; q++) {
-    m = max(m, pmax[(size_t)q * ncols + i]);
-    s += pdot[(size_t)q * ncols + i];
+  if (i < ncols)
+    for (int q = y; q < nb; q += 8) {
+      m = max(m, pmax[(size_t)q * ncols + i]);
+      s += pdot[(size_t)q * ncols + i];
+    }
+  sm[y][x] = m;
+  ss[y][x] = s;
+  __syncthreads();
+  if (y || i >= ncols) return;
+#pragma unroll
+  for (int q = 1; q < 8; q++) {
+    m = max(m, sm[q][x]);
+    s += ss[q][x];
   }
   odd[i] = (m >> 20) >= 2047u;  // an infinity or NaN: the column's products are NaN
   ex[i] = odd[i] ? 0 : oz_exp(m);
@@ -443,213 +543,307 @@ __global__ void lm_assemble(int n, int ld, const double* __restrict__ JJ,
 // ---- Cholesky -----------------------------------------------------------------
 constexpr int LM_NB = 64;  // columns of a panel
 
-// Diagonal block: L L^T = A for the panel's nb columns (identity beyond), and
-// 1 / L_ii.  A pivot that is not positive and finite marks the pair.
-// One SM per pair, so the chain over the 64 columns is what counts: one warp forms
-// 1/sqrt(pivot) (float seed, one third-order step), the block scales the
-// column and updates the rest, each thread a 4 x 8 block-cyclic share in
-// registers.
-__global__ void __launch_bounds__(128)
+// 1 / sqrt(p) for a positive finite p: p = m 2^(2q), m in [1, 4), a float
+// pair from the float estimate (its residual in exact float products), then one
+// Newton step in double.  Four dependent FP64 operations: each takes well over
+// a hundred clocks here, and the 64 pivots of a panel follow one another.
+__device__ __forceinline__ double lm_widen(float f) {  // a normal float, by its bits
+  const int b = __float_as_int(f);
+  return __hiloint2double((b & 0x80000000) | (((b & 0x7fffffff) >> 3) + 0x38000000), b << 29);
+}
+__device__ __forceinline__ double lm_rsqrt(double p) {
+  int hi = __double2hiint(p), lo = __double2loint(p), sub = 0;
+  if (hi < 0x00100000) {  // subnormal: 2^128 larger
+    p *= 3.402823669209384635e38;
+    hi = __double2hiint(p);
+    lo = __double2loint(p);
+    sub = 64;
+  }
+  const int q = ((hi >> 20) - 1023) >> 1, k = ((hi >> 20) - 1023) & 1;
+  const double m = __hiloint2double((hi & 0x000fffff) | ((1023 + k) << 20), lo);
+  // m as a float's 24 leading bits and the 29 below
+  const float mh = __int_as_float(((127 + k) << 23) | ((hi & 0x000fffff) << 3) | ((unsigned)lo >> 29));
+  const float ml = (float)(lo & 0x1fffffff) * (k ? 4.440892098500626e-16f : 2.220446049250313e-16f);
+  const float y = rsqrtf(mh);
+  const float s = __fmul_rn(y, y), se = fmaf(y, y, -s);
+  float g = fmaf(-mh, s, 1.f);
+  g = fmaf(-ml, s, g);
+  g = fmaf(-mh, se, g);
+  const double Y = lm_widen(y) + lm_widen(y * (g * fmaf(0.375f, g, 0.5f)));
+  const double h = fma(-m * Y, Y, 1.0);
+  // Y in (0.5, 1]: half of it and the result's scale by the exponent bits
+  const double r = fma(__hiloint2double(__double2hiint(Y) - 0x00100000, __double2loint(Y)), h, Y);
+  return __hiloint2double(__double2hiint(r) + ((sub - q) << 20), __double2loint(r));
+}
+
+// Diagonal block: L L^T = A for the panel's nb columns (identity beyond),
+// 1 / L_ii, and LT[j][k] = L_kj / L_jj (k > j) for lm_trsm.  A pivot that is not
+// positive and finite marks the pair.
+// One SM per pair, so the chain over the 64 columns is what counts.  An FP64
+// instruction holds its quarter of the SM for 64 clocks, and a chain that shares
+// the quarter with another warp's FP64 work waits 290 clocks an operation
+// instead of 65 (measured), so warp 0 has one to itself: it scales column c once
+// for all and, while warps 1 to 3 update with it (a 4 x 11 block-cyclic share
+// of the lower half per thread, in registers), forms the next pivot and its
+// inverse root.  (All four warps updating and a fifth for the chain: 75 us a panel.)
+constexpr int PF_T = 128;
+constexpr int PF_C = 6;                            // thread columns: 96 = 16 x 6
+constexpr int PF_Q = (LM_NB + PF_C - 1) / PF_C;    // columns of a share
+__global__ void __launch_bounds__(PF_T)
     lm_potrf(int n, int k0, int nb, int ld, double* __restrict__ S, double* __restrict__ dinv,
-             int* __restrict__ bad) {
+             double* __restrict__ LT, int* __restrict__ bad) {
   const int d = blockIdx.x;
   if (bad[d]) return;
   double* A = S + ((size_t)d * (n + 1) + k0) * ld + k0;
-  __shared__ double col[2][LM_NB];  // the current column, double buffered
-  __shared__ double s_inv;
+  // column c with its updates complete (buffer c & 1), column c + 1 without the
+  // update by column c, and column c scaled
+  __shared__ double col[2][LM_NB], nxt[2][LM_NB], scl[LM_NB], s_inv[LM_NB];
   __shared__ int s_bad;
-  const int tr = threadIdx.x & 15, tc = threadIdx.x >> 4;  // rows tr + 16a, columns tc + 8b
-  double x[4][8];
+  const bool chain = threadIdx.x < 32;
+  const int t = threadIdx.x - 32, tr = t & 15, tc = t >> 4;  // rows tr + 16a, columns tc + 6q
+  double x[4][PF_Q];
+  if (!chain) {
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+    for (int a = 0; a < 4; a++)
 #pragma unroll
-    for (int b = 0; b < 8; b++) {
-      const int r = tr + 16 * a, c = tc + 8 * b;
-      x[a][b] = (r < nb && c <= r) ? A[(size_t)r * ld + c] : (r == c ? 1.0 : 0.0);
-    }
-  if (threadIdx.x == 0) s_bad = 0;
-#pragma unroll
-  for (int b = 0; b < 8; b++) {
-    for (int cb = 0; cb < 8; cb++) {  // column c = cb + 8 b, held by tc == cb
-      const int c = cb + 8 * b;
-      double* cl = col[c & 1];
-      if (tc == cb) {
-#pragma unroll
-        for (int a = 0; a < 4; a++) cl[tr + 16 * a] = x[a][b];
+      for (int q = 0; q < PF_Q; q++) {
+        const int r = tr + 16 * a, c = tc + PF_C * q;
+        x[a][q] = (r < nb && c <= r) ? A[(size_t)r * ld + c] : (r == c ? 1.0 : 0.0);
+        if (c == 0) col[0][r] = x[a][q];
+        if (c == 1) nxt[0][r] = x[a][q];
       }
-      __syncthreads();
-      if (threadIdx.x < 32) {
-        const double p = cl[c];
-        if (!(p > 0.0) || !(p < 1.7e308)) {
-          if (threadIdx.x == 0) s_bad = 1;
-        } else if (threadIdx.x == 0) {
-          // 1/sqrt(p) with p = m 2^(2q), m in [1, 4)
-          const int e = ((__double2hiint(p) >> 20) - 1023) >> 1;
-          const double m = p * lm_pow2(-e) * lm_pow2(-e);
-          const double y = (double)rsqrtf((float)m);
-          const double h = fma(-m * y, y, 1.0);
-          const double r = fma(y * h, fma(h, 0.375, 0.5), y);
-          s_inv = r * lm_pow2(-e);
-          if (c < nb) dinv[(size_t)d * n + k0 + c] = s_inv;
-        }
+  }
+  if (threadIdx.x == 0) s_bad = 0;
+  __syncthreads();
+  double inv = 0.0;
+  auto pivot = [&](double p) {
+    const int hi = __double2hiint(p);  // not positive, infinite or not a number
+    if (hi < 0 || hi >= 0x7ff00000 || (hi | __double2loint(p)) == 0) {
+      if (threadIdx.x == 0) s_bad = 1;
+    } else {
+      inv = lm_rsqrt(p);
+    }
+  };
+  if (chain) pivot(col[0][0]);
+  // six columns at a time (one per thread column), so that which of a share's
+  // columns are left is known to the compiler
+#pragma unroll
+  for (int qc = 0; qc < PF_Q; qc++) {
+    for (int ct = 0; ct < PF_C; ct++) {
+      const int c = PF_C * qc + ct;
+      if (c >= LM_NB) break;
+      if (chain) {
+        scl[threadIdx.x] = col[c & 1][threadIdx.x] * inv;
+        scl[threadIdx.x + 32] = col[c & 1][threadIdx.x + 32] * inv;
       }
       __syncthreads();
       if (s_bad) {
         if (threadIdx.x == 0) bad[d] = 1;
         return;
       }
-      const double inv = s_inv;
-      double lr[4];
+      if (chain) {
+        if (threadIdx.x == 0) {
+          s_inv[c] = inv;
+          if (c < nb) dinv[(size_t)d * n + k0 + c] = inv;
+        }
+        if (c + 1 < LM_NB) {
+          const double l = scl[c + 1];
+          pivot(fma(-l, l, nxt[c & 1][c + 1]));
+        }
+      } else {
+        double lr[4];
 #pragma unroll
-      for (int a = 0; a < 4; a++) lr[a] = cl[tr + 16 * a] * inv;
-      if (tc == cb) {
+        for (int a = 0; a < 4; a++) lr[a] = scl[tr + 16 * a];
+        if (tc == ct) {
 #pragma unroll
-        for (int a = 0; a < 4; a++)
-          if (tr + 16 * a >= c) x[a][b] = lr[a];
+          for (int a = 0; a < 4; a++)
+            if (tr + 16 * a >= c) x[a][qc] = lr[a];
+        }
+        double* c1 = col[(c + 1) & 1] + tr;
+        double* c2 = nxt[(c + 1) & 1] + tr;
+#pragma unroll
+        for (int q = qc; q < PF_Q && q < qc + 2; q++) {  // the next two columns first
+          const int cc = tc + PF_C * q;
+          const double lc = (q > qc || tc > ct) && cc < LM_NB ? scl[min(cc, LM_NB - 1)] : 0.0;
+#pragma unroll
+          for (int a = 0; a < 4; a++)
+            if (16 * a + 15 >= PF_C * q) x[a][q] = fma(-lr[a], lc, x[a][q]);
+          if (cc == c + 1) {
+#pragma unroll
+            for (int a = 0; a < 4; a++) c1[16 * a] = x[a][q];
+          }
+          if (cc == c + 2) {
+#pragma unroll
+            for (int a = 0; a < 4; a++) c2[16 * a] = x[a][q];
+          }
+        }
+#pragma unroll
+        for (int q = qc + 2; q < PF_Q; q++) {
+          const int cc = tc + PF_C * q;
+          const double lc = cc < LM_NB ? scl[min(cc, LM_NB - 1)] : 0.0;
+#pragma unroll
+          for (int a = 0; a < 4; a++)  // rows above the diagonal of every column: none
+            if (16 * a + 15 >= PF_C * q) x[a][q] = fma(-lr[a], lc, x[a][q]);
+        }
       }
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const int cc = tc + 8 * q;
-        if (8 * q + 7 <= c) continue;  // no column of this share right of c
-        const double lc = cc > c ? cl[cc] * inv : 0.0;
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-          if (16 * a + 15 > c) x[a][q] = fma(-lr[a], lc, x[a][q]);
-      }
+      __syncthreads();  // the scaled column is consumed, the next published
     }
   }
+  if (chain) return;
+  double* lt = LT + (size_t)d * (LM_NB * LM_NB);
 #pragma unroll
   for (int a = 0; a < 4; a++)
 #pragma unroll
-    for (int b = 0; b < 8; b++) {
-      const int r = tr + 16 * a, c = tc + 8 * b;
-      if (r < nb && c <= r) A[(size_t)r * ld + c] = x[a][b];
+    for (int q = 0; q < PF_Q; q++) {
+      const int r = tr + 16 * a, c = tc + PF_C * q;
+      if (c >= LM_NB) continue;
+      const bool low = r < nb && c <= r;
+      if (low) A[(size_t)r * ld + c] = x[a][q];
+      lt[c * LM_NB + r] = low && c < r ? x[a][q] * s_inv[c] : 0.0;
     }
 }
 
-// Rows below the diagonal block (128 per block of threads, the right-hand row
+// Rows below the diagonal block (16 per block of threads, the right-hand row
 // last): X = A21 L11^-T in double, stored back, and the digits of X with a
-// scale per row.  Four lanes share a row (16 columns each), so that a warp's
-// FP64 instructions carry eight rows: with a thread per row a panel took one
-// warp's 2,000 FP64 instructions (64 us) however few rows were left.
-constexpr int TR_T = 512;
-constexpr size_t TR_SMEM = (size_t)(LM_NB * LM_NB + LM_NB + OZ_M * (LM_NB + 1)) * 8 + OZ_M * 4;
+// scale per row.  Eight lanes share a row (eight columns each): a warp's 350 FP64
+// instructions carry four rows (with a thread per row a panel took one warp's
+// 2,000 of them, 64 us, however few rows were left; with four lanes 32 us).
+constexpr int TR_L = 8;          // lanes of a row
+constexpr int TR_R = 16;         // rows of a block
+constexpr int TR_T = TR_L * TR_R;
+constexpr int TR_X = LM_NB / TR_L;
 __global__ void __launch_bounds__(TR_T)
     lm_trsm(int n, int k0, int nb, int ld, double* __restrict__ S, const double* __restrict__ dinv,
-            unsigned char* __restrict__ dig, size_t dig_stride, int* __restrict__ ex, int ex_stride,
-            const int* __restrict__ bad) {
-  extern __shared__ __align__(16) double tr_smem[];
+            const double* __restrict__ LT, unsigned char* __restrict__ dig, size_t dig_stride,
+            int* __restrict__ ex, int ex_stride, const int* __restrict__ bad) {
   const int d = blockIdx.y;
   if (bad[d]) return;
-  double* LT = tr_smem;               // [j][k] = L11[k][j]
-  double* inv = LT + LM_NB * LM_NB;   // 1 / L_jj
-  double* X = inv + LM_NB;            // [128][65]
-  int* se = reinterpret_cast<int*>(X + OZ_M * (LM_NB + 1));
+  __shared__ __align__(16) double lt[LM_NB * LM_NB];  // [j][k] = L_kj / L_jj
+  __shared__ double inv[LM_NB];                       // 1 / L_jj
+  __shared__ double X[TR_R][LM_NB + 1];
+  __shared__ int se[TR_R];
   double* base = S + (size_t)d * (n + 1) * ld;
-  const int r0 = k0 + nb + blockIdx.x * OZ_M;  // first row of this block
-  for (int t = threadIdx.x; t < LM_NB * LM_NB; t += TR_T) {
-    const int k = t / LM_NB, j = t % LM_NB;
-    LT[j * LM_NB + k] = (k < nb && j <= k) ? base[(size_t)(k0 + k) * ld + k0 + j] : 0.0;
+  const int r0 = k0 + nb + blockIdx.x * TR_R;  // first row of this block
+  {
+    const double2* src = reinterpret_cast<const double2*>(LT + (size_t)d * (LM_NB * LM_NB));
+    double2* dst = reinterpret_cast<double2*>(lt);
+#pragma unroll
+    for (int q = 0; q < LM_NB * LM_NB / 2 / TR_T; q++) dst[q * TR_T + threadIdx.x] = src[q * TR_T + threadIdx.x];
   }
-  for (int t = threadIdx.x; t < LM_NB; t += TR_T)
-    inv[t] = t < nb ? dinv[(size_t)d * n + k0 + t] : 1.0;
-  for (int t = threadIdx.x; t < OZ_M * LM_NB; t += TR_T) {
-    const int r = t / LM_NB, c = t % LM_NB;
-    X[r * (LM_NB + 1) + c] = (r0 + r <= n && c < nb) ? base[(size_t)(r0 + r) * ld + k0 + c] : 0.0;
+  if (threadIdx.x < LM_NB)
+    inv[threadIdx.x] = (int)threadIdx.x < nb ? dinv[(size_t)d * n + k0 + threadIdx.x] : 1.0;
+#pragma unroll
+  for (int q = 0; q < TR_R * LM_NB / TR_T; q++) {
+    const int t = q * TR_T + threadIdx.x, r = t / LM_NB, c = t % LM_NB;
+    X[r][c] = (r0 + r <= n && c < nb) ? base[(size_t)(r0 + r) * ld + k0 + c] : 0.0;
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, g = lane & 3;
-  const int row = (threadIdx.x >> 5) * 8 + (lane >> 2);
-  double x[16];
+  const int lane = threadIdx.x & 31, g = lane & (TR_L - 1);
+  const int row = threadIdx.x / TR_L;
+  double x[TR_X];
 #pragma unroll
-  for (int m = 0; m < 16; m++) x[m] = X[row * (LM_NB + 1) + 4 * m + g];
+  for (int m = 0; m < TR_X; m++) x[m] = X[row][TR_L * m + g];
 #pragma unroll
-  for (int m = 0; m < 16; m++) {
+  for (int m = 0; m < TR_X; m++) {
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int j = 4 * m + q;  // held by lane group q
-      const double xj = __shfl_sync(0xffffffffu, x[m] * inv[j], (lane & ~3) | q);
-      if (g == q) x[m] = xj;
-      const double* l = LT + j * LM_NB + g;
-      if (g > q) x[m] = fma(-xj, l[4 * m], x[m]);
+    for (int q = 0; q < TR_L; q++) {
+      // x_j before its division by L_jj (lt holds the division): the chain from
+      // column to column is a shuffle and one FMA
+      const double xj = __shfl_sync(0xffffffffu, x[m], (lane & ~(TR_L - 1)) | q);
+      const double* l = lt + (TR_L * m + q) * LM_NB + g;
+      x[m] = fma(-xj, l[TR_L * m], x[m]);  // (zero for columns up to j)
 #pragma unroll
-      for (int w = m + 1; w < 16; w++) x[w] = fma(-xj, l[4 * w], x[w]);
+      for (int w = m + 1; w < TR_X; w++) x[w] = fma(-xj, l[TR_L * w], x[w]);
     }
   }
   unsigned hw = 0;
 #pragma unroll
-  for (int m = 0; m < 16; m++) {
-    X[row * (LM_NB + 1) + 4 * m + g] = x[m];
+  for (int m = 0; m < TR_X; m++) {
+    x[m] *= inv[TR_L * m + g];
+    X[row][TR_L * m + g] = x[m];
     hw = max(hw, (unsigned)__double2hiint(x[m]) & 0x7fffffffu);
   }
   hw = max(hw, __shfl_xor_sync(0xffffffffu, hw, 1));
   hw = max(hw, __shfl_xor_sync(0xffffffffu, hw, 2));
+  hw = max(hw, __shfl_xor_sync(0xffffffffu, hw, 4));
   if (g == 0) {
     // not finite: the digits are zero and the diagonal this row updates stays
     // what it is; the entries themselves keep the value for the finish
     const int e = (hw >> 20) >= 2047u ? 1 << 20 : oz_exp(hw);
     se[row] = e;
-    ex[(size_t)d * ex_stride + blockIdx.x * OZ_M + row] = e == 1 << 20 ? 0 : e;
+    ex[(size_t)d * ex_stride + blockIdx.x * TR_R + row] = e == 1 << 20 ? 0 : e;
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < OZ_M * LM_NB; t += TR_T) {
-    const int r = t / LM_NB, c = t % LM_NB;
-    if (r0 + r <= n && c < nb) base[(size_t)(r0 + r) * ld + k0 + c] = X[r * (LM_NB + 1) + c];
+#pragma unroll
+  for (int q = 0; q < TR_R * LM_NB / TR_T; q++) {
+    const int t = q * TR_T + threadIdx.x, r = t / LM_NB, c = t % LM_NB;
+    if (r0 + r <= n && c < nb) base[(size_t)(r0 + r) * ld + k0 + c] = X[r][c];
   }
-  unsigned char* out = dig + d * dig_stride + (size_t)blockIdx.x * 2 * OZ_CHUNK;
-  for (int u = threadIdx.x; u < OZ_M * 8; u += TR_T) {
-    const int i = u & (OZ_M - 1), k8 = u / OZ_M;
-    const bool ok = se[i] != 1 << 20;
-    const double sc = ok ? lm_pow2(56 - se[i]) : 0.0;
-    oz_put8(out + (k8 >> 2) * OZ_CHUNK, k8 & 3, i, sc,
-            [&](int k) { return ok ? X[i * (LM_NB + 1) + 8 * k8 + k] : 0.0; });
-  }
+  constexpr int SUB = OZ_M / TR_R;  // blocks of threads per row block of digits
+  unsigned char* out = dig + d * dig_stride + (size_t)(blockIdx.x / SUB) * 2 * OZ_CHUNK;
+  const int sub = (blockIdx.x % SUB) * TR_R;
+  static_assert(TR_T == TR_R * 8, "a thread per row and eight columns");
+  const int i = threadIdx.x & (TR_R - 1), k8 = threadIdx.x / TR_R;
+  const bool ok = se[i] != 1 << 20;
+  const double sc = ok ? lm_pow2(56 - se[i]) : 0.0;
+  oz_put8(out + (k8 >> 2) * OZ_CHUNK, k8 & 3, sub + i, sc,
+          [&](int k) { return ok ? X[i][8 * k8 + k] : 0.0; });
 }
 
 // One block of up to 64 unknowns of L^T x = y, from the last: every block of
 // threads solves the triangle (one warp), the first stores it, and each takes
-// 64 of the rows above, y -= L21^T x.  y is the system's row n.
-__global__ void __launch_bounds__(64)
+// 64 of the rows above, y -= L21^T x, four threads to a row.  y is the system's
+// row n.  As in lm_trsm the triangle carries the divisions, so that the chain
+// is a shuffle and one FMA per unknown.
+constexpr int BK_T = 256;
+__global__ void __launch_bounds__(BK_T)
     lm_backstep(int n, int b0, int nb, int ld, double* __restrict__ S,
                 const double* __restrict__ dinv, double* __restrict__ x,
                 const int* __restrict__ bad) {
   const int d = blockIdx.y;
   if (bad[d]) return;
-  __shared__ double L[LM_NB][LM_NB + 1];
+  __shared__ double L[LM_NB][LM_NB + 1];  // [i][c] = L_ic / L_ii
   __shared__ double sx[LM_NB];
+  __shared__ double red[4][64];
   double* base = S + (size_t)d * (n + 1) * ld;
   double* y = base + (size_t)n * ld;
-  for (int t = threadIdx.x; t < LM_NB * LM_NB; t += 64) {
+  const double* di = dinv + (size_t)d * n + b0;
+  for (int t = threadIdx.x; t < LM_NB * LM_NB; t += BK_T) {
     const int r = t / LM_NB, c = t % LM_NB;
-    L[r][c] = (r < nb && c < r) ? base[(size_t)(b0 + r) * ld + b0 + c] : 0.0;
+    L[r][c] = (r < nb && c < r) ? base[(size_t)(b0 + r) * ld + b0 + c] * di[r] : 0.0;
   }
-  const double inv = (int)threadIdx.x < nb ? dinv[(size_t)d * n + b0 + threadIdx.x] : 0.0;
-  sx[threadIdx.x] = inv;
+  // the rows above: loads in flight during the triangle
+  const int part = threadIdx.x >> 6, r = blockIdx.x * 64 + (threadIdx.x & 63);
+  double l[16];
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+    const int i = 16 * part + q;
+    l[q] = (r < b0 && i < nb) ? base[(size_t)(b0 + i) * ld + r] : 0.0;
+  }
   __syncthreads();
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     double ya = lane < nb ? y[b0 + lane] : 0.0, yb = lane + 32 < nb ? y[b0 + 32 + lane] : 0.0;
-    const double ia = sx[lane], ib = sx[lane + 32];
+#pragma unroll 4
     for (int i = LM_NB - 1; i >= 32; i--) {
-      const double xi = __shfl_sync(0xffffffffu, yb * ib, i - 32);
-      ya = fma(-L[i][lane], xi, ya);
-      if (lane + 32 < i) yb = fma(-L[i][lane + 32], xi, yb);
+      const double yi = __shfl_sync(0xffffffffu, yb, i - 32);
+      yb = fma(-L[i][lane + 32], yi, yb);  // (zero from the diagonal on)
+      ya = fma(-L[i][lane], yi, ya);
     }
-    for (int i = 31; i >= 0; i--) {
-      const double xi = __shfl_sync(0xffffffffu, ya * ia, i);
-      if (lane < i) ya = fma(-L[i][lane], xi, ya);
-    }
-    sx[lane] = ya * ia;
-    sx[lane + 32] = yb * ib;
+#pragma unroll 4
+    for (int i = 31; i >= 0; i--) ya = fma(-L[i][lane], __shfl_sync(0xffffffffu, ya, i), ya);
+    sx[lane] = lane < nb ? ya * di[lane] : 0.0;
+    sx[lane + 32] = lane + 32 < nb ? yb * di[lane + 32] : 0.0;
   }
   __syncthreads();
   if (blockIdx.x == 0 && (int)threadIdx.x < nb) x[(size_t)d * n + b0 + threadIdx.x] = sx[threadIdx.x];
-  const int r = blockIdx.x * 64 + threadIdx.x;
-  if (r >= b0) return;
   double s = 0.0;
-#pragma unroll 8
-  for (int i = 0; i < nb; i++) s = fma(base[(size_t)(b0 + i) * ld + r], sx[i], s);
-  y[r] -= s;
+#pragma unroll
+  for (int q = 0; q < 16; q++) s = fma(l[q], sx[16 * part + q], s);
+  red[part][threadIdx.x & 63] = s;
+  __syncthreads();
+  if (part == 0 && r < b0)
+    y[r] -= (red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x]);
 }
 
 // ---- the systems that are not positive definite: LU with partial pivoting --------
@@ -1021,7 +1215,8 @@ extern "C" int ztm_lm_steps(ztm_ctx* c, const double* J, int nrows, int ncols, c
                       3 * WsCarver::need(n * 8) + WsCarver::need((size_t)s.slices * n * n * 8) +
                       WsCarver::need((size_t)nd * (n + 1) * ld * 8) + WsCarver::need(dig) +
                       WsCarver::need((size_t)nd * prb * OZ_M * 4) + 3 * WsCarver::need((size_t)nd * 8) +
-                      WsCarver::need((size_t)nd * n * 4) + 16384;
+                      WsCarver::need((size_t)nd * n * 4) + WsCarver::need((size_t)nd * LM_NB * LM_NB * 8) +
+                      16384;
   int rc = ztm_ws_reserve(c, need);
   if (rc) return rc;
   WsCarver wc(c->ws);
@@ -1035,6 +1230,7 @@ extern "C" int ztm_lm_steps(ztm_ctx* c, const double* J, int nrows, int ncols, c
   double* x = wc.take<double>((size_t)nd * n);
   double* g = wc.take<double>(n);
   double* dinv = wc.take<double>((size_t)nd * n);
+  double* LT = wc.take<double>((size_t)nd * LM_NB * LM_NB);
   double* pdot = wc.take<double>((size_t)nstat * n);
   unsigned* pmax = wc.take<unsigned>((size_t)nstat * n);
   int* ex = wc.take<int>(n);
@@ -1058,13 +1254,12 @@ extern "C" int ztm_lm_steps(ztm_ctx* c, const double* J, int nrows, int ncols, c
   cudaMemsetAsync(state, 0, (2 * (size_t)nd + 1) * 4, c->stream);
   cudaFuncSetAttribute(oz_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OZ_SMEM);
   cudaFuncSetAttribute(oz_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OZ_SMEM);
-  cudaFuncSetAttribute(lm_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TR_SMEM);
   long long launches = 0;
   {
     ZtmProf prof_(c, "lm");
     lm_colstat<<<dim3((unsigned)((n + 127) / 128), nstat), 128, 0, c->stream>>>(
         (const double*)pJ, nrows, ncols, (const double*)pr, pmax, pdot);
-    lm_colfinish<<<(unsigned)((n + 127) / 128), 128, 0, c->stream>>>(ncols, nstat, pmax, pdot, ex,
+    lm_colfinish<<<(unsigned)((n + 31) / 32), 256, 0, c->stream>>>(ncols, nstat, pmax, pdot, ex,
                                                                      odd, g);
     OzArgs o = {};
     o.dig = digits;
@@ -1080,7 +1275,9 @@ extern "C" int ztm_lm_steps(ztm_ctx* c, const double* J, int nrows, int ncols, c
       const int slices = (o.nkc + s.per - 1) / s.per;
       lm_slice<<<dim3(s.rb, o.nkc), 256, 0, c->stream>>>((const double*)pJ, k * OZ_KC, nrows, ncols,
                                                          ex, odd, digits);
-      oz_kernel<0><<<dim3(s.tiles, slices), OZ_T, OZ_SMEM, c->stream>>>(o);
+      o.tiles = s.tiles;
+      o.work = s.tiles * slices;
+      oz_kernel<0><<<std::min(o.work, std::max(c->num_sms, 1)), OZ_T, OZ_SMEM, c->stream>>>(o);
       const unsigned t32 = (unsigned)((n + 31) / 32);
       lm_reduce<<<dim3(t32, t32), 256, 0, c->stream>>>(ncols, slices, part, odd, k > 0, oJJ);
       launches += 3;
@@ -1102,20 +1299,23 @@ extern "C" int ztm_lm_steps(ztm_ctx* c, const double* J, int nrows, int ncols, c
     u.bad = bad;
     for (int k0 = 0; k0 < ncols; k0 += LM_NB) {
       const int nb = std::min(LM_NB, ncols - k0);
-      lm_potrf<<<nd, 128, 0, c->stream>>>(ncols, k0, nb, ld, S, dinv, bad);
+      lm_potrf<<<nd, PF_T, 0, c->stream>>>(ncols, k0, nb, ld, S, dinv, LT, bad);
       const int rows = ncols + 1 - (k0 + nb), rb = (rows + OZ_M - 1) / OZ_M;
-      lm_trsm<<<dim3(rb, nd), TR_T, TR_SMEM, c->stream>>>(ncols, k0, nb, ld, S, dinv, digits,
-                                                          dig_stride, pex, u.exp_stride, bad);
+      // whole row blocks of digits: the rows past the last are zeros
+      lm_trsm<<<dim3(rb * (OZ_M / TR_R), nd), TR_T, 0, c->stream>>>(
+          ncols, k0, nb, ld, S, dinv, LT, digits, dig_stride, pex, u.exp_stride, bad);
       launches += 2;
       if (rows > 1) {
         u.n = rows;
         u.r0 = k0 + nb;
-        oz_kernel<1><<<dim3(rb * (rb + 1), nd), OZ_T, OZ_SMEM, c->stream>>>(u);
+        u.tiles = rb * (rb + 1);
+        u.work = u.tiles * nd;
+        oz_kernel<1><<<std::min(u.work, std::max(c->num_sms, 1)), OZ_T, OZ_SMEM, c->stream>>>(u);
         launches++;
       }
     }
     for (int b0 = ((ncols - 1) / LM_NB) * LM_NB; b0 >= 0; b0 -= LM_NB) {
-      lm_backstep<<<dim3(std::max(1, b0 / 64), nd), 64, 0, c->stream>>>(
+      lm_backstep<<<dim3(std::max(1, b0 / 64), nd), BK_T, 0, c->stream>>>(
           ncols, b0, std::min(LM_NB, ncols - b0), ld, S, dinv, x, bad);
       launches++;
     }
