@@ -25,6 +25,7 @@
 
 #include <algorithm>
 
+#include "pm64.cuh"
 #include "ztm_internal.cuh"
 
 namespace {
@@ -250,6 +251,68 @@ __global__ void __launch_bounds__(PMA_TB)
   }
 }
 
+// Double, by levels (pm64.cuh): a block takes 128 selected nodes of one level
+// (the launch has blocks for full levels; those past a level's nodes end) and
+// a slice of the stations, 128 at a time in shared memory with this level's
+// z^2 and w dz.  A pair is two integer products, two FP64 instructions and
+// pm_cube_rsqrt.
+constexpr int P64_T = 128;
+__global__ void __launch_bounds__(P64_T, 8)
+    pma64_gather_kernel(PmParams p, const Pm64Node* __restrict__ node, const int* __restrict__ row,
+                        const double* __restrict__ surf, const double* __restrict__ w, int pblocks,
+                        int slice, long long pstride, double* __restrict__ partial) {
+  __shared__ double2 s_z[P64_T];  // z^2, w dz
+  __shared__ int2 s_ij[P64_T];    // the station's fine-grid i, j
+  const int k = (int)(blockIdx.x / pblocks) % p.kk, sl = (int)(blockIdx.x / pblocks) / p.kk;
+  const int e0 = row[(long long)k * p.jj] + (int)(blockIdx.x % pblocks) * P64_T;
+  const int e1 = row[(long long)(k + 1) * p.jj];
+  if (e0 >= e1) return;  // uniform
+  const int e = e0 + threadIdx.x;
+  const Pm64Node v = node[min(e, e1 - 1)];
+  const int xi = v.i, yj = (v.n / p.ii) % p.jj;
+  const int s0 = sl * slice, s1 = min(p.ns, s0 + slice);
+  double acc = 0.0;
+  for (int t0 = s0; t0 < s1; t0 += P64_T) {
+    __syncthreads();
+    {
+      const int s = t0 + threadIdx.x;
+      double2 z = make_double2(1.0, 0.0);  // past the slice: no weight
+      int2 ij = make_int2(0, 0);
+      if (s < s1) {
+        const int ci = p.bfr + s % p.ni, cj = p.bfr + s / p.ni, m = ci + cj * p.di;
+        const double dz = p.fh * (surf[m] - k * (1.0 / p.fv));
+        z = make_double2(dz * dz, w[m] * dz);
+        ij = make_int2(ci * p.fh, cj * p.fh);
+      }
+      s_z[threadIdx.x] = z;
+      s_ij[threadIdx.x] = ij;
+    }
+    __syncthreads();
+    const int cnt = min(P64_T, s1 - t0);
+#pragma unroll 2
+    for (int q = 0; q < cnt; q++) {
+      const double2 z = s_z[q];
+      const int2 ij = s_ij[q];
+      const int dx = ij.x - xi, dy = ij.y - yj;
+      acc = fma(z.y, pm_cube_rsqrt(z.x + pm_int_double((uint32_t)(dx * dx + dy * dy))), acc);
+    }
+  }
+  if (e < e1) partial[sl * pstride + e] = acc;
+}
+
+// g[n] = factor * sel(n) * sum over slices, for every selected node.
+__global__ void pma64_finalize(PmParams p, const Pm64Node* __restrict__ node,
+                               const int* __restrict__ total, const double* __restrict__ partial,
+                               int nslices, long long pstride, double factor,
+                               double* __restrict__ out) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= *total) return;
+  const Pm64Node v = node[t];
+  double s = 0.0;
+  for (int sl = 0; sl < nslices; sl++) s += partial[sl * pstride + t];
+  out[v.n] = factor * v.w * s;  // w: the node's multiplicity
+}
+
 // g[col + k*ncols] = factor * sel(n) * sum over slices, for every group level.
 template <int LV>
 __global__ void pma_finalize(PmParams p, const int* __restrict__ n_groups,
@@ -365,10 +428,32 @@ PmaShape pma_shape(const PmParams& p, bool f64, int num_sms) {
   return s;
 }
 
+// The double path by levels: offsets whose squares add up within 31 bits.
+bool pma64_use(const PmParams& p) {
+  return p.ii <= PM64_MAX_OFF && p.jj <= PM64_MAX_OFF && (long long)p.kk * p.jj < (1LL << 28);
+}
+// Blocks per level, and station slices of whole tiles: about four blocks for
+// each that is resident at once.
+void pma64_shape(const PmParams& p, int num_sms, int* pblocks, int* slices, int* slice) {
+  *pblocks = (int)(((long long)p.ii * p.jj + P64_T - 1) / P64_T);
+  const long long base = (long long)*pblocks * p.kk;
+  const int tiles = std::max(1, (p.ns + P64_T - 1) / P64_T);
+  const long long want = std::max(1LL, (32LL * std::max(num_sms, 1) + base - 1) / base);
+  const int per = (int)std::max(1LL, (tiles + want - 1) / want);
+  *slice = per * P64_T;
+  *slices = (tiles + per - 1) / per;
+}
+
 }  // namespace
 
 size_t ztm_pm_adjoint_ws(const PmParams& p, int precision, int num_sms, bool list) {
   const bool f64 = precision == ZTM_PREC_FP64;
+  if (f64 && pma64_use(p)) {
+    int pb, slices, slice;
+    pma64_shape(p, num_sms, &pb, &slices, &slice);
+    return ztm_pm64_list_ws(p) + WsCarver::need((size_t)slices * p.N * sizeof(double)) +
+           (list ? WsCarver::need((size_t)p.N * sizeof(int)) : 0);
+  }
   const PmaShape s = pma_shape(p, f64, num_sms);
   const int LV = f64 ? PmaT<true>::LV : PmaT<false>::LV;
   const long long ncols = (long long)p.ii * p.jj;
@@ -384,6 +469,33 @@ int ztm_launch_pm_adjoint(ztm_ctx* c, const PmParams& p, const double* d_drho, c
                           const double* d_surf, const double* d_w, double* d_g, double scale,
                           int precision, WsCarver& wc) {
   const bool f64 = precision == ZTM_PREC_FP64;
+  if (f64 && pma64_use(p)) {
+    cudaMemsetAsync(d_g, 0, (size_t)p.N * sizeof(double), c->stream);
+    if (p.ns == 0 || p.nnodes == 0) return ztm_after_launch(c, "point-mass adjoint");
+    int pblocks, slices, slice;
+    pma64_shape(p, c->num_sms, &pblocks, &slices, &slice);
+    double* partial = wc.take<double>((size_t)slices * p.N);
+    int* mult = nullptr;
+    if (d_nn) {
+      mult = wc.take<int>((size_t)p.N);
+      cudaMemsetAsync(mult, 0, (size_t)p.N * sizeof(int), c->stream);
+      pma_mark<<<(unsigned)((p.nnodes + 255) / 256), 256, 0, c->stream>>>(p.nnodes, p.N, d_nn, mult,
+                                                                          c->d_err);
+      c->launches++;
+    }
+    Pm64List list;
+    ztm_pm64_list(c, p, d_drho, mult, true, wc, &list);
+    {
+      ZtmProf prof_(c, "pointmass_adjoint");
+      pma64_gather_kernel<<<(unsigned)((long long)pblocks * p.kk * slices), P64_T, 0, c->stream>>>(
+          p, list.node, list.row, d_surf, d_w, pblocks, slice, p.N, partial);
+    }
+    // fine-grid lengths: dz / r^3 is fh^2 times smaller there
+    pma64_finalize<<<(unsigned)((p.N + 255) / 256), 256, 0, c->stream>>>(
+        p, list.node, list.row + p.kk * p.jj, partial, slices, p.N, scale * 66.7 / p.fv, d_g);
+    c->launches += 2;
+    return ztm_after_launch(c, "point-mass adjoint");
+  }
   const PmaShape s = pma_shape(p, f64, c->num_sms);
   const int LV = f64 ? PmaT<true>::LV : PmaT<false>::LV;
   const long long ncols = (long long)p.ii * p.jj;

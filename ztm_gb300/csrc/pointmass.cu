@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "pm64.cuh"
 #include "ztm_internal.cuh"
 
 namespace {
@@ -477,9 +478,7 @@ __global__ void __launch_bounds__(PM_TS)
   if (active) partial[(long long)blockIdx.y * p.ns + s] = acc.value();
 }
 
-// Double path by node columns: the same layout one node per entry,
-// (-k, w) in double, each column's (-i, -j) in double; per node the gather
-// forms Z, r^2 = Z^2 + (X^2 + Y^2), the rsqrt and the product in double.
+// Weight of node n in the double sums, 0 when it is not selected.
 __device__ __forceinline__ double pm_col_weight64(const PmParams& p,
                                                   const double* __restrict__ drho,
                                                   const int* __restrict__ mult, long long n) {
@@ -491,81 +490,119 @@ __device__ __forceinline__ double pm_col_weight64(const PmParams& p,
   return fabs(w) > p.thr ? w : 0.0;
 }
 
-__global__ void pm_cols_count64(PmParams p, const double* __restrict__ drho,
-                                const int* __restrict__ mult, int* __restrict__ counts,
-                                double2* __restrict__ colxy) {
-  const long long ncols = (long long)p.ii * p.jj;
-  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (c >= ncols) return;
-  const long long ni = c % p.ii, nj = c / p.ii;
-  colxy[c] = make_double2(-(ni * (1.0 / p.fh)), -(nj * (1.0 / p.fh)));
+// Double path (the context entry points): level by level over the selected
+// nodes in node order (pm64.cuh).  pm64_rows_count / a scan / pm64_rows_write:
+// a warp per row (k, j).  pm64_gather_kernel: a block takes 128 stations, one
+// level and a range of its rows; the rows' nodes stream through shared memory,
+// X^2 from a table of squares (lane: station), Y^2 + z^2 once per row.
+// ADJ: the adjoint's selection (a node's multiplicity, the threshold, or all).
+template <bool ADJ>
+__device__ __forceinline__ double pm64_weight(const PmParams& p, const double* __restrict__ drho,
+                                              const int* __restrict__ mult, long long n) {
+  if (!ADJ) return pm_col_weight64(p, drho, mult, n);
+  if (mult) return (double)mult[n];
+  if (drho) return fabs(drho[n]) > p.thr ? 1.0 : 0.0;
+  return 1.0;
+}
+
+template <bool ADJ>
+__global__ void __launch_bounds__(128)
+    pm64_rows_count(PmParams p, const double* __restrict__ drho, const int* __restrict__ mult,
+                    int* __restrict__ row) {
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= p.kk * p.jj) return;
   int cnt = 0;
-  for (int k = 0; k < p.kk; k++)
-    if (pm_col_weight64(p, drho, mult, c + k * ncols) != 0.0) cnt++;
-  counts[c] = cnt;
+  for (int i = lane; i < p.ii; i += 32)
+    cnt += pm64_weight<ADJ>(p, drho, mult, (long long)r * p.ii + i) != 0.0;
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if (lane == 0) row[r] = cnt;
 }
 
-__global__ void pm_cols_write64(PmParams p, const double* __restrict__ drho,
-                                const int* __restrict__ mult, const int* __restrict__ offs,
-                                double2* __restrict__ nodes) {
-  const long long ncols = (long long)p.ii * p.jj;
-  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (c >= ncols) return;
-  double2* out = nodes + offs[c];
-  int q = 0;
-  for (int k = 0; k < p.kk; k++) {
-    const double w = pm_col_weight64(p, drho, mult, c + k * ncols);
-    if (w != 0.0) out[q++] = make_double2(-(k * (1.0 / p.fv)), w);
-  }
-}
-
-__global__ void __launch_bounds__(PM_TS)
-    pm_gather_cols64_kernel(PmParams p, const double2* __restrict__ nodes,
-                            const int* __restrict__ offs, const double2* __restrict__ colxy,
-                            const double* __restrict__ surf, int cg_cols, int chunk_cols,
-                            double* __restrict__ partial) {
-  __shared__ double2 tile[PM_CT];
-  __shared__ int s_off[PM_CT + 1];
-  __shared__ double2 s_xy[PM_CT];
-  const int s = blockIdx.x * PM_TS + threadIdx.x;
-  const bool active = s < p.ns;
-  double i0 = 0.0, j0 = 0.0, k0 = 0.0;
-  if (active) {
-    const int si = p.bfr + s % p.ni, sj = p.bfr + s / p.ni;
-    i0 = (double)si;
-    j0 = (double)sj;
-    k0 = surf[si + sj * p.di];
-  }
-  const int ncols = p.ii * p.jj;
-  const int c0 = blockIdx.y * chunk_cols, c1 = min(ncols, c0 + chunk_cols);
-  double acc = 0.0;
-  for (int cg = c0; cg < c1; cg += cg_cols) {
-    const int ce = min(c1, cg + cg_cols);
-    __syncthreads();  // the previous group is consumed
-    for (int q = threadIdx.x; q <= ce - cg; q += PM_TS) {
-      s_off[q] = offs[cg + q];
-      if (q < ce - cg) s_xy[q] = colxy[cg + q];
+template <bool ADJ>
+__global__ void __launch_bounds__(128)
+    pm64_rows_write(PmParams p, const double* __restrict__ drho, const int* __restrict__ mult,
+                    const int* __restrict__ row, Pm64Node* __restrict__ node) {
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= p.kk * p.jj) return;
+  int o = row[r];
+  for (int i0 = 0; i0 < p.ii; i0 += 32) {
+    const int i = i0 + lane;
+    const long long n = (long long)r * p.ii + i;
+    const double w = i < p.ii ? pm64_weight<ADJ>(p, drho, mult, n) : 0.0;
+    const unsigned bal = __ballot_sync(0xffffffffu, w != 0.0);
+    if (w != 0.0) {
+      Pm64Node v;
+      v.w = w;
+      v.i = i;
+      v.n = (int)n;
+      node[o + __popc(bal & ((1u << lane) - 1u))] = v;
     }
+    o += __popc(bal);
+  }
+}
+
+constexpr int PM64_TILE = 256;  // nodes per shared-memory tile
+__global__ void __launch_bounds__(PM_TS, 8)
+    pm64_gather_kernel(PmParams p, const Pm64Node* __restrict__ node, const int* __restrict__ row,
+                       const double* __restrict__ surf, int tiles, int chunk_rows,
+                       double* __restrict__ partial) {
+  __shared__ Pm64Node tile[PM64_TILE];
+  extern __shared__ double pm64_smem[];
+  double* sq = pm64_smem;                                // d^2, d = 0 .. ii - 1
+  int* s_row = reinterpret_cast<int*>(pm64_smem + p.ii);  // offsets of this block's rows
+  const int k = (int)(blockIdx.x / tiles) % p.kk, chunk = (int)(blockIdx.x / tiles) / p.kk;
+  const int s = (int)(blockIdx.x % tiles) * PM_TS + threadIdx.x;
+  const int j0 = chunk * chunk_rows, j1 = min(p.jj, j0 + chunk_rows);
+  for (int t = threadIdx.x; t < p.ii; t += PM_TS) sq[t] = (double)t * t;
+  for (int t = threadIdx.x; t <= j1 - j0; t += PM_TS) s_row[t] = row[(long long)k * p.jj + j0 + t];
+  // threads past the last station repeat it
+  const int sc = min(s, p.ns - 1), ci = p.bfr + sc % p.ni, cj = p.bfr + sc / p.ni;
+  const int xi = ci * p.fh, yj = cj * p.fh;  // in fine-grid steps
+  const double dz = p.fh * (surf[ci + cj * p.di] - k * (1.0 / p.fv));
+  const double z2 = dz * dz;
+  __syncthreads();
+  const int e0 = s_row[0], e1 = s_row[j1 - j0];
+  double acc = 0.0;
+  int j = j0;
+  for (int t0 = e0; t0 < e1; t0 += PM64_TILE) {
+    const int cnt = min(PM64_TILE, e1 - t0);
     __syncthreads();
-    const int p0 = s_off[0], nnode = s_off[ce - cg] - p0;  // <= PM_CT (host)
-    for (int q = threadIdx.x; q < nnode; q += PM_TS) tile[q] = nodes[p0 + q];
+    for (int q = threadIdx.x; q < cnt; q += PM_TS) tile[q] = node[t0 + q];
     __syncthreads();
-    if (!active) continue;
-    for (int c = cg; c < ce; c++) {
-      const int a = s_off[c - cg] - p0, b = s_off[c - cg + 1] - p0;
-      const double2 xy = s_xy[c - cg];
-      const double X = i0 + xy.x, Y = j0 + xy.y;
-      const double rh = X * X + Y * Y;
-#pragma unroll 4
-      for (int q = a; q < b; q++) {
-        const double2 v = tile[q];  // (-k, w)
-        const double dz = k0 + v.x;
-        const double rs = rsqrt(dz * dz + rh);
-        acc += v.y * dz * (rs * rs * rs);
+    for (int q = 0; q < cnt;) {
+      while (s_row[j + 1 - j0] <= t0 + q) j++;
+      const int qe = min(cnt, s_row[j + 1 - j0] - t0), dy = yj - j;
+      const double zy = z2 + (double)dy * dy;
+#pragma unroll 2
+      for (; q < qe; q++) {
+        const Pm64Node v = tile[q];
+        acc = fma(v.w, pm_cube_rsqrt(zy + sq[abs(xi - v.i)]), acc);
       }
     }
   }
-  if (active) partial[(long long)blockIdx.y * p.ns + s] = acc;
+  if (s < p.ns) partial[(long long)(chunk * p.kk + k) * p.ns + s] = acc * dz;
+}
+
+// G[m] = factor * sum of the n partial sums for interior m, 0 elsewhere: 32
+// grid nodes a block, eight threads each, in a fixed order.
+__global__ void __launch_bounds__(256)
+    pm64_finalize_kernel(PmParams p, int n, const double* __restrict__ partial, double factor,
+                         double* __restrict__ G) {
+  __shared__ double sm[8][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, m = blockIdx.x * 32 + x;
+  const int i0 = m % p.di, j0 = m / p.di;
+  const bool in = m < p.di * p.dj && i0 >= p.bfr && i0 < p.di - p.bfr && j0 >= p.bfr && j0 < p.dj - p.bfr;
+  double g = 0.0;
+  if (in) {
+    const int s = (i0 - p.bfr) + (j0 - p.bfr) * p.ni;
+    for (int c = y; c < n; c += 8) g += partial[(long long)c * p.ns + s];
+  }
+  sm[y][x] = g;
+  __syncthreads();
+  if (y || m >= p.di * p.dj) return;
+#pragma unroll
+  for (int q = 1; q < 8; q++) g += sm[q][x];
+  G[m] = in ? g * factor : 0.0;
 }
 
 // G[m] = factor * sum_chunks partial for interior m, 0 elsewhere.
@@ -590,9 +627,7 @@ __global__ void pm_finalize_kernel(PmParams p, int nchunks,
 int pm_occupancy(int precision, bool compacted, bool cols = false) {
   int occ = 0;
   cudaError_t e;
-  if (precision == ZTM_PREC_FP64 && cols)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pm_gather_cols64_kernel, PM_TS, 0);
-  else if (precision == ZTM_PREC_FP64)
+  if (precision == ZTM_PREC_FP64)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pm_gather_kernel<true>, PM_TS, 0);
   else if (cols)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pm_gather_cols_kernel, PM_TS, 0);
@@ -626,21 +661,35 @@ void pm_shape(const PmParams& p, int num_sms, int occ, int* tiles, int* chunks, 
   *clen = len;
 }
 
-// Entries of one column's run: node pairs (float) or nodes (double).
-int pm_col_entries(const PmParams& p, bool f64) { return f64 ? p.kk : (p.kk + 1) / 2; }
-// The column path: a column's run fits one shared-memory tile.
-bool pm_use_cols(const PmParams& p, bool f64 = false) { return pm_col_entries(p, f64) <= PM_CT; }
+// Node pairs of one column's run (float), and the column path's condition: a
+// column's run fits one shared-memory tile.
+int pm_col_entries(const PmParams& p) { return (p.kk + 1) / 2; }
+bool pm_use_cols(const PmParams& p) { return pm_col_entries(p) <= PM_CT; }
+// The double path by levels: its table of squares fits, and the levels x station
+// tiles x row ranges of its grid.
+bool pm64_use(const PmParams& p) {
+  return p.ii <= PM64_MAX_II && (long long)p.kk * p.jj < (1LL << 28) &&
+         (long long)p.kk * std::max(1, (p.ns + PM_TS - 1) / PM_TS) < (1LL << 30);
+}
+// Row ranges per level: about four blocks for each that is resident at once.
+void pm64_shape(const PmParams& p, int num_sms, int* tiles, int* chunks, int* chunk_rows) {
+  *tiles = std::max(1, (p.ns + PM_TS - 1) / PM_TS);
+  const long long base = (long long)*tiles * p.kk;
+  const long long want = std::max(1LL, (32LL * std::max(num_sms, 1) + base - 1) / base);
+  *chunk_rows = (int)std::max(std::min(4LL, (long long)p.jj), (p.jj + want - 1) / want);
+  *chunks = (p.jj + *chunk_rows - 1) / *chunk_rows;
+}
 
 // Column gather shape: station tiles x column chunks of whole column groups
 // (cg_cols columns, at most PM_CT pairs), about sixteen waves of resident
 // blocks (62.4 ms at four waves, 61.2 at eight, 60.7 at sixteen on the
 // 256x256x65-node grid).
-void pm_cols_shape(const PmParams& p, int num_sms, bool f64, int* tiles, int* chunks,
-                   int* chunk_cols, int* cg_cols) {
-  const int occ = pm_occupancy(f64 ? ZTM_PREC_FP64 : ZTM_PREC_FP32, true, true);
+void pm_cols_shape(const PmParams& p, int num_sms, int* tiles, int* chunks, int* chunk_cols,
+                   int* cg_cols) {
+  const int occ = pm_occupancy(ZTM_PREC_FP32, true, true);
   *tiles = std::max(1, (p.ns + PM_TS - 1) / PM_TS);
   const long long ncols = (long long)p.ii * p.jj;
-  *cg_cols = std::max(1, PM_CT / std::max(1, pm_col_entries(p, f64)));
+  *cg_cols = std::max(1, PM_CT / std::max(1, pm_col_entries(p)));
   const long long want = std::max(1LL, (16LL * occ * std::max(num_sms, 1) + *tiles - 1) / *tiles);
   const long long groups = (ncols + *cg_cols - 1) / *cg_cols;
   const long long ch = std::max(1LL, std::min(std::min(want, groups), 65535LL));
@@ -655,13 +704,42 @@ void ztm_scan_ints(cudaStream_t s, int n, int* counts, int* total) {
   pm_nodes_scan<<<1, 1024, 0, s>>>(n, counts, total);
 }
 
+size_t ztm_pm64_list_ws(const PmParams& p) {
+  return WsCarver::need((size_t)p.N * sizeof(Pm64Node)) +
+         WsCarver::need(((size_t)p.kk * p.jj + 1) * sizeof(int));
+}
+
+void ztm_pm64_list(ztm_ctx* c, const PmParams& p, const double* d_drho, const int* d_mult, bool adj,
+                   WsCarver& wc, Pm64List* list) {
+  const int rows = p.kk * p.jj;
+  list->node = wc.take<Pm64Node>((size_t)p.N);
+  list->row = wc.take<int>((size_t)rows + 1);
+  const unsigned blocks = (unsigned)((rows + 3) / 4);
+  if (adj) {
+    pm64_rows_count<true><<<blocks, 128, 0, c->stream>>>(p, d_drho, d_mult, list->row);
+    ztm_scan_ints(c->stream, rows, list->row, list->row + rows);
+    pm64_rows_write<true><<<blocks, 128, 0, c->stream>>>(p, d_drho, d_mult, list->row, list->node);
+  } else {
+    pm64_rows_count<false><<<blocks, 128, 0, c->stream>>>(p, d_drho, d_mult, list->row);
+    ztm_scan_ints(c->stream, rows, list->row, list->row + rows);
+    pm64_rows_write<false><<<blocks, 128, 0, c->stream>>>(p, d_drho, d_mult, list->row, list->node);
+  }
+  c->launches += 3;
+}
+
 size_t ztm_pointmass_ws(const PmParams& p, int precision, int num_sms) {
   const bool f64 = precision == ZTM_PREC_FP64;
-  if (pm_use_cols(p, f64)) {  // the node columns
+  if (f64 && pm64_use(p)) {
+    int t64, c64, r64;
+    pm64_shape(p, num_sms, &t64, &c64, &r64);
+    return WsCarver::need((size_t)c64 * p.kk * std::max(p.ns, 1) * sizeof(double)) +
+           ztm_pm64_list_ws(p) + WsCarver::need((size_t)p.N * sizeof(int));  // nn multiplicities
+  }
+  if (!f64 && pm_use_cols(p)) {  // the node columns
     int ct, cc, ccols, cg;
-    pm_cols_shape(p, num_sms, f64, &ct, &cc, &ccols, &cg);
+    pm_cols_shape(p, num_sms, &ct, &cc, &ccols, &cg);
     const long long ncols = (long long)p.ii * p.jj;
-    const size_t entries = f64 ? (size_t)p.N + 2 : (size_t)((p.N + ncols) / 2 + 2);
+    const size_t entries = (size_t)((p.N + ncols) / 2 + 2);
     return WsCarver::need((size_t)cc * std::max(p.ns, 1) * sizeof(double)) +
            WsCarver::need((size_t)(ncols + 1) * sizeof(int)) +
            WsCarver::need((size_t)ncols * 16) + WsCarver::need(entries * 16) +
@@ -683,40 +761,48 @@ int ztm_launch_pointmass(ztm_ctx* c, const PmParams& p, const double* d_drho,
                          const int* d_nn, const double* d_surf, double* d_G,
                          double scale, int precision, WsCarver& wc) {
   const bool f64 = precision == ZTM_PREC_FP64;
-  const bool cols = pm_use_cols(p, f64);
+  const double factor = scale * 66.7 / ((double)p.fh * p.fh * p.fv);
+  // the listed nodes' multiplicities
+  auto mark = [&]() -> int* {
+    if (!d_nn) return nullptr;
+    int* mult = wc.take<int>((size_t)p.N);
+    cudaMemsetAsync(mult, 0, (size_t)p.N * sizeof(int), c->stream);
+    pm_nn_mark<<<(unsigned)((p.nnodes + 255) / 256), 256, 0, c->stream>>>(p, d_nn, mult, c->d_err);
+    c->launches++;
+    return mult;
+  };
+  if (f64 && pm64_use(p) && p.ns > 0 && p.nnodes > 0) {
+    int tiles, chunks, chunk_rows;
+    pm64_shape(p, c->num_sms, &tiles, &chunks, &chunk_rows);
+    double* partial = wc.take<double>((size_t)chunks * p.kk * p.ns);
+    Pm64List list;
+    int* mult = mark();
+    ztm_pm64_list(c, p, d_drho, mult, false, wc, &list);
+    const size_t smem = (size_t)p.ii * 8 + ((size_t)chunk_rows + 1) * 4;
+    if (smem > 40 * 1024)
+      cudaFuncSetAttribute(pm64_gather_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    {
+      ZtmProf prof_(c, "pointmass");
+      pm64_gather_kernel<<<(unsigned)((long long)tiles * p.kk * chunks), PM_TS, smem, c->stream>>>(
+          p, list.node, list.row, d_surf, tiles, chunk_rows, partial);
+    }
+    // fine-grid lengths: dz / r^3 is fh^2 times smaller there
+    pm64_finalize_kernel<<<(unsigned)((p.di * (long long)p.dj + 31) / 32), 256, 0, c->stream>>>(
+        p, p.kk * chunks, partial, factor * ((double)p.fh * p.fh), d_G);
+    c->launches += 2;
+    return ztm_after_launch(c, "point-mass kernels");
+  }
+  const bool cols = !f64 && pm_use_cols(p);
   int tiles, chunks, chunk_cols = 0, cg_cols = 0;
   long long len = 0;
   if (cols)
-    pm_cols_shape(p, c->num_sms, f64, &tiles, &chunks, &chunk_cols, &cg_cols);
+    pm_cols_shape(p, c->num_sms, &tiles, &chunks, &chunk_cols, &cg_cols);
   else
     pm_shape(p, c->num_sms, pm_occupancy(precision, true), &tiles, &chunks, &len);
   double* partial = wc.take<double>((size_t)chunks * std::max(p.ns, 1));
   if (p.ns > 0 && p.nnodes > 0) {
     dim3 grid(tiles, chunks);
-    if (cols && f64) {
-      const long long ncols = (long long)p.ii * p.jj;
-      int* offs = wc.take<int>((size_t)ncols + 1);
-      double2* colxy = wc.take<double2>((size_t)ncols);
-      double2* nodes = wc.take<double2>((size_t)p.N + 2);
-      int* mult = nullptr;
-      if (d_nn) {  // the listed nodes, with their multiplicities
-        mult = wc.take<int>((size_t)p.N);
-        cudaMemsetAsync(mult, 0, (size_t)p.N * sizeof(int), c->stream);
-        pm_nn_mark<<<(unsigned)((p.nnodes + 255) / 256), 256, 0, c->stream>>>(p, d_nn, mult,
-                                                                             c->d_err);
-        c->launches++;
-      }
-      const unsigned cb = (unsigned)((ncols + 255) / 256);
-      pm_cols_count64<<<cb, 256, 0, c->stream>>>(p, d_drho, mult, offs, colxy);
-      pm_nodes_scan<<<1, 1024, 0, c->stream>>>((int)ncols, offs, offs + ncols);
-      pm_cols_write64<<<cb, 256, 0, c->stream>>>(p, d_drho, mult, offs, nodes);
-      {
-        ZtmProf prof_(c, "pointmass");
-        pm_gather_cols64_kernel<<<grid, PM_TS, 0, c->stream>>>(p, nodes, offs, colxy, d_surf,
-                                                              cg_cols, chunk_cols, partial);
-      }
-      c->launches += 4;
-    } else if (precision == ZTM_PREC_FP64) {
+    if (precision == ZTM_PREC_FP64) {
       ZtmProf prof_(c, "pointmass");
       pm_gather_kernel<true><<<grid, PM_TS, 0, c->stream>>>(p, d_drho, d_nn, d_surf, len, partial,
                                                             c->d_err);
@@ -726,14 +812,7 @@ int ztm_launch_pointmass(ztm_ctx* c, const PmParams& p, const double* d_drho,
       int* offs = wc.take<int>((size_t)ncols + 1);
       float2* colxy = wc.take<float2>((size_t)ncols);
       float4* pairs = wc.take<float4>((size_t)((p.N + ncols) / 2 + 2));
-      int* mult = nullptr;
-      if (d_nn) {  // the listed nodes, with their multiplicities
-        mult = wc.take<int>((size_t)p.N);
-        cudaMemsetAsync(mult, 0, (size_t)p.N * sizeof(int), c->stream);
-        pm_nn_mark<<<(unsigned)((p.nnodes + 255) / 256), 256, 0, c->stream>>>(p, d_nn, mult,
-                                                                             c->d_err);
-        c->launches++;
-      }
+      int* mult = mark();
       const unsigned cb = (unsigned)((ncols + 255) / 256);
       pm_cols_count<<<cb, 256, 0, c->stream>>>(p, d_drho, mult, offs, colxy);
       pm_nodes_scan<<<1, 1024, 0, c->stream>>>((int)ncols, offs, offs + ncols);
@@ -763,7 +842,6 @@ int ztm_launch_pointmass(ztm_ctx* c, const PmParams& p, const double* d_drho,
   } else {
     chunks = 0;
   }
-  double factor = scale * 66.7 / ((double)p.fh * p.fh * p.fv);
   int M = p.di * p.dj;
   pm_finalize_kernel<<<(M + 255) / 256, 256, 0, c->stream>>>(p, chunks, partial, factor, d_G);
   c->launches++;
