@@ -150,7 +150,7 @@ using far64::D2;
 
 constexpr int F64_T = 128;       // threads per block: stations (forward), columns (adjoint)
 constexpr int F64_STAGE = 1024;  // float4 per shared-memory stage of the forward (16 KB)
-constexpr int F64_LG = 8;        // layers per thread of the adjoint
+constexpr int F64_LG = 16;       // layers per thread of the adjoint, at most
 constexpr int F64_ST = 32;       // stations per shared-memory tile of the adjoint
 constexpr int F64_MAX_NZ = F64_STAGE;
 constexpr int F64_MAX_SLOTS = 1024;
@@ -231,6 +231,7 @@ struct Fwd64Args {
   MeshDesc m;
   int ns, npair;
   int near_blocks, nparts;     // near blocks: 4 warps, one (station, part) each
+  int mix;                     // a near block at every mix-th place of the grid
   int tiles, chunk_pairs;      // far blocks: station tile x chunk of column pairs
   const float4* sxy;
   const float2* sz;
@@ -251,6 +252,7 @@ __device__ __forceinline__ void fwd_pair(const Far64Coef& f, const float4* col, 
                                          float n0, float2 ez, int2 a, int2 b, D2& acc) {
   const far64::Col o = far64::make_col<FORM>(f, X, Y);
   float n = n0;
+#pragma unroll 1  // by four 523 against 480 us (64x64x32, 32x32 stations): instruction fetches
   for (int l = 0; l < nz; l++, n += 1.f) {
     float zh, zl, qh, ql;
     far64::layer_z(n, f, ez.x, ez.y, &zh, &zl, &qh, &ql);
@@ -268,18 +270,19 @@ __global__ void __launch_bounds__(F64_T, 4) f64_fwd_kernel(const __grid_constant
   __shared__ float4 stage[F64_STAGE];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const MeshConst& k = a.k;
-  if ((int)blockIdx.x < a.near_blocks) {
-    // near regions first in the grid: their blocks start with the launch and
-    // use the FP64 pipe while the far blocks use the FMA pipe
-    const int w = blockIdx.x * (F64_T / 32) + warp;
+  // near blocks at every fourth place while there are any: an SM's four blocks
+  // then are one on the FP64 pipe and three on the FMA pipe (all near blocks
+  // first: 625 us for 64x64x32 under 32x32 stations, interleaved 567)
+  const int nbf = min((int)(blockIdx.x + a.mix - 1) / a.mix, a.near_blocks);  // near blocks before
+  if ((int)blockIdx.x % a.mix == 0 && nbf < a.near_blocks) {
+    const int w = nbf * (F64_T / 32) + warp;
     const int s = w / a.nparts, part = w % a.nparts;
     if (s < a.ns)
       near_station<double, true>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho,
-                           a.near + (size_t)part * a.ns, lane,
-                           nullptr, part, a.nparts);
+                                 a.near + (size_t)part * a.ns, lane, nullptr, part, a.nparts);
     return;
   }
-  const int item = blockIdx.x - a.near_blocks;
+  const int item = blockIdx.x - nbf;
   const int tile = item % a.tiles, chunk = item / a.tiles;
   const int slot = tile * F64_T + threadIdx.x;
   // threads past the last station repeat it (a finite value that is not stored)
@@ -347,8 +350,10 @@ __global__ void __launch_bounds__(512)
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const int s = blockIdx.x * 32 + x;
   double f = 0.0;
-  if (s < ns)
+  if (s < ns) {
+#pragma unroll 8
     for (int c = y; c < nchunks; c += 16) f += partial[(size_t)c * ns + s];
+  }
   sm[y][x] = f;
   __syncthreads();
   if (y || s >= ns) return;
@@ -367,8 +372,10 @@ struct Adj64Args {
   MeshConst k;
   MeshDesc m;
   int ns;
-  int near_blocks, cap;       // near blocks: 4 warps taking stations in turn
+  int near_blocks, cap;       // near blocks, taking stations in turn
+  int mix;                    // a near block at every mix-th place of the grid
   int ctiles, groups, slice;  // far blocks: column tile x layer group x station slice
+  int layers;                 // per group; the last may have fewer
   int fix_exp;                // near sums in fixed point: value * 2^(fix_exp - scale_exp)
   const float4* sxy;
   const float2* sz;
@@ -379,7 +386,7 @@ struct Adj64Args {
   const double* sxyz;
   const double* res;
   const unsigned* hw;         // high word of the largest |res|
-  double* phi;                // [near block][warp][cap] vertex values
+  double* phi;                // [near block][cap] vertex values
   unsigned long long* gnear;  // [np] fixed-point near sums, zeroed before
   double* partial;            // [slice][np]
 };
@@ -391,27 +398,36 @@ struct Adj64Smem {
   int4 box[F64_ST];                                                       // near box columns
   int id[F64_ST];
   float4 z[F64_ST / 2][F64_LG], q[F64_ST / 2][F64_LG];  // (hi, hi, lo, lo) of Z, Z^2
+  float4 acc[F64_LG][F64_T];
 };
 
-// One column's layers of the group against a station pair.
+// One column's layers of the group against a station pair.  The layer loop stays
+// a loop, with the sums in shared memory: unrolled over eight layers with the
+// sums in registers, the three forms and the masked one together are larger than
+// the instruction cache and half of all stalls were instruction fetches (61x47x23
+// prisms, 675 stations: 358 us; unrolled by four 325, by two 277, not at all 248).
 template <int FORM, bool MASK>
 __device__ __forceinline__ void adj_pair(const Far64Coef& f, const Adj64Smem& sm, int q, D2 X, D2 Y,
-                                         int2 a, int2 b, D2 (&acc)[F64_LG]) {
+                                         int2 a, int2 b, float4 (*acc)[F64_T], int nl) {
   const far64::Col o = far64::make_col<FORM>(f, X, Y);
   const float2 rh = sm.rh[q], rl = sm.rl[q];
-#pragma unroll
-  for (int l = 0; l < F64_LG; l++) {
+#pragma unroll 1
+  for (int l = 0; l < nl; l++) {
     const float4 z = sm.z[q][l], zz = sm.q[q][l];
     const D2 v = far64::value<FORM>(f, o, D2{make_float2(z.x, z.y), make_float2(z.z, z.w)},
                                     D2{make_float2(zz.x, zz.y), make_float2(zz.z, zz.w)});
-    far64::mac(acc[l], rh, rl, v, MASK && (unsigned)(l - a.x) <= (unsigned)(a.y - a.x),
+    const float4 t = acc[l][threadIdx.x];
+    D2 s{make_float2(t.x, t.y), make_float2(t.z, t.w)};
+    far64::mac(s, rh, rl, v, MASK && (unsigned)(l - a.x) <= (unsigned)(a.y - a.x),
                MASK && (unsigned)(l - b.x) <= (unsigned)(b.y - b.x));
+    acc[l][threadIdx.x] = make_float4(s.h.x, s.h.y, s.l.x, s.l.y);
   }
 }
 
-// Near region of station s by one warp: Phi at the vertices of a near prism,
-// then the signed corner sums, added in fixed point (order-independent).
-__device__ void adj64_near(const Adj64Args& a, int s, double* phi, int lane) {
+// Near region of station s by one block: Phi at the vertices of a near prism, a
+// quarter of them per warp, then the signed corner sums, added in fixed point
+// (order-independent).
+__device__ void adj64_near(const Adj64Args& a, int s, double* phi) {
   const MeshConst& k = a.k;
   const MeshDesc& m = a.m;
   const double r = a.res[s];
@@ -424,10 +440,12 @@ __device__ void adj64_near(const Adj64Args& a, int s, double* phi, int lane) {
   const double xs = a.sxyz[3 * s], ys = a.sxyz[3 * s + 1], zs = a.sxyz[3 * s + 2];
   const int nvx = b.x1 - b.x0 + 2, nvy = b.y1 - b.y0 + 2, nvz = L.y - L.x + 2;
   if (nvx * nvy * nvz > a.cap) return;  // the host sizes cap for the largest box
-  near_corners<double>(k, m, b, L, ivs, xs, ys, zs, a.cap, phi, lane);
+  near_corners<double>(k, m, b, L, ivs, xs, ys, zs, a.cap, phi, threadIdx.x & 31, threadIdx.x >> 5,
+                       F64_T / 32);
+  __syncthreads();
   const double sc = r * k.ninv * pow2(max(-1022, min(1022, a.fix_exp - scale_exp(hw))));
   const int bx = nvx - 1, by = nvy - 1, nb = bx * by * (nvz - 1);
-  for (int w = lane; w < nb; w += 32) {
+  for (int w = threadIdx.x; w < nb; w += F64_T) {
     const int qx = w % bx, qy = (w / bx) % by, qz = w / (bx * by);
     const short2 t = ivs[near_slot(b, b.x0 + qx, b.y0 + qy)];
     const int l = L.x + qz;
@@ -438,35 +456,38 @@ __device__ void adj64_near(const Adj64Args& a, int s, double* phi, int lane) {
     const long long p = (b.x0 + qx) + (long long)m.nx * (b.y0 + qy) + (long long)k.ncols * l;
     atomicAdd(&a.gnear[p], (unsigned long long)__double2ll_rn(sc * u));
   }
-  __syncwarp();
+  __syncthreads();  // the values are rewritten for the block's next station
 }
 
 __global__ void __launch_bounds__(F64_T, 4) f64_adj_kernel(const __grid_constant__ Adj64Args a) {
   __shared__ __align__(16) Adj64Smem sm;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const MeshConst& k = a.k;
-  if ((int)blockIdx.x < a.near_blocks) {
-    const int w = blockIdx.x * (F64_T / 32) + warp;
-    for (int s = w; s < a.ns; s += a.near_blocks * (F64_T / 32))
-      adj64_near(a, s, a.phi + (size_t)w * a.cap, lane);
+  const int nbf = min((int)(blockIdx.x + a.mix - 1) / a.mix, a.near_blocks);  // near blocks before
+  if ((int)blockIdx.x % a.mix == 0 && nbf < a.near_blocks) {
+    for (int s = nbf; s < a.ns; s += a.near_blocks) adj64_near(a, s, a.phi + (size_t)nbf * a.cap);
     return;
   }
-  int item = blockIdx.x - a.near_blocks;
+  int item = blockIdx.x - nbf;
   const int ct = item % a.ctiles;
   item /= a.ctiles;
   const int lg = item % a.groups, sl = item / a.groups;
-  const int cc = ct * F64_T + threadIdx.x, c = min(cc, k.ncols - 1);
-  const int ix = c % k.nx, iy = c / k.nx, l0 = lg * F64_LG;
+  // columns in strips of four rows, down a strip's columns one after another: a
+  // warp is an 8 x 4 patch (the last strip has the rows that are left), which
+  // crosses a form's circle or a near box less often than 32 columns of a row
+  const int cc = ct * F64_T + threadIdx.x, ci = min(cc, k.ncols - 1);
+  const int strip = ci / (4 * k.nx), in_strip = ci - strip * 4 * k.nx;
+  const int rows = min(4, k.ny - 4 * strip);
+  const int ix = in_strip / rows, iy = 4 * strip + in_strip % rows, c = ix + k.nx * iy;
+  const int l0 = lg * a.layers, nl = min(a.layers, k.nz - l0);
   const float fix = (float)ix, fiy = (float)iy;
   const double rsc = pow2(-scale_exp(*a.hw));
-  D2 acc[F64_LG];
-#pragma unroll
-  for (int l = 0; l < F64_LG; l++) acc[l] = far64::dd_dup(0.f, 0.f);
+  // (hi, hi, lo, lo) sums of the thread's own column
+  for (int l = 0; l < nl; l++) sm.acc[l][threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
   const int s0 = sl * a.slice, s1 = min(a.ns, s0 + a.slice);
   for (int t0 = s0; t0 < s1; t0 += F64_ST) {
     __syncthreads();
-    for (int q = threadIdx.x; q < F64_ST * F64_LG; q += F64_T) {
-      const int j = q / F64_LG, l = q % F64_LG, lane2 = j & 1;
+    for (int q = threadIdx.x; q < F64_ST * nl; q += F64_T) {
+      const int j = q / nl, l = q - j * nl, lane2 = j & 1;
       const bool ok = t0 + j < s1;
       const int s = a.perm[min(t0 + j, s1 - 1)];  // past the slice: repeated, zero residual
       const int4 h = a.si[s];
@@ -520,26 +541,29 @@ __global__ void __launch_bounds__(F64_T, 4) f64_adj_kernel(const __grid_constant
       }
       // the repeated station of an odd count may sit on a prism centre: masked
       const bool pad = t0 + 2 * q + 1 >= s1;
-      if (pad) iv[1] = make_int2(0, F64_LG);
+      if (pad) iv[1] = make_int2(0, nl);
       if (pad || __any_sync(0xffffffffu, near))
-        adj_pair<0, true>(a.fc, sm, q, X, Y, iv[0], iv[1], acc);
+        adj_pair<0, true>(a.fc, sm, q, X, Y, iv[0], iv[1], sm.acc, nl);
       else if (__all_sync(0xffffffffu, rh >= a.fc.rh_c))
-        adj_pair<2, false>(a.fc, sm, q, X, Y, iv[0], iv[1], acc);
+        adj_pair<2, false>(a.fc, sm, q, X, Y, iv[0], iv[1], sm.acc, nl);
       else if (__all_sync(0xffffffffu, rh >= a.fc.rh_b))
-        adj_pair<1, false>(a.fc, sm, q, X, Y, iv[0], iv[1], acc);
+        adj_pair<1, false>(a.fc, sm, q, X, Y, iv[0], iv[1], sm.acc, nl);
       else
-        adj_pair<0, false>(a.fc, sm, q, X, Y, iv[0], iv[1], acc);
+        adj_pair<0, false>(a.fc, sm, q, X, Y, iv[0], iv[1], sm.acc, nl);
     }
-#pragma unroll
-    for (int l = 0; l < F64_LG; l++) acc[l] = far64::quick(acc[l].h, acc[l].l);
+    for (int l = 0; l < nl; l++) {
+      const float4 t = sm.acc[l][threadIdx.x];
+      const D2 s = far64::quick(make_float2(t.x, t.y), make_float2(t.z, t.w));
+      sm.acc[l][threadIdx.x] = make_float4(s.h.x, s.h.y, s.l.x, s.l.y);
+    }
   }
   if (cc >= k.ncols) return;
   double* out = a.partial + (size_t)sl * ((size_t)k.ncols * k.nz) + c;
-#pragma unroll
-  for (int l = 0; l < F64_LG; l++)
-    if (l0 + l < k.nz)
-      out[(size_t)(l0 + l) * k.ncols] = ((double)acc[l].h.x + (double)acc[l].l.x) +
-                                        ((double)acc[l].h.y + (double)acc[l].l.y);
+  for (int l = 0; l < nl; l++) {
+    const float4 t = sm.acc[l][threadIdx.x];
+    out[(size_t)(l0 + l) * k.ncols] =
+        ((double)t.x + (double)t.z) + ((double)t.y + (double)t.w);
+  }
 }
 
 __global__ void f64_adj_finalize(long long np, int slices, const double* __restrict__ partial,
@@ -584,7 +608,7 @@ Fwd64Shape fwd64_shape(const MeshConst& k, int ns, int num_sms) {
 }
 
 struct Adj64Shape {
-  int ctiles, groups, slice, slices, near_blocks, cap;
+  int ctiles, groups, layers, slice, slices, near_blocks, cap;
 };
 
 int adj64_cap(const MeshConst& k) {
@@ -596,17 +620,23 @@ Adj64Shape adj64_shape(const MeshConst& k, int ns, int num_sms) {
   Adj64Shape f;
   f.ctiles = (k.ncols + F64_T - 1) / F64_T;
   f.groups = (k.nz + F64_LG - 1) / F64_LG;
+  f.layers = (k.nz + f.groups - 1) / f.groups;
   const long long per = (long long)f.ctiles * f.groups;
   long long want = std::max(1LL, (64LL * num_sms + per - 1) / per);
-  want = std::min(want, 16LL);  // the slices' partial sums are np doubles each
+  want = std::min(want, 32LL);  // the slices' partial sums are np doubles each
   long long sl = (ns + want - 1) / want;
-  sl = (sl + F64_ST - 1) / F64_ST * F64_ST;
+  sl = (sl + 1) / 2 * 2;
   f.slice = (int)sl;
   f.slices = (ns + f.slice - 1) / f.slice;
-  // two near blocks per SM at most: each warp owns a box of vertex values
-  f.near_blocks = (int)std::min<long long>(((long long)ns + F64_T / 32 - 1) / (F64_T / 32), 2LL * num_sms);
+  // eight near blocks per SM at most: each owns a box of vertex values
+  f.near_blocks = (int)std::min<long long>(ns, 8LL * num_sms);
   f.cap = adj64_cap(k);
   return f;
+}
+
+// Places of the near blocks: every fourth while the far blocks suffice.
+int near_mix(long long near, long long far) {
+  return (int)std::max(1LL, std::min(4LL, (near + far) / std::max(near, 1LL)));
 }
 
 // Preparation shared by both directions.
@@ -687,6 +717,7 @@ int ztm_launch_prism64(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int n
   a.npair = f.npair;
   a.near_blocks = f.near_blocks;
   a.nparts = f.nparts;
+  a.mix = near_mix(f.near_blocks, (long long)f.tiles * f.chunks);
   a.tiles = f.tiles;
   a.chunk_pairs = f.chunk_pairs;
   a.sxy = p.sxy;
@@ -715,7 +746,7 @@ size_t ztm_adjoint64_ws(const MeshDesc& m, int ns, int num_sms) {
   const MeshConst k = make_mesh_const(m, FAR64_Q);
   const Adj64Shape f = adj64_shape(k, ns, std::max(num_sms, 1));
   const size_t np = (size_t)k.ncols * k.nz;
-  return prep64_ws(k, ns) + WsCarver::need((size_t)f.near_blocks * (F64_T / 32) * f.cap * 8) +
+  return prep64_ws(k, ns) + WsCarver::need((size_t)f.near_blocks * f.cap * 8) +
          WsCarver::need(np * 8) + WsCarver::need((size_t)f.slices * np * 8);
 }
 
@@ -730,13 +761,15 @@ int ztm_launch_adjoint64(ztm_ctx* c, const MeshDesc& m, int ns, const double* d_
   const size_t np = (size_t)a.k.ncols * a.k.nz;
   Prep64 p;
   if (int rc = prep64(c, m, a.k, ns, d_sxyz, ns, d_res, wc, &p)) return rc;
-  a.phi = wc.take<double>((size_t)f.near_blocks * (F64_T / 32) * f.cap);
+  a.phi = wc.take<double>((size_t)f.near_blocks * f.cap);
   a.gnear = wc.take<unsigned long long>(np);
   a.partial = wc.take<double>((size_t)f.slices * np);
   a.near_blocks = f.near_blocks;
   a.cap = f.cap;
+  a.mix = near_mix(f.near_blocks, (long long)f.ctiles * f.groups * f.slices);
   a.ctiles = f.ctiles;
   a.groups = f.groups;
+  a.layers = f.layers;
   a.slice = f.slice;
   // |r U| < 2^(e+1) 2 pi dz for a prism (no more than an infinite slab), summed
   // over at most ns stations: below 2^62 in fixed point

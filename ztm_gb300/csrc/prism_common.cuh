@@ -227,21 +227,37 @@ __device__ __forceinline__ int near_slot(const NearBox& b, int ix, int iy) {
   return (ix - b.x0) + (b.x1 - b.x0 + 1) * (iy - b.y0);
 }
 
-// Corner function of a near region's vertex (offsets in m): double in scaled
-// lengths by phi64.cuh (the result times ninv is the corner function up to
-// terms linear in x and y, which the signed corner sums drop), float by the
-// library functions in metres.
+// A station's near region: the corner function of vertex (a, b, c), in double in
+// scaled lengths by phi64.cuh (the result times ninv is the corner function up
+// to terms linear in x and y, which the signed corner sums drop), in float by
+// the library functions in metres.
 template <typename T>
-__device__ __forceinline__ T near_phi(const MeshConst& k, double x, double y, double z);
+struct NearFrame;
 template <>
-__device__ __forceinline__ double near_phi<double>(const MeshConst& k, double x, double y,
-                                                   double z) {
-  return phi64::phi(x * k.nsc, y * k.nsc, z * k.nsc);
-}
+struct NearFrame<double> {
+  double x, y, z, dx, dy, dz;  // mesh origin minus station, cell edges
+  __device__ __forceinline__ NearFrame(const MeshConst& k, const MeshDesc& m, double xs, double ys,
+                                       double zs)
+      : x((m.x0 - xs) * k.nsc), y((m.y0 - ys) * k.nsc), z((m.zt - zs) * k.nsc), dx(m.dx * k.nsc),
+        dy(m.dy * k.nsc), dz(m.dz * k.nsc) {}
+  __device__ __forceinline__ double phi(int a, int b, int c) const {
+    return phi64::phi(fma(phi64::of_int(a), dx, x), fma(phi64::of_int(b), dy, y),
+                      fma(phi64::of_int(-c), dz, z));
+  }
+};
 template <>
-__device__ __forceinline__ float near_phi<float>(const MeshConst&, double x, double y, double z) {
-  return ztm_phi<float>((float)x, (float)y, (float)z);
-}
+struct NearFrame<float> {
+  const MeshDesc& m;
+  double xs, ys, zs;
+  __device__ __forceinline__ NearFrame(const MeshConst&, const MeshDesc& mesh, double x, double y,
+                                       double z)
+      : m(mesh), xs(x), ys(y), zs(z) {}
+  __device__ __forceinline__ float phi(int a, int b, int c) const {
+    return ztm_phi<float>((float)(fma((double)a, m.dx, m.x0) - xs),
+                          (float)(fma((double)b, m.dy, m.y0) - ys),
+                          (float)(fma(-(double)c, m.dz, m.zt) - zs));
+  }
+};
 
 // A warp's queue of near vertices (index, and density difference where one is
 // used), one entry per lane, held in registers so that full warps evaluate.
@@ -319,7 +335,7 @@ __device__ __forceinline__ void near_station(const MeshConst& k, const MeshDesc&
     return;
   }
   const short2* ivs = iv + (size_t)s * k.nslots;
-  const double xs = sxyz[3 * s], ys = sxyz[3 * s + 1], zs = sxyz[3 * s + 2];
+  const NearFrame<T> frame(k, m, sxyz[3 * s], sxyz[3 * s + 1], sxyz[3 * s + 2]);
   const int nvx = b.x1 - b.x0 + 2, nvy = b.y1 - b.y0 + 2, nvz = L.y - L.x + 2;
   const int nv = nvx * nvy * nvz;
   const long long plane = (long long)m.nx * m.ny;
@@ -327,10 +343,8 @@ __device__ __forceinline__ void near_station(const MeshConst& k, const MeshDesc&
   const int vb = (int)((long long)nv * part / nparts);
   const int ve = (int)((long long)nv * (part + 1) / nparts);
   auto eval = [&](int v, double D) {
-    const int a = b.x0 + v % nvx, bb = b.y0 + (v / nvx) % nvy, cz = L.x + v / (nvx * nvy);
-    acc = fma((T)D, near_phi<T>(k, fma((double)a, m.dx, m.x0) - xs,
-                                fma((double)bb, m.dy, m.y0) - ys,
-                                fma(-(double)cz, m.dz, m.zt) - zs), acc);
+    const int w = v / nvx;
+    acc = fma((T)D, frame.phi(b.x0 + v - w * nvx, b.y0 + w % nvy, L.x + w / nvy), acc);
     if (nphi) ++*nphi;
   };
   NearQueue q;
@@ -378,27 +392,30 @@ __device__ __forceinline__ void near_station(const MeshConst& k, const MeshDesc&
 
 // Corner functions of a near region's vertices, by one warp: phi[v] of every
 // vertex of the near box's layers L.x .. L.y + 1 (v = x + nvx (y + nvy z),
-// cap values at most) that is a corner of a near prism, the others untouched.
+// cap values at most) that is a corner of a near prism, the others untouched;
+// part of nparts: one of nparts equal ranges of the vertices.
 // Full warps evaluate, through a queue as in near_station; double values
 // are in scaled lengths (times ninv: metres).
 template <typename T>
 __device__ __forceinline__ void near_corners(const MeshConst& k, const MeshDesc& m,
                                              const NearBox& b, int2 L,
                                              const short2* __restrict__ ivs, double xs, double ys,
-                                             double zs, int cap, T* __restrict__ phi, int lane) {
+                                             double zs, int cap, T* __restrict__ phi, int lane,
+                                             int part = 0, int nparts = 1) {
   const int nvx = b.x1 - b.x0 + 2, nvy = b.y1 - b.y0 + 2, nvz = L.y - L.x + 2;
   const int nv = min(nvx * nvy * nvz, cap);
+  const NearFrame<T> frame(k, m, xs, ys, zs);
   auto eval = [&](int v, double) {
-    phi[v] = near_phi<T>(k, fma((double)(b.x0 + v % nvx), m.dx, m.x0) - xs,
-                         fma((double)(b.y0 + (v / nvx) % nvy), m.dy, m.y0) - ys,
-                         fma(-(double)(L.x + v / (nvx * nvy)), m.dz, m.zt) - zs);
+    const int w = v / nvx;
+    phi[v] = frame.phi(b.x0 + v - w * nvx, b.y0 + w % nvy, L.x + w / nvy);
   };
   NearQueue q;
   q.n = 0;
-  for (int v0 = 0; v0 < nv; v0 += 32) {
+  const int vb = nv * part / nparts, ve = nv * (part + 1) / nparts;
+  for (int v0 = vb; v0 < ve; v0 += 32) {
     const int v = v0 + lane;
     bool used = false;
-    if (v < nv) {
+    if (v < ve) {
       const int ax = v % nvx, ay = (v / nvx) % nvy, cz = L.x + v / (nvx * nvy);
 #pragma unroll
       for (int d = 0; d < 4; d++) {  // the (up to) four columns around the vertex
