@@ -39,7 +39,7 @@ constexpr int ADJ_LG = 32;     // layers per thread in the far kernel
 constexpr int ADJ_STILE = 64;  // stations per shared-memory tile
 constexpr int ADJ_SGRP = 32;   // stations per float sum
 
-constexpr int ADJ_NEAR_ST = 8;  // stations per near item (two per warp)
+constexpr int ADJ_NEAR_ST = 4;  // stations per near item (one per warp)
 
 struct AdjArgs {
   MeshConst k;
@@ -258,8 +258,11 @@ __device__ __forceinline__ void adj_near_station(const AdjArgs& a, int s, T* phi
 // counter, the near items at evenly spaced queue positions.  The grid is the
 // number of blocks resident at once.  T: the near regions' type (double for
 // the mixed method, float for the FP32 method).
+// Four blocks per SM at 128 registers: with five (96) the far loop spilled
+// (20.37 against 20.15 ms, 256x256x64 prisms under 128x128 stations; eight
+// blocks of 64 columns 20.31).
 template <typename T>
-__global__ void __launch_bounds__(ADJ_TS, 5) adj_kernel(AdjArgs a) {
+__global__ void __launch_bounds__(ADJ_TS, 4) adj_kernel(AdjArgs a) {
   __shared__ AdjSmem sm;
   __shared__ int s_item;
   const int n_far = a.tiles * a.slices;
@@ -447,12 +450,13 @@ int ztm_launch_adjoint(ztm_ctx* c, const MeshDesc& m, int ns, const double* d_sx
   if ((size_t)cap * 8 > 200 * 1024)
     return ztm_fail(c, ZTM_ERR_RANGE, "near_q too large for the adjoint's near box");
   const bool f64 = precision == ZTM_PREC_MIXED;
-  // station slices so that there are about sixteen far items per resident
-  // block (measured: 4 items 22.2 ms, 8 21.1, 16 20.4, 24 20.8, 32 20.7);
+  // station slices so that there are about 80 far items per SM (a thread's far
+  // sum is a chain of compensated float sums per slice, so the slices do not
+  // follow the launch's residency);
   // the slices' sums meet in g by double atomics (g zeroed first)
   const long long tiles = (long long)((k.ncols + ADJ_TS - 1) / ADJ_TS) * ngroups;
   const int grid = adj_grid(c->num_sms, f64);
-  long long slices = std::max(1LL, (16LL * grid + tiles - 1) / tiles);
+  long long slices = std::max(1LL, (80LL * std::max(c->num_sms, 1) + tiles - 1) / tiles);
   slices = std::min(slices, std::max(1LL, (long long)(ns + ADJ_STILE - 1) / ADJ_STILE));
   int slice = (int)((ns + slices - 1) / slices);
   slice = ((slice + ADJ_STILE - 1) / ADJ_STILE) * ADJ_STILE;

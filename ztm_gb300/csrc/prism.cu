@@ -37,7 +37,7 @@
 
 namespace {
 
-constexpr int FAR_TS = 128;   // stations per block in the far kernel
+constexpr int FAR_TILE = 128; // stations per tile of the work split (far_shape)
 constexpr int F64_TS = 64;    // stations per block in the plain double kernel
 
 // ---------------------------------------------------------------------------
@@ -204,8 +204,15 @@ __device__ __forceinline__ float far_pair(float rho, float Z, float rh, float a0
 // COUNT: the counting variant (ztm_ctx_count_forms): the same work, with the
 // evaluated slots of each form (and the near regions' Phi evaluations) added
 // to a.forms at the end.
-template <bool COUNT>
-__global__ void __launch_bounds__(FAR_TS, 6) far_kernel(FarArgs a) {
+// Sixteen warps per SM at 128 registers: the loop is bound by the FMA pipe and
+// the special-function unit together (nine packed operations, 18 clocks, and two
+// rsqrt, 16 clocks, per value pair; alone they sustain 20.5 with both), so
+// registers for more pairs in flight serve better than more warps (64-station
+// blocks, 256x256x64 prisms under 128x128 stations: 24 warps 21.3 ms, 20 warps
+// 21.10, 16 warps 20.93, 14 warps 21.28).
+// FAR_TS: stations per block and item.
+template <bool COUNT, int FAR_TS>
+__global__ void __launch_bounds__(FAR_TS, 512 / FAR_TS) far_kernel(FarArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
   float* stage = reinterpret_cast<float*>(smem_raw + 128);
@@ -384,21 +391,32 @@ __global__ void __launch_bounds__(FAR_TS, 6) far_kernel(FarArgs a) {
   }
 }
 
-// gz[s] = G5 * (far_scale * sum_c partial[c][s] + sum_q near[q][s])
-__global__ void finalize_kernel(int ns, int nchunks, const double* __restrict__ partial,
-                                double far_scale, const double* __restrict__ near, int nparts,
-                                double G5, double* __restrict__ gz) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ns) return;
-  double f = 0.0;
-  for (int c = 0; c < nchunks; c++) f += partial[(size_t)c * ns + s];
-  double g = far_scale * f;
-  if (near) {
-    double n = near[s];
-    for (int q = 1; q < nparts; q++) n += near[(size_t)q * ns + s];
-    g += n;
+// gz[s] = G5 * (far_scale * sum_c partial[c][s] + sum_q near[q][s]): 32 stations
+// per block, FIN_Y threads each over the chunks, summed in a fixed order (a
+// thread per station over all chunks is one chain of dependent adds and loads).
+constexpr int FIN_Y = 16;
+__global__ void __launch_bounds__(32 * FIN_Y)
+    finalize_kernel(int ns, int nchunks, const double* __restrict__ partial, double far_scale,
+                    const double* __restrict__ near, int nparts, double G5,
+                    double* __restrict__ gz) {
+  __shared__ double sm[2][FIN_Y][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int s = blockIdx.x * 32 + x;
+  double f = 0.0, n = 0.0;
+  if (s < ns) {
+#pragma unroll 4
+    for (int c = y; c < nchunks; c += FIN_Y) f += partial[(size_t)c * ns + s];
+    for (int q = y; q < nparts; q += FIN_Y) n += near[(size_t)q * ns + s];
   }
-  gz[s] = G5 * g;
+  sm[0][y][x] = f;
+  sm[1][y][x] = n;
+  __syncthreads();
+  if (y || s >= ns) return;
+  for (int q = 1; q < FIN_Y; q++) {
+    f += sm[0][q][x];
+    n += sm[1][q][x];
+  }
+  gz[s] = G5 * (far_scale * f + n);
 }
 
 // ---------------------------------------------------------------------------
@@ -588,9 +606,10 @@ __global__ void __launch_bounds__(F64_TS)
 int near_parts(int ns, int num_sms) {
   return std::max(1, std::min(16, (int)((16LL * std::max(num_sms, 1) + ns - 1) / ns)));
 }
-int near_units(int ns) { return std::max(4, std::min(32, ns / 2048 * 4)); }
+int near_units(int ns, int ts) { return ts / 32 * std::max(1, std::min(8, ns / 2048)); }
 
 struct FarShape {
+  int ts;  // stations per block and item: 128 or 64
   int tiles, chunks, chunk_cols, sc, grid;
   size_t smem;
 };
@@ -599,41 +618,75 @@ struct FarShape {
 // items per resident block}.  The first is the default.
 constexpr int FAR_SHAPES[][2] = {{32, 8}, {16, 16}, {16, 8}, {32, 16}, {64, 16}, {64, 8}};
 
+// Blocks per SM that the work split assumes for smem bytes of stages.
+int split_blocks(size_t smem) {
+  int dev = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) !=
+          cudaSuccess) {
+    cudaGetLastError();
+    return 6;
+  }
+  const long long block = ((long long)smem + 1024 + 28 + 127) / 128 * 128;
+  return (int)std::max(1LL, std::min(6LL, per_sm / block));
+}
+
+template <int TS>
+int far_occupancy(size_t smem) {
+  // stages above the default 48 KB need the opt-in (very deep meshes)
+  if (smem > 48 * 1024 &&
+      (cudaFuncSetAttribute(far_kernel<false, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)smem) != cudaSuccess ||
+       cudaFuncSetAttribute(far_kernel<true, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)smem) != cudaSuccess))
+    cudaGetLastError();
+  int occ = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, far_kernel<false, TS>, TS, smem) !=
+          cudaSuccess ||
+      occ < 1) {
+    cudaGetLastError();
+    occ = 1;
+  }
+  return occ;
+}
+
 // Launch shape of the far kernel: sc columns per stage, the grid = the blocks
 // resident at once, about ipb work items per block (more items: a shorter
 // tail when blocks finish unevenly; fewer: less partial-sum traffic).
 FarShape far_shape(const MeshConst& k, int ns, int num_sms, const ztm_opts* o, int sc_want = 16,
                    int ipb = 16) {
   FarShape f;
-  f.tiles = std::max(1, (ns + FAR_TS - 1) / FAR_TS);
   int sc = std::max(1, (24 * 1024) / (k.nzp * 4));
   sc = std::min(sc, 64);
   if (sc_want > 0) sc = std::max(1, std::min(sc, sc_want));
+  // A thread's far sum is a chain of compensated float sums per chunk, so the
+  // chunks are the split's (tiles of FAR_TILE stations, ipb items per block of
+  // six to an SM as far as two stages of sc columns fit) whatever the launch.
+  // A block takes half a tile where eight such blocks' stages fit an SM: shorter
+  // items at the end of the queue and cheaper barriers (256x256x64 prisms,
+  // 128x128 stations: 21.55 ms with whole tiles, 20.93 with halves, 21.49 with
+  // quarters); deeper meshes keep whole tiles for their warps per SM.
+  const int split_occ = split_blocks(128 + 2 * (size_t)sc * k.nzp * 4);
   f.sc = sc;
   f.smem = 128 + 2 * (size_t)sc * k.nzp * 4;
-  // stages above the default 48 KB need the opt-in (very deep meshes)
-  if (f.smem > 48 * 1024 &&
-      (cudaFuncSetAttribute(far_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)f.smem) != cudaSuccess ||
-       cudaFuncSetAttribute(far_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)f.smem) != cudaSuccess))
-    cudaGetLastError();
+  f.ts = f.smem <= 27 * 1024 ? FAR_TILE / 2 : FAR_TILE;
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, far_kernel<false>, FAR_TS, f.smem) !=
-          cudaSuccess ||
-      occ < 1) {
-    cudaGetLastError();
-    occ = 1;
-  }
+  if (f.ts == FAR_TILE)
+    occ = far_occupancy<FAR_TILE>(f.smem);
+  else
+    occ = far_occupancy<FAR_TILE / 2>(f.smem);
   const long long resident = (long long)occ * std::max(num_sms, 1);
-  long long chunks = (ipb * resident + f.tiles - 1) / f.tiles;
+  const long long tiles = (ns + FAR_TILE - 1) / FAR_TILE;
+  long long chunks =
+      (ipb * (long long)split_occ * std::max(num_sms, 1) + tiles - 1) / std::max(tiles, 1LL);
   if (o && o->chunk > 0) chunks = (k.ncols + o->chunk - 1) / o->chunk;
   chunks = std::max(1LL, std::min(chunks, (long long)std::max(1, k.ncols / sc)));
   int cc = (int)((k.ncols + chunks - 1) / chunks);
   cc = ((cc + sc - 1) / sc) * sc;
   f.chunk_cols = cc;
   f.chunks = (k.ncols + cc - 1) / cc;
-  const int nu = near_units(ns);
+  f.tiles = std::max(1, (ns + f.ts - 1) / f.ts);
+  const int nu = near_units(ns, f.ts);
   const long long n_near = ((long long)ns * near_parts(ns, num_sms) + nu - 1) / nu;
   f.grid = (int)std::min(resident, (long long)f.tiles * f.chunks + n_near);
   return f;
@@ -745,7 +798,7 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
       mesh_f64_kernel<<<dim3(tiles, (unsigned)ch), F64_TS, 0, c->stream>>>(m, ns, d_sxyz, D, len,
                                                                            partial);
     }
-    finalize_kernel<<<(ns + 255) / 256, 256, 0, c->stream>>>(ns, (int)ch, partial, 1.0, nullptr,
+    finalize_kernel<<<(ns + 31) / 32, 32 * FIN_Y, 0, c->stream>>>(ns, (int)ch, partial, 1.0, nullptr,
                                                              0, G5, d_gz);
     c->launches += 3;
     return ztm_after_launch(c, "prism FP64 kernels");
@@ -789,8 +842,6 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
   a.err = c->d_err;
   a.counter = counter;
   a.nparts = nparts;
-  a.near_units = near_units(ns);
-  a.n_near = (int)(((long long)ns * nparts + a.near_units - 1) / a.near_units);
   a.near_f64 = precision == ZTM_PREC_MIXED;
   a.m = m;
   a.sxyz = d_sxyz;
@@ -805,10 +856,13 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
     a.chunk_cols = t.chunk_cols;
     a.sc = t.sc;
     cudaMemsetAsync(counter, 0, sizeof(int), c->stream);
-    if (c->count_forms && c->d_forms)
-      far_kernel<true><<<t.grid, FAR_TS, t.smem, c->stream>>>(a);
-    else
-      far_kernel<false><<<t.grid, FAR_TS, t.smem, c->stream>>>(a);
+    a.near_units = near_units(ns, t.ts);
+    a.n_near = (int)(((long long)ns * nparts + a.near_units - 1) / a.near_units);
+    const bool count = c->count_forms && c->d_forms;
+    auto* fn = t.ts == FAR_TILE
+                   ? (count ? far_kernel<true, FAR_TILE> : far_kernel<false, FAR_TILE>)
+                   : (count ? far_kernel<true, FAR_TILE / 2> : far_kernel<false, FAR_TILE / 2>);
+    fn<<<t.grid, t.ts, t.smem, c->stream>>>(a);
     c->launches++;
   };
   if (o && (o->flags & ZTM_FLAG_AUTOTUNE) && !(o->chunk > 0) && it == c->tuned.end()) {
@@ -842,7 +896,7 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
     launch_far(f);
   }
   const double far_scale = k.L0 * (double)k.dxn * k.dyn * k.dzn;
-  finalize_kernel<<<(ns + 255) / 256, 256, 0, c->stream>>>(ns, f.chunks, partial, far_scale, near,
+  finalize_kernel<<<(ns + 31) / 32, 32 * FIN_Y, 0, c->stream>>>(ns, f.chunks, partial, far_scale, near,
                                                            nparts, G5, d_gz);
   c->launches++;
   return ztm_after_launch(c, "prism mixed kernels");
@@ -891,7 +945,7 @@ int ztm_launch_prism_list(ztm_ctx* c, long long np, const double* d_geom, const 
   } else {
     ch = 0;
   }
-  finalize_kernel<<<(ns + 255) / 256, 256, 0, c->stream>>>(ns, (int)ch, partial, 1.0, nullptr, 0, G5,
+  finalize_kernel<<<(ns + 31) / 32, 32 * FIN_Y, 0, c->stream>>>(ns, (int)ch, partial, 1.0, nullptr, 0, G5,
                                                            d_gz);
   c->launches++;
   return ztm_after_launch(c, "prism list kernels");
