@@ -42,7 +42,8 @@ constexpr int IF_NEAR_WPB = 4;
 // took 1.75 ms at 8 (under one wave), 1.6 at 24, 1.55 at 48
 constexpr int IF_FWD_PER_SM = 48;
 constexpr int IF_SUB = 32;       // columns per second-order test in the forward
-constexpr float IF_FAR = 1.0e6f; // -index of a padding column (far away)
+constexpr float IF_FAR = 1.0e6f; // -index of a padding column, height of a padding station
+constexpr int IF_ROWS = 3;       // rows of the adjoint's table of Y terms
 // the forward's tile load: each warp loads whole blocks of IF_SUB columns
 static_assert(IF_SUB == 32 && IF_TILE % IF_TS == 0 && IF_TS % 32 == 0, "tile load layout");
 
@@ -101,8 +102,9 @@ struct IStation {  // per-station float data
 
 __global__ void iface_station_prep(IMeshDesc m, double L0, int ns, const double* __restrict__ sxyz,
                                    const double* __restrict__ res, IStation* __restrict__ sf,
-                                   int2* __restrict__ si) {
+                                   int2* __restrict__ si, unsigned* __restrict__ ticket) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s == 0 && ticket) *ticket = 0u;
   if (s >= ns) return;
   double xs = sxyz[3 * s], ys = sxyz[3 * s + 1], zs = sxyz[3 * s + 2];
   const double lim = 1.0e9;
@@ -189,13 +191,13 @@ __global__ void iface_near_mask(IConst k, int ns, const double* __restrict__ sxy
 }
 
 // The unit face integral of the far expansion for two pairs, given 1/r of
-// the column top.  T2: second order only (pairs beyond rt2_t2).
+// the column top.  T2: second order only (pairs beyond rt2_t2).  cbY = cB Y2.
 template <bool T2>
-__device__ __forceinline__ float2 face_unit_far2(float2 X2, float2 Y2, float2 ut, float2 rinv,
-                                                 const FarCoef& f) {
+__device__ __forceinline__ float2 face_unit_far2(float2 X2, float2 Y2, float2 cbY, float2 ut,
+                                                 float2 rinv, const FarCoef& f) {
   const float2 Z2 = __fmul2_rn(ut, ut);
   const float2 ri2 = __fmul2_rn(rinv, rinv), ri4 = __fmul2_rn(ri2, ri2);
-  const float2 a0 = __ffma2_rn(X2, make_float2(f.cA, f.cA), __fmul2_rn(Y2, make_float2(f.cB, f.cB)));
+  const float2 a0 = __ffma2_rn(X2, make_float2(f.cA, f.cA), cbY);
   const float2 n2 = __ffma2_rn(make_float2(f.a1, f.a1), Z2, a0);
   float2 t;
   if (T2) {
@@ -212,16 +214,24 @@ __device__ __forceinline__ float2 face_unit_far2(float2 X2, float2 Y2, float2 ut
   return __ffma2_rn(base, t, base);
 }
 
+// a / b, subnormals flushed (PTX div.approx.ftz.f32): far-field quotients are
+// never subnormal, and the flush spares the scaling around the reciprocal.
+__device__ __forceinline__ float div_ftz(float a, float b) {
+  float q;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(q) : "f"(a), "f"(b));
+  return q;
+}
+
 // Unit column integral (normalised, without dx dy) for two far pairs on the
 // packed FP32 path: the exact vertical integral of the column axis plus the
 // horizontal correction at its top and bottom, to 4th order, or to 2nd order
-// when T2 (pairs beyond rt2_t2).  rt2 = ut^2 + rh.  The SFU operations stay
-// scalar.  Also hands back 1/r of the column top.
+// when T2 (pairs beyond rt2_t2).  rt2 = ut^2 + rh, qY = q2y Y2.  The SFU
+// operations stay scalar.  Also hands back 1/r of the column top.
 template <bool T2>
-__device__ __forceinline__ float2 col_unit2(float2 X2, float2 Y2, float2 rh, float2 ut,
-                                            float2 rt2, float2 th, const IConst& k,
+__device__ __forceinline__ float2 col_unit2(float2 X2, float2 Y2, float2 qY, float2 rh,
+                                            float2 ut, float2 rt2, float2 th, const IConst& k,
                                             float2* it_out) {
-  const float2 Q2 = __ffma2_rn(make_float2(k.q2x, k.q2x), X2, __fmul2_rn(make_float2(k.q2y, k.q2y), Y2));
+  const float2 Q2 = __ffma2_rn(make_float2(k.q2x, k.q2x), X2, qY);
   const float2 ub = __fadd2_rn(ut, th);
   const float2 rb2 = __ffma2_rn(ub, ub, rh);
   const float2 it = make_float2(rsqrt_ftz(rt2.x), rsqrt_ftz(rt2.y));
@@ -230,7 +240,7 @@ __device__ __forceinline__ float2 col_unit2(float2 X2, float2 Y2, float2 rh, flo
   const float2 itb = __fmul2_rn(it, ib);
   const float2 num = __fmul2_rn(__fmul2_rn(th, __fadd2_rn(ut, ub)), __fmul2_rn(itb, itb));
   const float2 den = __fadd2_rn(it, ib);
-  const float2 L = make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
+  const float2 L = make_float2(div_ftz(num.x, den.x), div_ftz(num.y, den.y));
   // the corrections it^5 (Q0 rt^2 + Q2) + it^9 (P0 rt^4 + P2 rt^2 + P4) at the
   // top (and the same at the bottom), with rt^2 it^2 = 1 folded in:
   //   it^3 (Q0 + it^2 ((Q2 + P0) + it^2 (P2 + it^2 P4)))
@@ -261,8 +271,14 @@ __device__ __forceinline__ float2 col_unit2(float2 X2, float2 Y2, float2 rh, flo
 // never runs.
 // FACE: the top-face integral instead of the column integral (the depth
 // directional derivative, with the columns weighted by rho * direction).
+//
+// Bound by the FMA pipe (a column pair takes about 34 packed operations and six
+// special-function results).  A block of columns in one row forms the terms of
+// Y once, quotients skip the subnormal scaling, and twenty warps at 96 registers
+// do not spill: 128x128 columns, 64x64 stations 109 -> 91 us (32 warps at 64
+// registers 96 us).
 template <bool FACE>
-__global__ void __launch_bounds__(IF_TS, 8)
+__global__ void __launch_bounds__(IF_TS, 5)
     iface_far_fwd(IConst k, int ns, const IStation* __restrict__ sf, const int2* __restrict__ si,
                   const float4* __restrict__ cf, const uint32_t* __restrict__ mask,
                   const int* __restrict__ anynear, const int* __restrict__ perm, int chunk_len,
@@ -337,31 +353,41 @@ __global__ void __launch_bounds__(IF_TS, 8)
       const float gy = gap(fmaf((float)(hi.y - yb), k.dyn, st.ey), fmaf((float)(hi.y - ya), k.dyn, st.ey));
       const float gz = fmaxf(0.f, st.zs + s_tmin[q0 / IF_SUB]);
       const bool t2 = __all_sync(__activemask(), fmaf(gz, gz, fmaf(gx, gx, gy * gy)) >= k.rt2_t2);
-      auto run = [&](auto t2c) {
-        constexpr bool T2 = decltype(t2c)::value;
+      // the terms of Y, of columns in row iy
+      auto row = [&](float2 ny2, float2* Y2, float2* qY, float2* cbY) {
+        const float2 Y = __ffma2_rn(__fadd2_rn(hy2, ny2), dyn2, ey2);
+        *Y2 = __fmul2_rn(Y, Y);
+        *qY = __fmul2_rn(make_float2(k.q2y, k.q2y), *Y2);
+        *cbY = __fmul2_rn(*Y2, make_float2(k.face.cB, k.face.cB));
+      };
+      // ROW: the block's columns lie in one row, whose terms of Y are formed once
+      auto run = [&](auto t2c, auto rowc) {
+        constexpr bool T2 = decltype(t2c)::value, ROW = decltype(rowc)::value;
+        float2 Y2, qY, cbY;
+        if (ROW) row(make_float2(-(float)ya, -(float)ya), &Y2, &qY, &cbY);
         float2 g = make_float2(0.f, 0.f);  // plain sums over IF_SUB columns, Kahan across
 #pragma unroll 4
         for (int q = q0; q < qe; q += 2) {
           // columns q and q+1 (past the end of the tile: a padding column)
           const float2 nx2 = *reinterpret_cast<const float2*>(s_nx + q);
-          const float2 ny2 = *reinterpret_cast<const float2*>(s_ny + q);
           const float2 X = __ffma2_rn(__fadd2_rn(hx2, nx2), dxn2, ex2);
-          const float2 Y = __ffma2_rn(__fadd2_rn(hy2, ny2), dyn2, ey2);
-          const float2 X2 = __fmul2_rn(X, X), Y2 = __fmul2_rn(Y, Y), rh = __fadd2_rn(X2, Y2);
+          if (!ROW) row(*reinterpret_cast<const float2*>(s_ny + q), &Y2, &qY, &cbY);
+          const float2 X2 = __fmul2_rn(X, X), rh = __fadd2_rn(X2, Y2);
           const float2 ut = __fadd2_rn(zs2, *reinterpret_cast<const float2*>(s_top + q));
           const float2 rt2 = __ffma2_rn(ut, ut, rh);
           const float2 th = *reinterpret_cast<const float2*>(s_th + q);
           float2 itop, u;
           if (FACE) {
             itop = make_float2(rsqrt_ftz(rt2.x), rsqrt_ftz(rt2.y));
-            u = face_unit_far2<T2>(X2, Y2, ut, itop, k.face);
+            u = face_unit_far2<T2>(X2, Y2, cbY, ut, itop, k.face);
           } else {
-            u = col_unit2<T2>(X2, Y2, rh, ut, rt2, th, k, &itop);
+            u = col_unit2<T2>(X2, Y2, qY, rh, ut, rt2, th, k, &itop);
           }
           float2 v = __fmul2_rn(*reinterpret_cast<const float2*>(s_w + q), u);
           if (warp_near) {
             // near columns contribute through the double path: select, which
             // also drops a NaN
+            const float2 ny2 = *reinterpret_cast<const float2*>(s_ny + q);
             const int ixa = -(int)nx2.x, iya = -(int)ny2.x, ixb = -(int)nx2.y, iyb = -(int)ny2.y;
             if (ixa >= wx0 && ixa <= wx1 && iya >= wy0 && iya <= wy1 &&
                 near_bit(mask, s, ixa - wx0 + wbw * (iya - wy0), k))
@@ -374,10 +400,19 @@ __global__ void __launch_bounds__(IF_TS, 8)
         }
         acc.add(g.x + g.y);
       };
-      if (t2)
-        run(std::true_type{});
-      else
-        run(std::false_type{});
+      // a padding column of a one-row block takes the row's Y: it stays IF_FAR
+      // away in X
+      if (ya == yb) {
+        if (t2)
+          run(std::true_type{}, std::true_type{});
+        else
+          run(std::false_type{}, std::true_type{});
+      } else {
+        if (t2)
+          run(std::true_type{}, std::false_type{});
+        else
+          run(std::false_type{}, std::false_type{});
+      }
     }
   }
   if (active) partial[(size_t)blockIdx.y * ns + s] = acc.value();
@@ -416,16 +451,75 @@ __global__ void iface_near_fwd(IConst k, IMeshDesc m, int ns, const double* __re
   if (lane == 0) out[s] = acc;
 }
 
-__global__ void iface_finalize(int ns, int nchunks, const double* __restrict__ partial,
-                               double far_scale, const double* __restrict__ near, double G5,
-                               double* __restrict__ gz) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ns) return;
+// What the misfit takes from the forward's last kernel: r = gz - data (also as
+// the float that the far adjoint reads) and 0.5 * sum r^2.
+struct IfMisfit {
+  const double* data;
+  double* r;
+  IStation* sf;      // null: no float copy
+  double* misfit;
+  double* part;      // [blocks] sums of r^2
+  unsigned* ticket;  // zeroed before: the block that takes the last one adds the parts
+};
+
+// gz[s] = G5 * (far_scale * sum_c partial[c][s] + near[s]): 32 stations per
+// block, FIN_Y threads each over the chunks, summed in a fixed order (a thread
+// per station over all chunks is one chain of dependent loads: 11.5 us at 64
+// chunks, 5 now).  MISFIT: the residual and the misfit too (a kernel of one block
+// for them took 9 us for 4,096 stations and 17 us for 16,384).
+constexpr int FIN_Y = 16;
+template <bool MISFIT>
+__global__ void __launch_bounds__(32 * FIN_Y)
+    iface_finalize(int ns, int nchunks, const double* __restrict__ partial, double far_scale,
+                   const double* __restrict__ near, double G5, double* __restrict__ gz,
+                   IfMisfit mf) {
+  __shared__ double sm[FIN_Y][33];
+  __shared__ bool last;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int s = blockIdx.x * 32 + x;
   double f = 0.0;
-  for (int c = 0; c < nchunks; c++) f += partial[(size_t)c * ns + s];
-  double g = far_scale * f;
-  if (near) g += near[s];
-  gz[s] = G5 * g;
+  if (s < ns) {
+#pragma unroll 4
+    for (int c = y; c < nchunks; c += FIN_Y) f += partial[(size_t)c * ns + s];
+  }
+  sm[y][x] = f;
+  __syncthreads();
+  if (y == 0) {
+    for (int q = 1; q < FIN_Y; q++) f += sm[q][x];
+    double r2 = 0.0;
+    if (s < ns) {
+      double g = far_scale * f;
+      if (near) g += near[s];
+      const double v = G5 * g;
+      gz[s] = v;
+      if (MISFIT) {
+        const double r = v - mf.data[s];
+        mf.r[s] = r;
+        if (mf.sf) mf.sf[s].r = (float)r;
+        r2 = r * r;
+      }
+    }
+    if (MISFIT) {
+      r2 = warp_sum_d(r2);
+      if (x == 0) {
+        mf.part[blockIdx.x] = r2;
+        __threadfence();
+        last = atomicAdd(mf.ticket, 1u) == gridDim.x - 1;
+      }
+    }
+  }
+  if (!MISFIT) return;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double a = 0.0;
+  for (unsigned q = threadIdx.x; q < gridDim.x; q += 32 * FIN_Y) a += __ldcg(mf.part + q);
+  a = warp_sum_d(a);
+  if (x == 0) sm[y][0] = a;
+  __syncthreads();
+  if (threadIdx.x) return;
+  for (int q = 1; q < FIN_Y; q++) a += sm[q][0];
+  *mf.misfit = 0.5 * a;
 }
 
 // ---- forward, plain double --------------------------------------------------
@@ -455,7 +549,13 @@ __global__ void __launch_bounds__(64)
 }
 
 // ---- adjoint, far (thread per column) --------------------------------------
-__global__ void __launch_bounds__(IF_TS, 8)
+// ROWS: the block's columns lie in at most IF_ROWS rows; a station's terms of Y
+// are formed once per row and block, in shared memory (with fewer columns in x a
+// block has too many rows for that to pay, and each pair forms them).  Bound by
+// the FMA pipe, as the forward: 128x128 columns, 64x64 stations 155 -> 124 us;
+// with 256x256 columns and 128x128 stations both directions 3.47 -> 2.82 ms.
+template <bool ROWS>
+__global__ void __launch_bounds__(IF_TS, 5)
     iface_far_adj(IConst k, int ns, const IStation* __restrict__ sf, const int2* __restrict__ si,
                   const float4* __restrict__ cf, const uint32_t* __restrict__ mask,
                   const int* __restrict__ anynear, int chunk_len, double* __restrict__ p_rho,
@@ -470,6 +570,7 @@ __global__ void __launch_bounds__(IF_TS, 8)
   __shared__ __align__(8) float s_hy[IF_TILE + 2];
   __shared__ int2 s_i[IF_TILE + 2];
   __shared__ int s_nf[IF_TILE + 2];  // the station has a near column
+  __shared__ __align__(8) float s_y[ROWS ? 3 : 1][ROWS ? IF_ROWS : 1][IF_TILE + 2];  // Y2, q2y Y2, cB Y2
   const int c = blockIdx.x * IF_TS + threadIdx.x;
   const bool active = c < k.ncols;
   const int ix = active ? c % k.nx : 0, iy = active ? c / k.nx : 0;
@@ -480,11 +581,15 @@ __global__ void __launch_bounds__(IF_TS, 8)
   // this block's slice of the stations (grid.y)
   const int s0 = blockIdx.y * chunk_len, s1 = min(ns, s0 + chunk_len);
   Kahan ar, ad;
+  const int row0 = blockIdx.x * IF_TS / k.nx, myrow = iy - row0;
   for (int t0 = s0; t0 < s1; t0 += IF_TILE) {
     __syncthreads();
+    int nf = 0;
     for (int q = threadIdx.x; q < IF_TILE + 2; q += IF_TS) {
       const bool ok = t0 + q < s1;
-      IStation z = {0.f, 0.f, 0.f, 0.f};
+      // a padding station has no residual and lies far above: its terms are
+      // finite and add zero
+      IStation z = {0.f, 0.f, IF_FAR, 0.f};
       const IStation f = ok ? sf[t0 + q] : z;
       const int2 h = ok ? si[t0 + q] : make_int2(0, 0);
       s_ex[q] = f.ex;
@@ -495,42 +600,62 @@ __global__ void __launch_bounds__(IF_TS, 8)
       s_hy[q] = (float)h.y;
       s_i[q] = h;
       s_nf[q] = ok ? anynear[t0 + q] : 0;
+      nf |= s_nf[q];
+      if (ROWS) {
+#pragma unroll
+        for (int j = 0; j < IF_ROWS; j++) {
+          const float Y = fmaf((float)h.y - (float)(row0 + j), k.dyn, f.ey);
+          const float Y2 = __fmul_rn(Y, Y);
+          s_y[0][j][q] = Y2;
+          s_y[1][j][q] = __fmul_rn(k.q2y, Y2);
+          s_y[2][j][q] = __fmul_rn(Y2, k.face.cB);
+        }
+      }
     }
-    __syncthreads();
+    const bool tile_near = __syncthreads_or(nf);
     if (!active) continue;
     const int cnt = min(IF_TILE, s1 - t0);
     float2 gr = make_float2(0.f, 0.f), gd = make_float2(0.f, 0.f);  // 32 stations, Kahan across
 #pragma unroll 4
     for (int q = 0; q < cnt; q += 2) {
-      // stations q and q+1 (the second is dropped past the end of the tile)
+      // stations q and q+1 (past the end of the tile: a padding station)
       const float2 hx = *reinterpret_cast<const float2*>(s_hx + q);
-      const float2 hy = *reinterpret_cast<const float2*>(s_hy + q);
       const float2 X = __ffma2_rn(__fadd2_rn(hx, nix2), dxn2,
                                   *reinterpret_cast<const float2*>(s_ex + q));
-      const float2 Y = __ffma2_rn(__fadd2_rn(hy, niy2), dyn2,
-                                  *reinterpret_cast<const float2*>(s_ey + q));
-      const float2 X2 = __fmul2_rn(X, X), Y2 = __fmul2_rn(Y, Y), rh = __fadd2_rn(X2, Y2);
+      float2 Y2, qY, cbY;
+      if (ROWS) {
+        Y2 = *reinterpret_cast<const float2*>(&s_y[0][myrow][q]);
+        qY = *reinterpret_cast<const float2*>(&s_y[1][myrow][q]);
+        cbY = *reinterpret_cast<const float2*>(&s_y[2][myrow][q]);
+      } else {
+        const float2 hy = *reinterpret_cast<const float2*>(s_hy + q);
+        const float2 Y = __ffma2_rn(__fadd2_rn(hy, niy2), dyn2,
+                                    *reinterpret_cast<const float2*>(s_ey + q));
+        Y2 = __fmul2_rn(Y, Y);
+        qY = __fmul2_rn(make_float2(k.q2y, k.q2y), Y2);
+        cbY = __fmul2_rn(Y2, make_float2(k.face.cB, k.face.cB));
+      }
+      const float2 X2 = __fmul2_rn(X, X), rh = __fadd2_rn(X2, Y2);
       const float2 ut = __fadd2_rn(*reinterpret_cast<const float2*>(s_zs + q), cy2);
       const float2 rt2 = __ffma2_rn(ut, ut, rh);
       float2 itop, u, f;
       // second order when every lane's pairs are far enough (warp-uniform)
       if (__all_sync(__activemask(), fminf(rt2.x, rt2.y) >= k.rt2_t2)) {
-        u = col_unit2<true>(X2, Y2, rh, ut, rt2, cz2, k, &itop);
-        f = face_unit_far2<true>(X2, Y2, ut, itop, k.face);
+        u = col_unit2<true>(X2, Y2, qY, rh, ut, rt2, cz2, k, &itop);
+        f = face_unit_far2<true>(X2, Y2, cbY, ut, itop, k.face);
       } else {
-        u = col_unit2<false>(X2, Y2, rh, ut, rt2, cz2, k, &itop);
-        f = face_unit_far2<false>(X2, Y2, ut, itop, k.face);
+        u = col_unit2<false>(X2, Y2, qY, rh, ut, rt2, cz2, k, &itop);
+        f = face_unit_far2<false>(X2, Y2, cbY, ut, itop, k.face);
       }
       const float2 r = *reinterpret_cast<const float2*>(s_r + q);
       float2 vr = __fmul2_rn(r, u), vd = __fmul2_rn(r, f);
       // near pairs go through the double path: select, which also drops a
       // NaN.  Every lane has the same stations, so the test is uniform.
-      if (s_nf[q] | s_nf[q + 1]) {
+      if (tile_near && (s_nf[q] | s_nf[q + 1])) {
         const int2 ha = s_i[q], hb = s_i[q + 1];
         if (is_near(mask, t0 + q, ha.x, ha.y, ix, iy, k)) vr.x = vd.x = 0.f;
         if (q + 1 < cnt && is_near(mask, t0 + q + 1, hb.x, hb.y, ix, iy, k)) vr.y = vd.y = 0.f;
       }
-      if (q + 1 >= cnt) vr.y = vd.y = 0.f;  // the padding station
       gr = __fadd2_rn(gr, vr);
       gd = __fadd2_rn(gd, vd);
       if ((q & 30) == 30) {
@@ -557,6 +682,7 @@ __global__ void iface_far_adj_finalize(long long nc, int nchunks, const double* 
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= nc) return;
   double r = 0.0, d = 0.0;
+#pragma unroll 4
   for (int q = 0; q < nchunks; q++) {
     r += p_rho[(size_t)q * nc + c];
     d += p_dep[(size_t)q * nc + c];
@@ -640,26 +766,14 @@ __global__ void iface_f64_adj_finalize(long long nc, int nchunks, const double* 
   if (g_dep) g_dep[c] = -G5 * rho[c] * b;
 }
 
-// residual and misfit: r = gz - data, misfit = 0.5 * sum r^2 (one block,
-// fixed reduction order).
-__global__ void residual_kernel(int ns, const double* __restrict__ gz,
-                                const double* __restrict__ data, double* __restrict__ r,
-                                double* __restrict__ misfit) {
-  __shared__ double red[1024];
-  double a = 0.0;
-  for (int s = threadIdx.x; s < ns; s += blockDim.x) {
-    double v = gz[s] - data[s];
-    r[s] = v;
-    a += v * v;
-  }
-  red[threadIdx.x] = a;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *misfit = 0.5 * red[0];
-}
+// What a mixed forward prepares and the adjoint of the same call takes over.
+struct IfPrep {
+  IStation* sf;  // the residuals are in place once the forward's finalize has run
+  int2* si;
+  float4* cf;
+  uint32_t* mask;
+  int* anynear;
+};
 
 int chunks_for(long long units, int tiles, int num_sms, int minlen, int* len, int per_sm = 8) {
   long long want = std::max(1LL, ((long long)per_sm * std::max(num_sms, 1)) / std::max(tiles, 1));
@@ -670,18 +784,12 @@ int chunks_for(long long units, int tiles, int num_sms, int minlen, int* len, in
   return (int)((units + *len - 1) / *len);
 }
 
-// Station slices of the mixed adjoint: about twelve waves of blocks of
-// column tiles x slices (blocks finish unevenly; three waves left the end of
-// the launch half idle), slices of at least one shared-memory tile.
+// Station slices of the mixed adjoint: about 96 blocks per SM of column tiles
+// x slices (blocks finish unevenly; 24 left the end of the launch half idle),
+// slices of at least one shared-memory tile.
 int iface_adj_chunks(int ns, long long nc, int num_sms, int* len) {
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, iface_far_adj, IF_TS, 0) != cudaSuccess ||
-      occ < 1) {
-    cudaGetLastError();
-    occ = 1;
-  }
   const long long tiles = std::max(1LL, (nc + IF_TS - 1) / IF_TS);
-  long long ch = std::max(1LL, 12LL * occ * std::max(num_sms, 1) / tiles);
+  long long ch = std::max(1LL, 96LL * std::max(num_sms, 1) / tiles);
   ch = std::min(ch, std::max(1LL, (long long)(ns + IF_TILE - 1) / IF_TILE));
   ch = std::min(ch, 65535LL);
   *len = (int)((std::max(ns, 1) + ch - 1) / ch);
@@ -724,10 +832,16 @@ template <bool FACE>
 static int iface_forward_impl(ztm_ctx* c, const IMeshDesc& m, const double* d_depth,
                               const double* d_rho, const double* d_vdep, int ns,
                               const double* d_sxyz, double* d_gz, double G, int precision,
-                              const ztm_opts* o, WsCarver& wc) {
+                              const ztm_opts* o, WsCarver& wc, IfMisfit* mf = nullptr,
+                              IfPrep* prep = nullptr) {
   const double G5 = G * 1.0e5;
   const double sign = FACE ? -1.0 : 1.0;
   const long long nc = (long long)m.nx * m.ny;
+  auto finalize = [&](int chunks, const double* partial, double far_scale, const double* near) {
+    auto* fn = mf ? iface_finalize<true> : iface_finalize<false>;
+    fn<<<(ns + 31) / 32, 32 * FIN_Y, 0, c->stream>>>(ns, chunks, partial, far_scale, near,
+                                                     sign * G5, d_gz, mf ? *mf : IfMisfit{});
+  };
   if (precision == ZTM_PREC_FP64) {
     int tiles = std::max(1, (ns + 63) / 64), len;
     int ch = chunks_for(nc, tiles, c->num_sms, 64, &len);
@@ -737,8 +851,8 @@ static int iface_forward_impl(ztm_ctx* c, const IMeshDesc& m, const double* d_de
       iface_f64_fwd<FACE><<<dim3(tiles, ch), 64, 0, c->stream>>>(m, ns, d_sxyz, d_depth, d_rho,
                                                                  d_vdep, len, partial);
     }
-    iface_finalize<<<(ns + 255) / 256, 256, 0, c->stream>>>(ns, ch, partial, 1.0, nullptr,
-                                                            sign * G5, d_gz);
+    if (mf) cudaMemsetAsync(mf->ticket, 0, sizeof(unsigned), c->stream);
+    finalize(ch, partial, 1.0, nullptr);
     c->launches += 2;
     return ztm_after_launch(c, "interface FP64 kernels");
   }
@@ -749,17 +863,20 @@ static int iface_forward_impl(ztm_ctx* c, const IMeshDesc& m, const double* d_de
   int2* si = wc.take<int2>(ns);
   float4* cf = wc.take<float4>(nc);
   double* near = wc.take<double>(ns);
-  iface_station_prep<<<(ns + 127) / 128, 128, 0, c->stream>>>(m, k.L0, ns, d_sxyz, nullptr, sf,
-                                                              si);
-  int* perm = wc.take<int>(ns);
-  if (int rc = ztm_station_order(c, c->stream, ns, reinterpret_cast<const int*>(si), 2, m.nx, m.ny,
-                                 perm, wc))
-    return rc;
-  iface_col_prep<<<(unsigned)((nc + 255) / 256), 256, 0, c->stream>>>(m, k.L0, d_depth, d_rho,
-                                                                   FACE ? d_vdep : nullptr, cf);
+  iface_station_prep<<<(ns + 127) / 128, 128, 0, c->stream>>>(m, k.L0, ns, d_sxyz, nullptr, sf, si,
+                                                              mf ? mf->ticket : nullptr);
   uint32_t* mask = wc.take<uint32_t>((size_t)ns * k.words);
   int* anynear = wc.take<int>((size_t)ns);
-  iface_near_mask<<<(ns + 3) / 4, 128, 0, c->stream>>>(k, ns, d_sxyz, si, d_depth, mask, anynear);
+  int* perm = wc.take<int>(ns);
+  // the columns and near masks on the side stream, beside the station order
+  ztm_fork(c);
+  iface_col_prep<<<(unsigned)((nc + 255) / 256), 256, 0, c->aux>>>(m, k.L0, d_depth, d_rho,
+                                                                   FACE ? d_vdep : nullptr, cf);
+  iface_near_mask<<<(ns + 3) / 4, 128, 0, c->aux>>>(k, ns, d_sxyz, si, d_depth, mask, anynear);
+  const int order_rc = ztm_station_order(c, c->stream, ns, reinterpret_cast<const int*>(si), 2,
+                                         m.nx, m.ny, perm, wc);
+  ztm_join(c);
+  if (order_rc) return order_rc;
   // double near columns on the side stream, concurrently with the float far field
   ztm_fork(c);
   {
@@ -779,8 +896,9 @@ static int iface_forward_impl(ztm_ctx* c, const IMeshDesc& m, const double* d_de
   // the column integral is in units of L0 (x dx dy / L0^2), the face
   // integral is dimensionless (x dx dy / L0^2)
   const double far_scale = (FACE ? 1.0 : k.L0) * (double)k.dxn * k.dyn;
-  iface_finalize<<<(ns + 255) / 256, 256, 0, c->stream>>>(ns, ch, partial, far_scale, near,
-                                                          sign * G5, d_gz);
+  if (mf) mf->sf = sf;
+  finalize(ch, partial, far_scale, near);
+  if (prep) *prep = IfPrep{sf, si, cf, mask, anynear};
   c->launches += 6;
   return ztm_after_launch(c, "interface mixed kernels");
 }
@@ -800,10 +918,10 @@ int ztm_launch_iface_jvp(ztm_ctx* c, const IMeshDesc& m, const double* d_depth,
                                   o, wc);
 }
 
-int ztm_launch_iface_adj(ztm_ctx* c, const IMeshDesc& m, const double* d_depth,
-                         const double* d_rho, int ns, const double* d_sxyz, const double* d_res,
-                         double* d_grho, double* d_gdep, double G, int precision,
-                         const ztm_opts* o, WsCarver& wc) {
+static int iface_adjoint_impl(ztm_ctx* c, const IMeshDesc& m, const double* d_depth,
+                              const double* d_rho, int ns, const double* d_sxyz,
+                              const double* d_res, double* d_grho, double* d_gdep, double G,
+                              int precision, const ztm_opts* o, WsCarver& wc, const IfPrep* prep) {
   const double G5 = G * 1.0e5;
   const long long nc = (long long)m.nx * m.ny;
   if (ns == 0) {
@@ -829,36 +947,55 @@ int ztm_launch_iface_adj(ztm_ctx* c, const IMeshDesc& m, const double* d_depth,
   const double nq = (o && o->near_q > 0) ? o->near_q : 6.0;
   IConst k = make_iconst(m, nq);
   if (k.words > 64) return ztm_fail(c, ZTM_ERR_RANGE, "near_q too large for the interface window");
-  IStation* sf = wc.take<IStation>(ns);
-  int2* si = wc.take<int2>(ns);
-  float4* cf = wc.take<float4>(nc);
-  iface_station_prep<<<(ns + 127) / 128, 128, 0, c->stream>>>(m, k.L0, ns, d_sxyz, d_res, sf, si);
-  iface_col_prep<<<(unsigned)((nc + 255) / 256), 256, 0, c->stream>>>(m, k.L0, d_depth, d_rho,
-                                                                   nullptr, cf);
+  IfPrep p;
+  if (prep) {
+    p = *prep;
+  } else {
+    p.sf = wc.take<IStation>(ns);
+    p.si = wc.take<int2>(ns);
+    p.cf = wc.take<float4>(nc);
+    p.mask = wc.take<uint32_t>((size_t)ns * k.words);
+    p.anynear = wc.take<int>((size_t)ns);
+    iface_station_prep<<<(ns + 127) / 128, 128, 0, c->stream>>>(m, k.L0, ns, d_sxyz, d_res, p.sf,
+                                                                p.si, nullptr);
+    iface_col_prep<<<(unsigned)((nc + 255) / 256), 256, 0, c->stream>>>(m, k.L0, d_depth, d_rho,
+                                                                     nullptr, p.cf);
+    iface_near_mask<<<(ns + 3) / 4, 128, 0, c->stream>>>(k, ns, d_sxyz, p.si, d_depth, p.mask,
+                                                         p.anynear);
+    c->launches += 3;
+  }
   // face integral is dimensionless: dx dy / L0^2 * (u / r^3 in 1/L0^2 units)
   const double sc_rho = G5 * k.L0 * (double)k.dxn * k.dyn;
   const double sc_dep = G5 * (double)k.dxn * k.dyn;
-  uint32_t* mask = wc.take<uint32_t>((size_t)ns * k.words);
-  int* anynear = wc.take<int>((size_t)ns);
-  iface_near_mask<<<(ns + 3) / 4, 128, 0, c->stream>>>(k, ns, d_sxyz, si, d_depth, mask, anynear);
   int alen;
   const int ach = iface_adj_chunks(ns, nc, c->num_sms, &alen);
   double* p_rho = wc.take<double>((size_t)ach * nc);
   double* p_dep = wc.take<double>((size_t)ach * nc);
   {
     ZtmProf prof_(c, "iface_far");
-    iface_far_adj<<<dim3((unsigned)((nc + IF_TS - 1) / IF_TS), ach), IF_TS, 0, c->stream>>>(
-        k, ns, sf, si, cf, mask, anynear, alen, p_rho, p_dep);
+    // rows that IF_TS columns can touch
+    const bool rows = (IF_TS - 2) / m.nx + 2 <= IF_ROWS;
+    const dim3 grid((unsigned)((nc + IF_TS - 1) / IF_TS), ach);
+    (rows ? iface_far_adj<true> : iface_far_adj<false>)<<<grid, IF_TS, 0, c->stream>>>(
+        k, ns, p.sf, p.si, p.cf, p.mask, p.anynear, alen, p_rho, p_dep);
   }
   iface_far_adj_finalize<<<(unsigned)((nc + 255) / 256), 256, 0, c->stream>>>(
       nc, ach, p_rho, p_dep, sc_rho, sc_dep, d_grho, d_gdep);
   {  // after the far kernel has written every entry: double atomics add the near pairs
     ZtmProf prof_(c, "iface_near");
     iface_near_adj<<<(ns + IF_NEAR_WPB - 1) / IF_NEAR_WPB, IF_NEAR_WPB * 32, 0, c->stream>>>(
-        k, m, ns, d_sxyz, si, d_depth, d_rho, d_res, mask, G5, d_grho, d_gdep);
+        k, m, ns, d_sxyz, p.si, d_depth, d_rho, d_res, p.mask, G5, d_grho, d_gdep);
   }
-  c->launches += 6;
+  c->launches += 3;
   return ztm_after_launch(c, "interface mixed adjoint");
+}
+
+int ztm_launch_iface_adj(ztm_ctx* c, const IMeshDesc& m, const double* d_depth,
+                         const double* d_rho, int ns, const double* d_sxyz, const double* d_res,
+                         double* d_grho, double* d_gdep, double G, int precision,
+                         const ztm_opts* o, WsCarver& wc) {
+  return iface_adjoint_impl(c, m, d_depth, d_rho, ns, d_sxyz, d_res, d_grho, d_gdep, G, precision,
+                            o, wc, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -893,7 +1030,7 @@ extern "C" int ztm_gfm_interface_misfit(ztm_ctx* c, const ztm_imesh* mesh, const
     }
   } restore{prev, c->device};
   size_t need = 2 * WsCarver::need(nc * 8) + WsCarver::need((size_t)ns * 24) +
-                4 * WsCarver::need((size_t)ns * 8) + 2 * WsCarver::need(nc * 8) + 256 +
+                5 * WsCarver::need((size_t)ns * 8) + 2 * WsCarver::need(nc * 8) + 512 +
                 ztm_iface_ws(m, ns, prec, c->num_sms) + 4096;
   int rc = ztm_ws_reserve(c, need);
   if (rc) return rc;
@@ -905,6 +1042,8 @@ extern "C" int ztm_gfm_interface_misfit(ztm_ctx* c, const ztm_imesh* mesh, const
   double* s_gz = wc.take<double>(ns);
   double* s_r = wc.take<double>(ns);
   double* s_mis = wc.take<double>(1);
+  double* s_part = wc.take<double>((ns + 31) / 32);
+  unsigned* s_ticket = wc.take<unsigned>(1);
   double* s_gr = wc.take<double>(nc);
   double* s_gd = wc.take<double>(nc);
   const void *pd, *pr, *px, *pdat;
@@ -913,18 +1052,18 @@ extern "C" int ztm_gfm_interface_misfit(ztm_ctx* c, const ztm_imesh* mesh, const
   if ((rc = ztm_stage_in(c, sxyz, (size_t)ns * 24, dev, s_xyz, &px))) return rc;
   if ((rc = ztm_stage_in(c, data, (size_t)ns * 8, dev, s_dat, &pdat))) return rc;
   double* ogz = (dev && gz) ? gz : s_gz;
+  // the residual and misfit come out of the forward's last kernel; the mixed
+  // adjoint takes over what the forward prepared
+  IfMisfit mf{(const double*)pdat, s_r, nullptr, dev ? misfit : s_mis, s_part, s_ticket};
+  IfPrep prep;
   rc = iface_forward_impl<false>(c, m, (const double*)pd, (const double*)pr, nullptr, ns,
-                                 (const double*)px, ogz,
-                          G, prec, o, wc);
+                                 (const double*)px, ogz, G, prec, o, wc, &mf, &prep);
   if (rc) return rc;
-  double* omis = dev ? misfit : s_mis;
-  residual_kernel<<<1, 1024, 0, c->stream>>>(ns, ogz, (const double*)pdat, s_r, omis);
-  c->launches++;
   double* ogr = g_rho ? (dev ? g_rho : s_gr) : nullptr;
   double* ogd = g_depth ? (dev ? g_depth : s_gd) : nullptr;
   if (ogr || ogd) {
-    rc = ztm_launch_iface_adj(c, m, (const double*)pd, (const double*)pr, ns, (const double*)px,
-                              s_r, ogr, ogd, G, prec, o, wc);
+    rc = iface_adjoint_impl(c, m, (const double*)pd, (const double*)pr, ns, (const double*)px, s_r,
+                            ogr, ogd, G, prec, o, wc, prec == ZTM_PREC_FP64 ? nullptr : &prep);
     if (rc) return rc;
   }
   if ((rc = ztm_cuda_check(c, cudaGetLastError(), "interface misfit kernels"))) return rc;
