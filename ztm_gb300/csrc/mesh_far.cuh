@@ -57,11 +57,11 @@ __device__ __forceinline__ float2 far_group(const float* col, int l0, float fl,
 // All layers of one column: groups [0, lmask) with the near mask, full
 // groups up to nz8 without, a masked tail group if nz is not a multiple of 8.
 // Plain float sums over 32 layers (two lanes of 16), compensated across.
-template <bool T2>
+template <bool T2, class ACC>
 __device__ __forceinline__ void far_column(const float* col, int lmask, int nz8, int nz,
                                            const float2 (&Zb)[4], float2 zstep,
                                            const ColPoly2& cp2, float2 c2t, int elo,
-                                           unsigned espan, Kahan& acc) {
+                                           unsigned espan, ACC& acc) {
   float2 g = make_float2(0.f, 0.f);
   int l0 = 0;
   float fl = 0.f;
@@ -146,10 +146,11 @@ __device__ __forceinline__ float2 far_group_pair(const float* colA, const float*
 // Layers 0 .. nl - 1 of two columns (nl a multiple of 8: nz, or the padded
 // nzp where the padding layers' K is finite): plain float sums over 16
 // layers of both (32 terms), compensated across.
+template <class ACC>
 __device__ __forceinline__ void far_column_pair(const float* colA, const float* colB, int nl,
                                                 const float2 (&Zb)[4], float2 zstep,
                                                 const ColPoly2& cpA, float2 c2tA,
-                                                const ColPoly2& cpB, float2 c2tB, Kahan& acc) {
+                                                const ColPoly2& cpB, float2 c2tB, ACC& acc) {
   int l0 = 0;
   float fl = 0.f;
   const float2 z0 = make_float2(0.f, 0.f);
@@ -179,11 +180,14 @@ __device__ __forceinline__ void far_column_pair(const float* colA, const float* 
 // on dummy data) for the warp votes.
 // COUNT: add the (station, prism) slots this thread evaluates to cnt by
 // form: [0] sixth order, [1] second order, [2] second order by column pairs.
-template <bool COUNT>
+// PART: only the columns and column pairs that start in [qa, qb) are evaluated;
+// which columns form pairs is found from the stage's first column on, so that the
+// parts together make the same sequence of acc.add.
+template <bool COUNT, bool PART = false, class ACC = Kahan>
 __device__ __forceinline__ void far_stage(const short2* __restrict__ ivs, const MeshConst& k,
                                           const FarCoef& fc, const FarStation& t, int s, int Lm,
-                                          const float* rs, int cs, int ncol, Kahan& acc,
-                                          unsigned (&cnt)[3]) {
+                                          const float* rs, int cs, int ncol, ACC& acc,
+                                          unsigned (&cnt)[3], int qa = 0, int qb = 0) {
   const float2 zstep = make_float2(k.dzn, k.dzn);
   // Z of layers 2j, 2j+1 of a group at l0 = 0; a group at l0 adds l0 dz
   float2 Zb[4];
@@ -199,7 +203,7 @@ __device__ __forceinline__ void far_stage(const short2* __restrict__ ivs, const 
   // that K there is finite and the zero density adds nothing
   const bool pairs = nz8 == k.nz || __all_sync(0xffffffffu, t.izs < k.nz);
   int ix = cs % k.nx, iy = cs / k.nx;
-  for (int q = 0; q < ncol; q++) {
+  for (int q = 0; q < (PART ? min(ncol, qb) : ncol); q++) {
     // two unmasked second-order columns at once where the warp allows it
     if (pairs && q + 1 < ncol) {
       int ix1 = ix + 1, iy1 = iy;
@@ -217,6 +221,16 @@ __device__ __forceinline__ void far_stage(const short2* __restrict__ ivs, const 
       const bool nclB = ix1 >= t.nb.x0 && ix1 <= t.nb.x1 && iy1 >= t.nb.y0 && iy1 <= t.nb.y1;
       const bool unmasked = lm8 == 0 || !__any_sync(0xffffffffu, nclA || nclB);
       if (unmasked && __all_sync(0xffffffffu, fminf(rhA, rhB) >= k.rh_t2)) {
+        if (PART && q < qa) {
+          q++;
+          ix = ix1 + 1;
+          iy = iy1;
+          if (ix == k.nx) {
+            ix = 0;
+            ++iy;
+          }
+          continue;
+        }
         const float cA = fmaf(-fc.a1, rhA, fmaf(XA2, fc.cA, YA2 * fc.cB));
         const float cB = fmaf(-fc.a1, rhB, fmaf(XB2, fc.cA, YB2 * fc.cB));
         ColPoly2 cpA, cpB;
@@ -237,6 +251,13 @@ __device__ __forceinline__ void far_stage(const short2* __restrict__ ivs, const 
         }
         continue;
       }
+    }
+    if (PART && q < qa) {
+      if (++ix == k.nx) {
+        ix = 0;
+        ++iy;
+      }
+      continue;
     }
     const float X = fmaf((float)(t.ixs - ix), k.dxn, t.ex);
     const float Y = fmaf((float)(t.iys - iy), k.dyn, t.ey);

@@ -154,6 +154,7 @@ struct FarArgs {
   int tiles, chunks;  // work items: tiles x chunks
   int chunk_cols;     // columns per item
   int sc;             // columns per shared-memory stage
+  int group;          // stations per block of far_kernel (far_split_kernel)
   int* counter;       // next work item (zeroed before the launch)
   int n_near;         // near items, spread through the queue
   int near_units;     // (station, part) units per near item, a warp each
@@ -389,6 +390,94 @@ __global__ void __launch_bounds__(FAR_TS, 512 / FAR_TS) far_kernel(FarArgs a) {
       if (lane == 0 && v[j]) atomicAdd(&a.forms[j], v[j]);
     }
   }
+}
+
+// The mixed forward of few stations over a small mesh.  An item of far_kernel is
+// a warp's stations against a chunk of columns one after another; where that
+// makes fewer warps than the chip has quarters, the chain of columns is the
+// call's time (33x29x14 prisms, 63 stations: 60 warps, 60 us).  Here a block
+// takes 32 stations (a warp of far_kernel) and a chunk, its eight warps a part of
+// each stage's columns; they leave the sums that far_kernel would add to its
+// compensated sum in shared memory, and one warp adds them in the same order:
+// the same result, bit by bit.  Near units (a warp each) are blocks of the same
+// launch.
+constexpr int SPLIT_W = 8;                      // warps per block
+constexpr int SPLIT_SC = 32;                    // columns per stage, at most
+constexpr int SPLIT_CW = SPLIT_SC / SPLIT_W;    // columns per warp
+// sums of the columns that start in a warp's part: nzp/32 + 1 a column at most,
+// a pair that starts in the last one included
+__host__ __device__ constexpr int split_sums(int nzp) { return (SPLIT_CW + 1) * (nzp / 32 + 1); }
+size_t split_smem(int nzp) {
+  return (size_t)SPLIT_W * split_sums(nzp) * 32 * 4 + (size_t)SPLIT_SC * nzp * 4;
+}
+
+struct SumList {  // stands in for the compensated sum: what would be added to it
+  float* p;
+  int n = 0;
+  __device__ __forceinline__ void add(float x) { p[32 * n++] = x; }
+};
+
+__global__ void __launch_bounds__(32 * SPLIT_W, 2) far_split_kernel(FarArgs a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ int s_n[SPLIT_W];
+  const MeshConst& k = a.k;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_far = a.tiles * a.chunks;
+  if ((int)blockIdx.x >= n_far) {
+    const int u = ((int)blockIdx.x - n_far) * SPLIT_W + warp, s = u / a.nparts, part = u % a.nparts;
+    if (s >= a.ns) return;
+    double* out = a.near + (size_t)part * a.ns;
+    if (a.near_f64)
+      near_station<double, false>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho, out, lane, nullptr,
+                                  part, a.nparts);
+    else
+      near_station<float, false>(k, a.m, s, a.sxyz, a.si, a.iv, a.lr, a.rho, out, lane, nullptr,
+                                 part, a.nparts);
+    return;
+  }
+  const int nsum = split_sums(k.nzp);
+  float* list = reinterpret_cast<float*>(smem_raw);  // [warp][sum][lane]
+  float* stage = list + SPLIT_W * nsum * 32;
+  const FarCoef fc = k.fc;
+  const int tile = blockIdx.x % a.tiles, chunk = blockIdx.x / a.tiles;
+  const int slot = tile * 32 + lane;
+  const bool active = slot < a.ns;
+  const int s = active ? a.perm[slot] : 0;
+  meshfar::FarStation t = {0.f, 0.f, 0.f, 0, 0, 0, {1, 0, 1, 0, 1, 0}};
+  if (active) {
+    const float4 fv = a.sf[s];
+    const int4 i = a.si[s];
+    t.ex = fv.x; t.ey = fv.y; t.ez = fv.z;
+    t.ixs = i.x; t.iys = i.y; t.izs = i.z;
+    t.nb = near_box(i, k);
+  }
+  // lowest near layer of the stations of far_kernel's block
+  const int other = tile / (a.group / 32) * a.group;
+  int Lm = 0;
+  for (int q = other + lane; q < min(a.ns, other + a.group); q += 32)
+    Lm = max(Lm, near_box(a.si[a.perm[q]], k).l1 + 1);
+  Lm = min(__reduce_max_sync(0xffffffffu, Lm), k.nz);
+  const int c0 = chunk * a.chunk_cols, c1 = min(k.ncols, c0 + a.chunk_cols);
+  Kahan acc;
+  for (int cs = c0; cs < c1; cs += a.sc) {
+    const int ncol = min(a.sc, c1 - cs);
+    const float4* src = reinterpret_cast<const float4*>(a.rhoT + (size_t)cs * k.nzp);
+    for (int q = threadIdx.x; q < ncol * k.nzp / 4; q += 32 * SPLIT_W)
+      reinterpret_cast<float4*>(stage)[q] = src[q];
+    __syncthreads();
+    SumList sums{list + warp * nsum * 32 + lane};
+    unsigned c3[3];
+    const int cw = (a.sc + SPLIT_W - 1) / SPLIT_W;
+    meshfar::far_stage<false, true>(a.iv, k, fc, t, s, Lm, stage, cs, ncol, sums, c3, warp * cw,
+                                    warp * cw + cw);
+    if (lane == 0) s_n[warp] = sums.n;
+    __syncthreads();
+    if (warp == 0)
+      for (int w = 0; w < SPLIT_W; w++)
+        for (int j = 0; j < s_n[w]; j++) acc.add(list[(w * nsum + j) * 32 + lane]);
+    __syncthreads();
+  }
+  if (warp == 0 && active) a.partial[(size_t)chunk * a.ns + s] = acc.value();
 }
 
 // gz[s] = G5 * (far_scale * sum_c partial[c][s] + sum_q near[q][s]): 32 stations
@@ -855,6 +944,21 @@ int ztm_launch_prism(ztm_ctx* c, const MeshDesc& m, const double* d_rho, int ns,
     a.chunks = t.chunks;
     a.chunk_cols = t.chunk_cols;
     a.sc = t.sc;
+    // few warps of stations x chunks: the columns of each spread over a block.
+    // A call of 60 warps (33x29x14 prisms, 63 stations) 94 -> 58 us, 256 warps
+    // (64x64x32, 49) 111 -> 74, 313 (100x100x64, 64) 213 -> 94; at 1,024
+    // (64x64x16, 256) 102 -> 99, at 1,600 (40x40x40, 1,000) 150 against 179.
+    const int groups = (ns + 31) / 32;
+    if ((long long)groups * t.chunks <= 8LL * c->num_sms && t.sc <= SPLIT_SC &&
+        split_smem(k.nzp) <= 46 * 1024 && !a.poll_limit && !(c->count_forms && c->d_forms)) {
+      a.group = t.ts;
+      a.tiles = groups;
+      const long long units = (long long)ns * nparts;
+      const unsigned blocks = (unsigned)(groups * t.chunks + (units + SPLIT_W - 1) / SPLIT_W);
+      far_split_kernel<<<blocks, 32 * SPLIT_W, split_smem(k.nzp), c->stream>>>(a);
+      c->launches++;
+      return;
+    }
     cudaMemsetAsync(counter, 0, sizeof(int), c->stream);
     a.near_units = near_units(ns, t.ts);
     a.n_near = (int)(((long long)ns * nparts + a.near_units - 1) / a.near_units);
