@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "iface_host.h"
 #include "prism_common.cuh"
 #include "ztm_internal.cuh"
 
@@ -554,7 +555,9 @@ __global__ void __launch_bounds__(64)
 // block has too many rows for that to pay, and each pair forms them).  Bound by
 // the FMA pipe, as the forward: 128x128 columns, 64x64 stations 155 -> 124 us;
 // with 256x256 columns and 128x128 stations both directions 3.47 -> 2.82 ms.
-template <bool ROWS>
+// RHO: the density gradient too (without it, as in an inversion for the depths, a
+// pair is its face term alone: 124 -> 70 us at 128x128 columns, 64x64 stations).
+template <bool ROWS, bool RHO>
 __global__ void __launch_bounds__(IF_TS, 5)
     iface_far_adj(IConst k, int ns, const IStation* __restrict__ sf, const int2* __restrict__ si,
                   const float4* __restrict__ cf, const uint32_t* __restrict__ mask,
@@ -638,13 +641,14 @@ __global__ void __launch_bounds__(IF_TS, 5)
       const float2 X2 = __fmul2_rn(X, X), rh = __fadd2_rn(X2, Y2);
       const float2 ut = __fadd2_rn(*reinterpret_cast<const float2*>(s_zs + q), cy2);
       const float2 rt2 = __ffma2_rn(ut, ut, rh);
-      float2 itop, u, f;
+      float2 itop, u = make_float2(0.f, 0.f), f;
+      if (!RHO) itop = make_float2(rsqrt_ftz(rt2.x), rsqrt_ftz(rt2.y));
       // second order when every lane's pairs are far enough (warp-uniform)
       if (__all_sync(__activemask(), fminf(rt2.x, rt2.y) >= k.rt2_t2)) {
-        u = col_unit2<true>(X2, Y2, qY, rh, ut, rt2, cz2, k, &itop);
+        if (RHO) u = col_unit2<true>(X2, Y2, qY, rh, ut, rt2, cz2, k, &itop);
         f = face_unit_far2<true>(X2, Y2, cbY, ut, itop, k.face);
       } else {
-        u = col_unit2<false>(X2, Y2, qY, rh, ut, rt2, cz2, k, &itop);
+        if (RHO) u = col_unit2<false>(X2, Y2, qY, rh, ut, rt2, cz2, k, &itop);
         f = face_unit_far2<false>(X2, Y2, cbY, ut, itop, k.face);
       }
       const float2 r = *reinterpret_cast<const float2*>(s_r + q);
@@ -669,7 +673,7 @@ __global__ void __launch_bounds__(IF_TS, 5)
   }
   if (!active) return;
   const size_t o = (size_t)blockIdx.y * k.ncols + c;
-  p_rho[o] = ar.value();
+  if (RHO) p_rho[o] = ar.value();
   p_dep[o] = (double)col.x * ad.value();
 }
 
@@ -684,7 +688,7 @@ __global__ void iface_far_adj_finalize(long long nc, int nchunks, const double* 
   double r = 0.0, d = 0.0;
 #pragma unroll 4
   for (int q = 0; q < nchunks; q++) {
-    r += p_rho[(size_t)q * nc + c];
+    if (p_rho) r += p_rho[(size_t)q * nc + c];
     d += p_dep[(size_t)q * nc + c];
   }
   if (g_rho) g_rho[c] = sc_rho * r;
@@ -969,14 +973,16 @@ static int iface_adjoint_impl(ztm_ctx* c, const IMeshDesc& m, const double* d_de
   const double sc_dep = G5 * (double)k.dxn * k.dyn;
   int alen;
   const int ach = iface_adj_chunks(ns, nc, c->num_sms, &alen);
-  double* p_rho = wc.take<double>((size_t)ach * nc);
+  double* p_rho = d_grho ? wc.take<double>((size_t)ach * nc) : nullptr;
   double* p_dep = wc.take<double>((size_t)ach * nc);
   {
     ZtmProf prof_(c, "iface_far");
     // rows that IF_TS columns can touch
     const bool rows = (IF_TS - 2) / m.nx + 2 <= IF_ROWS;
     const dim3 grid((unsigned)((nc + IF_TS - 1) / IF_TS), ach);
-    (rows ? iface_far_adj<true> : iface_far_adj<false>)<<<grid, IF_TS, 0, c->stream>>>(
+    auto* fn = rows ? (d_grho ? iface_far_adj<true, true> : iface_far_adj<true, false>)
+                    : (d_grho ? iface_far_adj<false, true> : iface_far_adj<false, false>);
+    fn<<<grid, IF_TS, 0, c->stream>>>(
         k, ns, p.sf, p.si, p.cf, p.mask, p.anynear, alen, p_rho, p_dep);
   }
   iface_far_adj_finalize<<<(unsigned)((nc + 255) / 256), 256, 0, c->stream>>>(
@@ -1074,4 +1080,125 @@ extern "C" int ztm_gfm_interface_misfit(ztm_ctx* c, const ztm_imesh* mesh, const
   if (g_depth) cudaMemcpyAsync(g_depth, s_gd, nc * 8, cudaMemcpyDeviceToHost, c->stream);
   if ((rc = ztm_cuda_check(c, cudaStreamSynchronize(c->stream), "interface misfit"))) return rc;
   return ztm_check_device_error(c);
+}
+
+// ---------------------------------------------------------------------------
+// an inversion's evaluations on host arrays
+namespace {
+
+struct HostDevice {  // the arrays in c->inv
+  double *rho, *xyz, *data, *depth, *v, *jv, *g, *mis;
+  HostDevice(char* base, long long nc, int ns) {
+    WsCarver wc(base);
+    rho = wc.take<double>(nc);
+    xyz = wc.take<double>((size_t)ns * 3);
+    data = wc.take<double>(ns);
+    depth = wc.take<double>(nc);
+    v = wc.take<double>(nc);
+    jv = wc.take<double>(ns);
+    g = wc.take<double>(nc + 1);  // the misfit after the gradient: one copy out
+    mis = g + nc;
+  }
+  static size_t bytes(long long nc, int ns) {
+    return 4 * WsCarver::need((nc + 1) * 8) + WsCarver::need((size_t)ns * 24) +
+           2 * WsCarver::need((size_t)ns * 8);
+  }
+};
+
+struct OnDevice {
+  int prev = -1, dev;
+  explicit OnDevice(int d) : dev(d) {
+    cudaGetDevice(&prev);
+    if (prev != d) cudaSetDevice(d);
+  }
+  ~OnDevice() {
+    if (prev >= 0 && prev != dev) cudaSetDevice(prev);
+  }
+};
+
+IfaceHost host_arrays(ztm_ctx* c, long long nc) {
+  double* p = reinterpret_cast<double*>(c->pin);
+  return {p, p + nc, p + 2 * nc};
+}
+
+// The gradient (and the double behind it) and the error word, and the wait.
+int host_result(ztm_ctx* c, const HostDevice& d, const IfaceHost& h, long long nc) {
+  int* err = reinterpret_cast<int*>(h.g + nc + 1);
+  cudaMemcpyAsync(h.g, d.g, (nc + 1) * 8, cudaMemcpyDeviceToHost, c->stream);
+  cudaMemcpyAsync(err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+  if (int rc = ztm_cuda_check(c, cudaStreamSynchronize(c->stream), "interface inversion")) return rc;
+  return *err ? ztm_check_device_error(c) : ZTM_OK;
+}
+
+}  // namespace
+
+int ztm_iface_host_begin(ztm_ctx* c, const ztm_imesh* mesh, const double* rho, int ns,
+                         const double* sxyz, const double* data, IfaceHost* h) {
+  c->err.clear();
+  if (mesh->nx < 1 || mesh->ny < 1 || !(mesh->dx > 0) || !(mesh->dy > 0))
+    return ztm_fail(c, ZTM_ERR_ARG, "bad interface mesh");
+  const long long nc = (long long)mesh->nx * mesh->ny;
+  OnDevice guard(c->device);
+  const size_t need = HostDevice::bytes(nc, ns), pin = ((size_t)nc * 3 + 2) * 8;
+  int rc = ztm_cuda_check(c, cudaStreamSynchronize(c->stream), "sync before an inversion");
+  if (rc) return rc;
+  if (need > c->inv_size) {
+    if (c->inv) cudaFree(c->inv);
+    c->inv = nullptr;
+    c->inv_size = 0;
+    if (cudaMalloc((void**)&c->inv, need) != cudaSuccess) {
+      cudaGetLastError();
+      c->inv = nullptr;
+      return ztm_fail(c, ZTM_ERR_ALLOC, "inversion arrays: device allocation failed");
+    }
+    c->inv_size = need;
+  }
+  if (pin > c->pin_size) {
+    if (c->pin) cudaFreeHost(c->pin);
+    c->pin = nullptr;
+    c->pin_size = 0;
+    if (cudaMallocHost((void**)&c->pin, pin) != cudaSuccess) {
+      cudaGetLastError();
+      c->pin = nullptr;
+      return ztm_fail(c, ZTM_ERR_ALLOC, "inversion arrays: pinned allocation failed");
+    }
+    c->pin_size = pin;
+  }
+  const HostDevice d(c->inv, nc, ns);
+  cudaMemcpyAsync(d.rho, rho, nc * 8, cudaMemcpyHostToDevice, c->stream);
+  cudaMemcpyAsync(d.xyz, sxyz, (size_t)ns * 24, cudaMemcpyHostToDevice, c->stream);
+  cudaMemcpyAsync(d.data, data, (size_t)ns * 8, cudaMemcpyHostToDevice, c->stream);
+  *h = host_arrays(c, nc);
+  return ztm_cuda_check(c, cudaGetLastError(), "copy the inversion's arrays to the device");
+}
+
+int ztm_iface_host_misfit(ztm_ctx* c, const ztm_imesh* mesh, int ns, const ztm_opts* o,
+                          double* misfit) {
+  const long long nc = (long long)mesh->nx * mesh->ny;
+  OnDevice guard(c->device);
+  const HostDevice d(c->inv, nc, ns);
+  const IfaceHost h = host_arrays(c, nc);
+  ztm_opts od = *o;
+  od.flags |= ZTM_FLAG_DEVICE_PTRS;
+  cudaMemcpyAsync(d.depth, h.depth, nc * 8, cudaMemcpyHostToDevice, c->stream);
+  int rc = ztm_gfm_interface_misfit(c, mesh, d.depth, d.rho, ns, d.xyz, d.data, d.mis, nullptr,
+                                    nullptr, d.g, &od);
+  if (rc || (rc = host_result(c, d, h, nc))) return rc;
+  *misfit = h.g[nc];
+  return ZTM_OK;
+}
+
+int ztm_iface_host_product(ztm_ctx* c, const ztm_imesh* mesh, int ns, const ztm_opts* o) {
+  const long long nc = (long long)mesh->nx * mesh->ny;
+  OnDevice guard(c->device);
+  const HostDevice d(c->inv, nc, ns);
+  const IfaceHost h = host_arrays(c, nc);
+  ztm_opts od = *o;
+  od.flags |= ZTM_FLAG_DEVICE_PTRS;
+  cudaMemcpyAsync(d.depth, h.depth, nc * 8, cudaMemcpyHostToDevice, c->stream);
+  cudaMemcpyAsync(d.v, h.v, nc * 8, cudaMemcpyHostToDevice, c->stream);
+  int rc = ztm_gfm_interface_jvp(c, mesh, d.depth, d.rho, d.v, ns, d.xyz, d.jv, &od);
+  if (!rc)
+    rc = ztm_gfm_interface_adjoint(c, mesh, d.depth, d.rho, ns, d.xyz, d.jv, nullptr, d.g, &od);
+  return rc ? rc : host_result(c, d, h, nc);
 }

@@ -1,6 +1,6 @@
 // invert.cpp - nonlinear interface (Moho depth) inversion driven through the
 // C ABI: every iteration runs the forward and the adjoint on the GPU
-// (ztm_gfm_interface_misfit) and the optimiser on the host.
+// and the optimiser on the host.
 //
 // Objective, with m = depth in km (column tops) and r = gz(m) - data:
 //   phi(m) = 0.5 |r|^2 + 0.5 * lambda * sum over neighbouring columns of
@@ -23,104 +23,117 @@
 #include <string>
 #include <vector>
 
-#include "ztm_grav.h"
+#include "iface_host.h"
 
 namespace {
 
 struct Problem {
   ztm_ctx* ctx;
   const ztm_imesh* mesh;
-  const double* rho;
   int ns;
-  const double* sxyz;
-  const double* data;
   double lambda;
   ztm_opts opts;
   int nx, ny;
-  long long evals = 0;
+  IfaceHost io;
 };
+
+// Sums in eight partial sums (a chain of dependent adds over 128 x 128 columns
+// took 20 us, a dozen times an iteration).
+constexpr size_t LANES = 8;
+double total(const double* s) {
+  return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+}
+double dot(const double* a, const double* b, size_t n) {
+  double s[LANES] = {};
+  size_t i = 0;
+  for (; i + LANES <= n; i += LANES)
+    for (size_t j = 0; j < LANES; j++) s[j] += a[i + j] * b[i + j];
+  for (size_t j = 0; i < n; i++, j++) s[j] += a[i] * b[i];
+  return total(s);
+}
+// sum of (a - b)^2
+double dist2(const double* a, const double* b, size_t n) {
+  double s[LANES] = {};
+  size_t i = 0;
+  for (; i + LANES <= n; i += LANES)
+    for (size_t j = 0; j < LANES; j++) {
+      const double d = a[i + j] - b[i + j];
+      s[j] += d * d;
+    }
+  for (size_t j = 0; i < n; i++, j++) s[j] += (a[i] - b[i]) * (a[i] - b[i]);
+  return total(s);
+}
+// d = (d - a y) scale, and the new d . z
+double step_dot(size_t n, double* __restrict d, double a, const double* __restrict y, double scale,
+                const double* __restrict z) {
+  double s[LANES] = {};
+  size_t i = 0;
+  for (; i + LANES <= n; i += LANES)
+    for (size_t j = 0; j < LANES; j++) {
+      const double v = (d[i + j] - a * y[i + j]) * scale;
+      d[i + j] = v;
+      s[j] += v * z[i + j];
+    }
+  for (size_t j = 0; i < n; i++, j++) {
+    d[i] = (d[i] - a * y[i]) * scale;
+    s[j] += d[i] * z[i];
+  }
+  return total(s);
+}
+double dot(const std::vector<double>& a, const std::vector<double>& b) {
+  return dot(a.data(), b.data(), a.size());
+}
+
+// out = 1000 g + lambda L x: a gradient per metre to one per km plus the
+// smoothing term's (graph Laplacian of the column grid, first-order differences),
+// a row at a time.
+void add_smoothing(const Problem& P, const double* x, const double* g, double* out) {
+  const double lam = P.lambda;
+  const int nx = P.nx;
+  for (int iy = 0; iy < P.ny; iy++) {
+    const size_t r = (size_t)nx * iy;
+    const double *m = x + r, *up = m - nx, *down = m + nx;
+    double* o = out + r;
+    for (int i = 0; i < nx; i++) o[i] = 1000.0 * g[r + i];
+    if (iy > 0)
+      for (int i = 0; i < nx; i++) o[i] -= lam * (up[i] - m[i]);
+    for (int i = 1; i < nx; i++) o[i] -= lam * (m[i - 1] - m[i]);
+    for (int i = 0; i + 1 < nx; i++) o[i] += lam * (m[i] - m[i + 1]);
+    if (iy + 1 < P.ny)
+      for (int i = 0; i < nx; i++) o[i] += lam * (m[i] - down[i]);
+  }
+}
 
 // phi and its gradient (per km) at depth m (km).
 int evaluate(Problem& P, const std::vector<double>& m, double* f, std::vector<double>& g,
              double* data_misfit) {
   const size_t nc = m.size();
-  std::vector<double> dm(nc), g_dep(nc);
-  for (size_t c = 0; c < nc; c++) dm[c] = 1000.0 * m[c];
+  for (size_t c = 0; c < nc; c++) P.io.depth[c] = 1000.0 * m[c];
   double mis = 0.0;
-  int rc = ztm_gfm_interface_misfit(P.ctx, P.mesh, dm.data(), P.rho, P.ns, P.sxyz, P.data, &mis,
-                                    nullptr, nullptr, g_dep.data(), &P.opts);
-  if (rc) return rc;
-  P.evals++;
+  if (int rc = ztm_iface_host_misfit(P.ctx, P.mesh, P.ns, &P.opts, &mis)) return rc;
+  add_smoothing(P, m.data(), P.io.g, g.data());  // d/dm (km) = 1000 d/ddepth (m)
   double reg = 0.0;
-  g.assign(nc, 0.0);
-  for (size_t c = 0; c < nc; c++) g[c] = 1000.0 * g_dep[c];  // d/dm (km) = 1000 d/ddepth (m)
-  for (int iy = 0; iy < P.ny; iy++)
-    for (int ix = 0; ix < P.nx; ix++) {
-      const size_t c = ix + (size_t)P.nx * iy;
-      if (ix + 1 < P.nx) {
-        const double d = m[c] - m[c + 1];
-        reg += d * d;
-        g[c] += P.lambda * d;
-        g[c + 1] -= P.lambda * d;
-      }
-      if (iy + 1 < P.ny) {
-        const double d = m[c] - m[c + P.nx];
-        reg += d * d;
-        g[c] += P.lambda * d;
-        g[c + P.nx] -= P.lambda * d;
-      }
-    }
+  for (int iy = 0; iy < P.ny; iy++) {
+    const double* r = m.data() + (size_t)P.nx * iy;
+    reg += dist2(r, r + 1, P.nx - 1);
+    if (iy + 1 < P.ny) reg += dist2(r, r + P.nx, P.nx);
+  }
   *f = mis + 0.5 * P.lambda * reg;
   if (data_misfit) *data_misfit = mis;
   return ZTM_OK;
 }
 
-double dot(const std::vector<double>& a, const std::vector<double>& b) {
-  double s = 0.0;
-  for (size_t i = 0; i < a.size(); i++) s += a[i] * b[i];
-  return s;
-}
-
-// out += lambda * L v: the Hessian of the smoothing term (graph Laplacian of
-// the column grid, first-order differences).
-void add_smoothing_hessian(const Problem& P, const std::vector<double>& v, std::vector<double>& out) {
-  for (int iy = 0; iy < P.ny; iy++)
-    for (int ix = 0; ix < P.nx; ix++) {
-      const size_t c = ix + (size_t)P.nx * iy;
-      if (ix + 1 < P.nx) {
-        const double d = P.lambda * (v[c] - v[c + 1]);
-        out[c] += d;
-        out[c + 1] -= d;
-      }
-      if (iy + 1 < P.ny) {
-        const double d = P.lambda * (v[c] - v[c + P.nx]);
-        out[c] += d;
-        out[c + P.nx] -= d;
-      }
-    }
-}
-
 // Gauss-Newton Hessian product at depth m (km): (J^T J + lambda L) v, with J
-// the depth derivative of the forward per km (ztm_gfm_interface_jvp for J v,
-// the depth adjoint for J^T w; one of each per product).
+// the depth derivative of the forward per km (one J v and one J^T w).
 int gn_product(Problem& P, const std::vector<double>& m, const std::vector<double>& v,
                std::vector<double>& out) {
   const size_t nc = m.size();
-  std::vector<double> dm(nc), dv(nc), g_dep(nc), jv(P.ns);
   for (size_t c = 0; c < nc; c++) {
-    dm[c] = 1000.0 * m[c];
-    dv[c] = 1000.0 * v[c];  // km -> m
+    P.io.depth[c] = 1000.0 * m[c];
+    P.io.v[c] = 1000.0 * v[c];  // km -> m
   }
-  int rc = ztm_gfm_interface_jvp(P.ctx, P.mesh, dm.data(), P.rho, dv.data(), P.ns, P.sxyz,
-                                 jv.data(), &P.opts);
-  if (rc) return rc;
-  rc = ztm_gfm_interface_adjoint(P.ctx, P.mesh, dm.data(), P.rho, P.ns, P.sxyz, jv.data(), nullptr,
-                                 g_dep.data(), &P.opts);
-  if (rc) return rc;
-  P.evals++;
-  out.assign(nc, 0.0);
-  for (size_t c = 0; c < nc; c++) out[c] = 1000.0 * g_dep[c];
-  add_smoothing_hessian(P, v, out);
+  if (int rc = ztm_iface_host_product(P.ctx, P.mesh, P.ns, &P.opts)) return rc;
+  add_smoothing(P, v.data(), P.io.g, out.data());
   return ZTM_OK;
 }
 
@@ -137,53 +150,56 @@ extern "C" int ztm_invert_interface(ztm_ctx* ctx, const ztm_imesh* mesh, double*
   Problem P;
   P.ctx = ctx;
   P.mesh = mesh;
-  P.rho = rho_col;
   P.ns = ns;
-  P.sxyz = sxyz;
-  P.data = data;
   P.lambda = lambda;
   memset(&P.opts, 0, sizeof P.opts);
   if (opt) P.opts = *opt;
   P.nx = mesh->nx;
   P.ny = mesh->ny;
+  int rc = ztm_iface_host_begin(ctx, mesh, rho_col, ns, sxyz, data, &P.io);
+  if (rc) return rc;
   const size_t nc = (size_t)mesh->nx * mesh->ny;
   const double dmax = -mesh->z_base / 1000.0;  // tops stay above the bases
   std::vector<double> m(nc), g(nc), mt(nc), gt(nc), d(nc);
   for (size_t c = 0; c < nc; c++) m[c] = std::min(std::max(depth[c] / 1000.0, 0.0), dmax);
   double f = 0.0, mis = 0.0;
-  int rc = evaluate(P, m, &f, g, &mis);
+  rc = evaluate(P, m, &f, g, &mis);
   if (rc) return rc;
   const int H = 8;
-  std::vector<std::vector<double>> S, Y;
-  std::vector<double> rhoh;
+  // steps and gradient changes: S[p], Y[p] for p = kept.front() .. kept.back()
+  std::vector<std::vector<double>> S(H), Y(H);
+  std::vector<int> kept;
+  double rhoh[H], alpha[H], yy[H];
+  std::vector<double> spare_s, spare_y;
   int it = 0;
   for (; it < iterations; it++) {
     if (history) history[it] = mis;
-    // two-loop recursion: d = -H g
-    d = g;
-    std::vector<double> alpha(S.size());
-    for (int k = (int)S.size() - 1; k >= 0; k--) {
-      alpha[k] = rhoh[k] * dot(S[k], d);
-      for (size_t i = 0; i < nc; i++) d[i] -= alpha[k] * Y[k][i];
-    }
-    double gamma;
-    if (!S.empty()) {
-      gamma = dot(S.back(), Y.back()) / dot(Y.back(), Y.back());
+    // two-loop recursion: d = -H g; a pass over d both updates it and forms the
+    // next dot product
+    const int n = (int)kept.size();
+    if (n) {
+      d = g;
+      const double gamma = 1.0 / (rhoh[kept[n - 1]] * yy[kept[n - 1]]);
+      double sd = dot(S[kept[n - 1]], d);
+      for (int k = n - 1; k >= 0; k--) {
+        const int q = kept[k];
+        alpha[q] = rhoh[q] * sd;
+        sd = step_dot(nc, d.data(), alpha[q], Y[q].data(), k ? 1.0 : gamma,
+                      k ? S[kept[k - 1]].data() : Y[q].data());
+      }
+      for (int k = 0; k < n; k++) {
+        const int q = kept[k], z = kept[std::min(k + 1, n - 1)];
+        sd = step_dot(nc, d.data(), rhoh[q] * sd - alpha[q], S[q].data(), k + 1 < n ? 1.0 : -1.0,
+                      Y[z].data());
+      }
     } else {
-      double gn = sqrt(dot(g, g));
-      gamma = gn > 0 ? 1.0 / gn : 1.0;  // first step: 1 km along -g/|g|
+      const double gn = sqrt(dot(g, g));
+      const double gamma = gn > 0 ? 1.0 / gn : 1.0;  // first step: 1 km along -g/|g|
+      for (size_t i = 0; i < nc; i++) d[i] = -(g[i] * gamma);
     }
-    for (size_t i = 0; i < nc; i++) d[i] *= gamma;
-    for (int k = 0; k < (int)S.size(); k++) {
-      const double beta = rhoh[k] * dot(Y[k], d);
-      for (size_t i = 0; i < nc; i++) d[i] += S[k][i] * (alpha[k] - beta);
-    }
-    for (size_t i = 0; i < nc; i++) d[i] = -d[i];
     double slope = dot(g, d);
     if (!(slope < 0)) {  // not a descent direction: restart on steepest descent
-      S.clear();
-      Y.clear();
-      rhoh.clear();
+      kept.clear();
       double gn = sqrt(dot(g, g));
       if (gn == 0) break;
       for (size_t i = 0; i < nc; i++) d[i] = -g[i] / gn;
@@ -203,21 +219,24 @@ extern "C" int ztm_invert_interface(ztm_ctx* ctx, const ztm_imesh* mesh, double*
       step *= 0.5;
     }
     if (!accepted) break;
-    std::vector<double> s(nc), y(nc);
-    for (size_t i = 0; i < nc; i++) {
-      s[i] = mt[i] - m[i];
-      y[i] = gt[i] - g[i];
-    }
-    const double sy = dot(s, y);
-    if (sy > 1e-12 * sqrt(dot(s, s) * dot(y, y))) {
-      S.push_back(s);
-      Y.push_back(y);
-      rhoh.push_back(1.0 / sy);
-      if ((int)S.size() > H) {
-        S.erase(S.begin());
-        Y.erase(Y.begin());
-        rhoh.erase(rhoh.begin());
-      }
+    // the pair in a place that is free: the oldest's once there are H
+    int p = kept.size() < (size_t)H ? 0 : kept[0];
+    if (kept.size() < (size_t)H)
+      while (std::find(kept.begin(), kept.end(), p) != kept.end()) p++;
+    spare_s.resize(nc);
+    spare_y.resize(nc);
+    double *s = spare_s.data(), *y = spare_y.data();
+    for (size_t i = 0; i < nc; i++) s[i] = mt[i] - m[i];
+    for (size_t i = 0; i < nc; i++) y[i] = gt[i] - g[i];
+    const double sy = dot(s, y, nc);
+    const double ss = dot(s, s, nc), y2 = dot(y, y, nc);
+    if (sy > 1e-12 * sqrt(ss * y2)) {
+      S[p].swap(spare_s);
+      Y[p].swap(spare_y);
+      rhoh[p] = 1.0 / sy;
+      yy[p] = y2;
+      if (kept.size() == (size_t)H) kept.erase(kept.begin());
+      kept.push_back(p);
     }
     m.swap(mt);
     g.swap(gt);
@@ -247,21 +266,20 @@ extern "C" int ztm_invert_interface_gn(ztm_ctx* ctx, const ztm_imesh* mesh, doub
   Problem P;
   P.ctx = ctx;
   P.mesh = mesh;
-  P.rho = rho_col;
   P.ns = ns;
-  P.sxyz = sxyz;
-  P.data = data;
   P.lambda = lambda;
   memset(&P.opts, 0, sizeof P.opts);
   if (opt) P.opts = *opt;
   P.nx = mesh->nx;
   P.ny = mesh->ny;
+  int rc = ztm_iface_host_begin(ctx, mesh, rho_col, ns, sxyz, data, &P.io);
+  if (rc) return rc;
   const size_t nc = (size_t)mesh->nx * mesh->ny;
   const double dmax = -mesh->z_base / 1000.0;
   std::vector<double> m(nc), g(nc), mt(nc), gt(nc), x(nc), r(nc), p(nc), Ap(nc);
   for (size_t c = 0; c < nc; c++) m[c] = std::min(std::max(depth[c] / 1000.0, 0.0), dmax);
   double f = 0.0, mis = 0.0;
-  int rc = evaluate(P, m, &f, g, &mis);
+  rc = evaluate(P, m, &f, g, &mis);
   if (rc) return rc;
   int it = 0;
   for (; it < iterations; it++) {

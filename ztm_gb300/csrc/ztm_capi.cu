@@ -277,6 +277,8 @@ void ztm_ctx_destroy(ztm_ctx* c) {
   }
   for (auto e : c->prof_pool) cudaEventDestroy(e);
   if (c->ws) cudaFree(c->ws);
+  if (c->inv) cudaFree(c->inv);
+  if (c->pin) cudaFreeHost(c->pin);
   if (c->d_err) cudaFree(c->d_err);
   if (c->d_forms) cudaFree(c->d_forms);
   if (c->aux) {

@@ -42,6 +42,11 @@ struct ztm_ctx {
   // grow-only device workspace; carved per call
   char* ws = nullptr;
   size_t ws_size = 0;
+  // an inversion's arrays on the device and their pinned host side (iface.cu)
+  char* inv = nullptr;
+  size_t inv_size = 0;
+  char* pin = nullptr;
+  size_t pin_size = 0;
   // device error word written by bounded waits / bounds checks
   int* d_err = nullptr;
   // batched-launch graph cache and the host copy of the last job table
