@@ -60,3 +60,24 @@ def test_a_station_on_a_node_is_not_finite(ctx):
     surf[10] = 2.0
     out = ctx.pointmass(g, drho, surf)
     assert not np.isfinite(out[10]) and np.all(np.isfinite(np.delete(out, 10)))
+
+
+@pytest.mark.parametrize("lift", [1e-3, 0.5, 7.3, 33.0, 1e3, 1.04e6, 1.06e6, 3e6])
+def test_every_pair(ctx, lift):
+    """Single pairs, element by element, over a wide grid: r^2 in fixed point,
+    near pairs whose r^2 is added in double instead, and heights around the
+    fixed point's limit (2^20 spacings).  TOLERANCE: 5e-15, r^-3 to 1e-15 and
+    three products here, as much again in the oracle."""
+    g = ztm_gb300.make_grid(121, 47, 2, 1, 2, 0)
+    n = 121 * 47 * 3
+    surf = np.full(121 * 47, 1.0 + lift)
+    w = np.zeros(121 * 47)
+    for node, station in ((0, 5686), (121 * 47 + 121 * 20 + 60, 121 * 23 + 57), (n - 1, 0)):
+        drho = np.zeros(n)
+        drho[node] = 0.7
+        ref = oracle.pointmass_tfm(g, drho, surf)
+        assert np.all(np.abs(ctx.pointmass(g, drho, surf) - ref) <= 5e-15 * np.abs(ref))
+        w[:] = 0.0
+        w[station] = 1.3
+        ref = oracle.pointmass_adjoint(g, surf, w)
+        assert np.all(np.abs(ctx.pointmass_adjoint(g, surf, w) - ref) <= 5e-15 * np.abs(ref))

@@ -254,8 +254,7 @@ __global__ void __launch_bounds__(PMA_TB)
 // Double, by levels (pm64.cuh): a block takes 128 selected nodes of one level
 // (the launch has blocks for full levels; those past a level's nodes end) and
 // a slice of the stations, 128 at a time in shared memory with this level's
-// z^2 and w dz.  A pair is two integer products, two FP64 instructions and
-// pm_cube_rsqrt.
+// z^2 (in fixed point too) and w dz.
 constexpr int P64_T = 128;
 __global__ void __launch_bounds__(P64_T, 8)
     pma64_gather_kernel(PmParams p, const Pm64Node* __restrict__ node, const int* __restrict__ row,
@@ -263,6 +262,7 @@ __global__ void __launch_bounds__(P64_T, 8)
                         int slice, long long pstride, double* __restrict__ partial) {
   __shared__ double2 s_z[P64_T];  // z^2, w dz
   __shared__ int2 s_ij[P64_T];    // the station's fine-grid i, j
+  __shared__ PmFixed s_f[P64_T];
   const int k = (int)(blockIdx.x / pblocks) % p.kk, sl = (int)(blockIdx.x / pblocks) / p.kk;
   const int e0 = row[(long long)k * p.jj] + (int)(blockIdx.x % pblocks) * P64_T;
   const int e1 = row[(long long)(k + 1) * p.jj];
@@ -284,18 +284,27 @@ __global__ void __launch_bounds__(P64_T, 8)
         z = make_double2(dz * dz, w[m] * dz);
         ij = make_int2(ci * p.fh, cj * p.fh);
       }
+      const int mx = max(ij.x, p.ii - 1 - ij.x), my = max(ij.y, p.jj - 1 - ij.y);
+      s_f[threadIdx.x].set(z.x, (uint32_t)(mx * mx) + (uint32_t)(my * my), true);
       s_z[threadIdx.x] = z;
       s_ij[threadIdx.x] = ij;
     }
     __syncthreads();
     const int cnt = min(P64_T, s1 - t0);
-#pragma unroll 2
+    double tile_sum = 0.0;  // short chains keep the sums' rounding below the pairs'
+#pragma unroll 4
     for (int q = 0; q < cnt; q++) {
       const double2 z = s_z[q];
       const int2 ij = s_ij[q];
       const int dx = ij.x - xi, dy = ij.y - yj;
-      acc = fma(z.y, pm_cube_rsqrt(z.x + pm_int_double((uint32_t)(dx * dx + dy * dy))), acc);
+      const uint32_t n = (uint32_t)(dx * dx + dy * dy);
+      const PmFixed f = s_f[q];
+      const uint64_t F = f.r2(n);
+      const double r3 = (uint32_t)(F >> 32) >= PM_FIXED_MIN ? pm_cube_rsqrt_fixed(F, f.sh)
+                                                     : pm_cube_rsqrt(z.x + pm_int_double(n));
+      tile_sum = fma(z.y, r3, tile_sum);
     }
+    acc += tile_sum;
   }
   if (e < e1) partial[sl * pstride + e] = acc;
 }

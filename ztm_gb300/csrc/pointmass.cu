@@ -560,6 +560,11 @@ __global__ void __launch_bounds__(PM_TS, 8)
   const int xi = ci * p.fh, yj = cj * p.fh;  // in fine-grid steps
   const double dz = p.fh * (surf[ci + cj * p.di] - k * (1.0 / p.fv));
   const double z2 = dz * dz;
+  PmFixed fix;
+  {
+    const int mx = max(xi, p.ii - 1 - xi), my = max(abs(yj - j0), abs(yj - (j1 - 1)));
+    fix.set(z2, (uint32_t)(mx * mx) + (uint32_t)my * (uint32_t)my, my <= PM64_MAX_OFF);
+  }
   __syncthreads();
   const int e0 = s_row[0], e1 = s_row[j1 - j0];
   double acc = 0.0;
@@ -573,35 +578,43 @@ __global__ void __launch_bounds__(PM_TS, 8)
       while (s_row[j + 1 - j0] <= t0 + q) j++;
       const int qe = min(cnt, s_row[j + 1 - j0] - t0), dy = yj - j;
       const double zy = z2 + (double)dy * dy;
-#pragma unroll 2
+      const uint32_t n0 = (uint32_t)dy * (uint32_t)dy;
+      double row_sum = 0.0;  // short chains keep the sums' rounding below the pairs'
+#pragma unroll 4
       for (; q < qe; q++) {
         const Pm64Node v = tile[q];
-        acc = fma(v.w, pm_cube_rsqrt(zy + sq[abs(xi - v.i)]), acc);
+        const int dx = xi - v.i;
+        const uint64_t F = fix.r2((uint32_t)(dx * dx) + n0);
+        const double r3 = (uint32_t)(F >> 32) >= PM_FIXED_MIN ? pm_cube_rsqrt_fixed(F, fix.sh)
+                                                         : pm_cube_rsqrt(zy + sq[abs(dx)]);
+        row_sum = fma(v.w, r3, row_sum);
       }
+      acc += row_sum;
     }
   }
   if (s < p.ns) partial[(long long)(chunk * p.kk + k) * p.ns + s] = acc * dz;
 }
 
 // G[m] = factor * sum of the n partial sums for interior m, 0 elsewhere: 32
-// grid nodes a block, eight threads each, in a fixed order.
-__global__ void __launch_bounds__(256)
+// grid nodes a block, sixteen threads each, in a fixed order.
+__global__ void __launch_bounds__(512)
     pm64_finalize_kernel(PmParams p, int n, const double* __restrict__ partial, double factor,
                          double* __restrict__ G) {
-  __shared__ double sm[8][33];
+  __shared__ double sm[16][33];
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5, m = blockIdx.x * 32 + x;
   const int i0 = m % p.di, j0 = m / p.di;
   const bool in = m < p.di * p.dj && i0 >= p.bfr && i0 < p.di - p.bfr && j0 >= p.bfr && j0 < p.dj - p.bfr;
   double g = 0.0;
   if (in) {
     const int s = (i0 - p.bfr) + (j0 - p.bfr) * p.ni;
-    for (int c = y; c < n; c += 8) g += partial[(long long)c * p.ns + s];
+#pragma unroll 8
+    for (int c = y; c < n; c += 16) g += partial[(long long)c * p.ns + s];
   }
   sm[y][x] = g;
   __syncthreads();
   if (y || m >= p.di * p.dj) return;
 #pragma unroll
-  for (int q = 1; q < 8; q++) g += sm[q][x];
+  for (int q = 1; q < 16; q++) g += sm[q][x];
   G[m] = in ? g * factor : 0.0;
 }
 
@@ -787,7 +800,7 @@ int ztm_launch_pointmass(ztm_ctx* c, const PmParams& p, const double* d_drho,
           p, list.node, list.row, d_surf, tiles, chunk_rows, partial);
     }
     // fine-grid lengths: dz / r^3 is fh^2 times smaller there
-    pm64_finalize_kernel<<<(unsigned)((p.di * (long long)p.dj + 31) / 32), 256, 0, c->stream>>>(
+    pm64_finalize_kernel<<<(unsigned)((p.di * (long long)p.dj + 31) / 32), 512, 0, c->stream>>>(
         p, p.kk * chunks, partial, factor * ((double)p.fh * p.fh), d_G);
     c->launches += 2;
     return ztm_after_launch(c, "point-mass kernels");
