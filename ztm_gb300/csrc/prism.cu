@@ -80,7 +80,7 @@ __global__ void transpose_kernel(MeshConst k, int nmodels, const double* __restr
 // near box).  The predicate is that of double arithmetic: float decides where
 // its squared distance, from offsets to the home cell's centre, is off the limit
 // by more than its error (below 6e-6 R^2 + 3e-6 R dx), double where it is not
-// (all in double: 16 us for 1,024 stations, bound by the FP64 pipe).
+// (all in double: 16 us for 1,024 stations, bound by the FP64 pipe; now 9).
 constexpr int NEAR_IV_TS = 128;
 __global__ void __launch_bounds__(NEAR_IV_TS)
     near_iv_kernel(MeshConst k, MeshDesc m, int ns, const int4* __restrict__ si,
