@@ -390,8 +390,8 @@ __global__ void pm_cols_count(PmParams p, const double* __restrict__ drho,
   const int ni = (int)(c % p.ii), nj = (int)(c / p.ii);
   colxy[c] = make_float2(-(float)(ni * (1.0 / p.fh)), -(float)(nj * (1.0 / p.fh)));
   int cnt = 0;
-  for (int k = 0; k < p.kk; k++)
-    if (pm_col_weight(p, drho, mult, c + k * ncols) != 0.f) cnt++;
+#pragma unroll 8
+  for (int k = 0; k < p.kk; k++) cnt += pm_col_weight(p, drho, mult, c + k * ncols) != 0.f;
   counts[c] = (cnt + 1) >> 1;
 }
 
@@ -404,17 +404,24 @@ __global__ void pm_cols_write(PmParams p, const double* __restrict__ drho,
   float4* out = pairs + offs[c];
   int q = 0;
   float ka = 0.f, wa = 0.f;
-  for (int k = 0; k < p.kk; k++) {
-    const float w = pm_col_weight(p, drho, mult, c + k * ncols);
-    if (w == 0.f) continue;
-    const float kz = -(float)(k * (1.0 / p.fv));  // -k in grid units (TFM.cpp:97)
-    if (q & 1)
-      out[q >> 1] = make_float4(ka, kz, wa, w);
-    else {
-      ka = kz;
-      wa = w;
+  for (int k0 = 0; k0 < p.kk; k0 += 8) {
+    float ws[8];  // loaded together: the loop below cannot run ahead
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      ws[k] = k0 + k < p.kk ? pm_col_weight(p, drho, mult, c + (k0 + k) * ncols) : 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const float w = ws[k];
+      if (w == 0.f) continue;
+      const float kz = -(float)((k0 + k) * (1.0 / p.fv));  // -k in grid units (TFM.cpp:97)
+      if (q & 1)
+        out[q >> 1] = make_float4(ka, kz, wa, w);
+      else {
+        ka = kz;
+        wa = w;
+      }
+      q++;
     }
-    q++;
   }
   if (q & 1) out[q >> 1] = make_float4(ka, -1.0e18f, wa, 0.f);
 }
@@ -488,6 +495,30 @@ __device__ __forceinline__ double pm_col_weight64(const PmParams& p,
     return m ? w * m : 0.0;
   }
   return fabs(w) > p.thr ? w : 0.0;
+}
+
+// G[m] = factor * sum of the n partial sums for interior m, 0 elsewhere: 32
+// grid nodes a block, sixteen threads each, in a fixed order (a thread
+// each took 31 us for 219 sums of 128x128 nodes, this 13).
+__global__ void __launch_bounds__(512)
+    pm_finalize_kernel(PmParams p, int n, const double* __restrict__ partial, double factor,
+                         double* __restrict__ G) {
+  __shared__ double sm[16][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, m = blockIdx.x * 32 + x;
+  const int i0 = m % p.di, j0 = m / p.di;
+  const bool in = m < p.di * p.dj && i0 >= p.bfr && i0 < p.di - p.bfr && j0 >= p.bfr && j0 < p.dj - p.bfr;
+  double g = 0.0;
+  if (in) {
+    const int s = (i0 - p.bfr) + (j0 - p.bfr) * p.ni;
+#pragma unroll 8
+    for (int c = y; c < n; c += 16) g += partial[(long long)c * p.ns + s];
+  }
+  sm[y][x] = g;
+  __syncthreads();
+  if (y || m >= p.di * p.dj) return;
+#pragma unroll
+  for (int q = 1; q < 16; q++) g += sm[q][x];
+  G[m] = in ? g * factor : 0.0;
 }
 
 // Double path (the context entry points): level by level over the selected
@@ -593,45 +624,6 @@ __global__ void __launch_bounds__(PM_TS, 8)
     }
   }
   if (s < p.ns) partial[(long long)(chunk * p.kk + k) * p.ns + s] = acc * dz;
-}
-
-// G[m] = factor * sum of the n partial sums for interior m, 0 elsewhere: 32
-// grid nodes a block, sixteen threads each, in a fixed order.
-__global__ void __launch_bounds__(512)
-    pm64_finalize_kernel(PmParams p, int n, const double* __restrict__ partial, double factor,
-                         double* __restrict__ G) {
-  __shared__ double sm[16][33];
-  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, m = blockIdx.x * 32 + x;
-  const int i0 = m % p.di, j0 = m / p.di;
-  const bool in = m < p.di * p.dj && i0 >= p.bfr && i0 < p.di - p.bfr && j0 >= p.bfr && j0 < p.dj - p.bfr;
-  double g = 0.0;
-  if (in) {
-    const int s = (i0 - p.bfr) + (j0 - p.bfr) * p.ni;
-#pragma unroll 8
-    for (int c = y; c < n; c += 16) g += partial[(long long)c * p.ns + s];
-  }
-  sm[y][x] = g;
-  __syncthreads();
-  if (y || m >= p.di * p.dj) return;
-#pragma unroll
-  for (int q = 1; q < 16; q++) g += sm[q][x];
-  G[m] = in ? g * factor : 0.0;
-}
-
-// G[m] = factor * sum_chunks partial for interior m, 0 elsewhere.
-__global__ void pm_finalize_kernel(PmParams p, int nchunks,
-                                   const double* __restrict__ partial,
-                                   double factor, double* __restrict__ G) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= p.di * p.dj) return;
-  int i0 = m % p.di, j0 = m / p.di;
-  double g = 0.0;
-  if (i0 >= p.bfr && i0 < p.di - p.bfr && j0 >= p.bfr && j0 < p.dj - p.bfr) {
-    int s = (i0 - p.bfr) + (j0 - p.bfr) * p.ni;
-    for (int c = 0; c < nchunks; c++) g += partial[(long long)c * p.ns + s];
-    g *= factor;
-  }
-  G[m] = g;
 }
 
 // Resident blocks per SM of the gather kernel that a call runs (the float
@@ -800,7 +792,7 @@ int ztm_launch_pointmass(ztm_ctx* c, const PmParams& p, const double* d_drho,
           p, list.node, list.row, d_surf, tiles, chunk_rows, partial);
     }
     // fine-grid lengths: dz / r^3 is fh^2 times smaller there
-    pm64_finalize_kernel<<<(unsigned)((p.di * (long long)p.dj + 31) / 32), 512, 0, c->stream>>>(
+    pm_finalize_kernel<<<(unsigned)((p.di * (long long)p.dj + 31) / 32), 512, 0, c->stream>>>(
         p, p.kk * chunks, partial, factor * ((double)p.fh * p.fh), d_G);
     c->launches += 2;
     return ztm_after_launch(c, "point-mass kernels");
@@ -826,10 +818,12 @@ int ztm_launch_pointmass(ztm_ctx* c, const PmParams& p, const double* d_drho,
       float2* colxy = wc.take<float2>((size_t)ncols);
       float4* pairs = wc.take<float4>((size_t)((p.N + ncols) / 2 + 2));
       int* mult = mark();
-      const unsigned cb = (unsigned)((ncols + 255) / 256);
-      pm_cols_count<<<cb, 256, 0, c->stream>>>(p, d_drho, mult, offs, colxy);
+      // small blocks: a column's weights take FP64 conversions, so every SM's
+      // pipe counts (128x128 columns, 65 levels: 26 us in 64 blocks)
+      const unsigned cb = (unsigned)((ncols + 63) / 64);
+      pm_cols_count<<<cb, 64, 0, c->stream>>>(p, d_drho, mult, offs, colxy);
       pm_nodes_scan<<<1, 1024, 0, c->stream>>>((int)ncols, offs, offs + ncols);
-      pm_cols_write<<<cb, 256, 0, c->stream>>>(p, d_drho, mult, offs, pairs);
+      pm_cols_write<<<cb, 64, 0, c->stream>>>(p, d_drho, mult, offs, pairs);
       {
         ZtmProf prof_(c, "pointmass");
         pm_gather_cols_kernel<<<grid, PM_TS, 0, c->stream>>>(p, pairs, offs, colxy, d_surf,
@@ -856,7 +850,7 @@ int ztm_launch_pointmass(ztm_ctx* c, const PmParams& p, const double* d_drho,
     chunks = 0;
   }
   int M = p.di * p.dj;
-  pm_finalize_kernel<<<(M + 255) / 256, 256, 0, c->stream>>>(p, chunks, partial, factor, d_G);
+  pm_finalize_kernel<<<(M + 31) / 32, 512, 0, c->stream>>>(p, chunks, partial, factor, d_G);
   c->launches++;
   return ztm_after_launch(c, "point-mass kernels");
 }
@@ -1020,7 +1014,7 @@ extern "C" int ztm_gfm_pointmass_noalloc(const ztm_grid* g, const double* drho,
   }
   const double factor = g->scale * 66.7 / ((double)p.fh * p.fh * p.fv);
   const int M = p.di * p.dj;
-  pm_finalize_kernel<<<(M + 255) / 256, 256, 0, s>>>(p, chunks, partial, factor, G);
+  pm_finalize_kernel<<<(M + 31) / 32, 512, 0, s>>>(p, chunks, partial, factor, G);
   // a launch error here is this call's own (none was pending at entry)
   if (cudaGetLastError() != cudaSuccess) return ZTM_ERR_CUDA;
   return ZTM_OK;
