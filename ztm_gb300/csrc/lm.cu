@@ -26,8 +26,10 @@
 //                              JJ + d0 M + d1 A with J^T r as a further row
 //   lm_potrf, lm_trsm,         Cholesky by panels of 64 columns, all pairs at
 //   oz_kernel<1>               once: diagonal block and panel in double, the
-//                              trailing update on the tensor cores.  The further
-//                              row comes out as the forward substitution.
+//                              trailing update on the tensor cores, for the next
+//                              panel's columns first, for the others beside that
+//                              panel.  The further row comes out as the forward
+//                              substitution.
 //   lm_backstep                L^T x = y, 64 unknowns a launch
 //   lm_finish                  B = b + x
 //   lm_lu_all                  the systems that are not positive definite (a
@@ -146,7 +148,9 @@ struct OzArgs {
   size_t s_stride;
   int ld, r0;                // the trailing block starts at row and column r0
   const int* bad;            // per pair: not positive definite
+  int part;                  // the columns of the next panel, or the others
 };
+enum { OZ_NEXT = 1, OZ_REST = 2 };
 
 // Tile w of the launch: matrix (row slice or pair), row block, column tile.
 struct OzTile {
@@ -160,8 +164,12 @@ __device__ __forceinline__ OzTile oz_tile(const OzArgs& a, int w) {
   if (MODE == 0) {  // upper: column tiles from the diagonal on
     while (jt >= a.tiles_j - 2 * ib) jt -= a.tiles_j - 2 * ib++;
     jt += 2 * ib;
-  } else {  // lower: column tiles up to the diagonal
-    while (jt >= 2 * ib + 2) jt -= 2 * ib++ + 2;
+  } else if (a.part == OZ_NEXT) {  // lower: the first column tile
+    ib = jt;
+    jt = 0;
+  } else {  // column tiles from the second up to the diagonal
+    while (jt >= 2 * ib + 1) jt -= 2 * ib++ + 1;
+    jt++;
   }
   t.ib = ib;
   t.jt = jt;
@@ -215,7 +223,11 @@ __global__ void __launch_bounds__(OZ_T, 1) oz_kernel(const __grid_constant__ OzA
   tc_fence_after();
   const uint32_t tmem = sh.tmem;
   volatile int* fail = &sh.fail;
-  auto skip = [&](const OzTile& t) { return MODE == 1 && a.bad[t.z] != 0; };
+  // (beside the next panel's kernels, which may mark a pair meanwhile, nothing is
+  // skipped: a marked pair's matrix is formed anew for the LU)
+  auto skip = [&](const OzTile& t) {
+    return MODE == 1 && a.part == OZ_NEXT && a.bad[t.z] != 0;
+  };
   if (warp < 8) {
     int ph = 0;
     for (int w = blockIdx.x; w < a.work; w += gridDim.x) {
@@ -1208,13 +1220,13 @@ extern "C" int ztm_lm_steps(ztm_ctx* c, const double* J, int nrows, int ncols, c
   const int nstat = (nrows + LM_STAT_ROWS - 1) / LM_STAT_ROWS;
   const size_t prb = (n + OZ_M) / OZ_M;  // row blocks below the first panel (the right-hand row included)
   const size_t dig_stride = prb * 2 * OZ_CHUNK;
-  const size_t dig = std::max((size_t)s.rb * s.kcs * OZ_CHUNK, (size_t)nd * dig_stride);
+  const size_t dig = std::max((size_t)s.rb * s.kcs * OZ_CHUNK, 2 * (size_t)nd * dig_stride);
   const size_t need = WsCarver::need(m * n * 8) + 3 * WsCarver::need(m * 8 + n * 8) +
                       WsCarver::need(n * n * 8) + WsCarver::need((size_t)nd * 16) +
                       2 * WsCarver::need((size_t)nd * n * 8) + WsCarver::need((size_t)nstat * n * 12) +
                       3 * WsCarver::need(n * 8) + WsCarver::need((size_t)s.slices * n * n * 8) +
                       WsCarver::need((size_t)nd * (n + 1) * ld * 8) + WsCarver::need(dig) +
-                      WsCarver::need((size_t)nd * prb * OZ_M * 4) + 3 * WsCarver::need((size_t)nd * 8) +
+                      WsCarver::need(2 * (size_t)nd * prb * OZ_M * 4) + 3 * WsCarver::need((size_t)nd * 8) +
                       WsCarver::need((size_t)nd * n * 4) + WsCarver::need((size_t)nd * LM_NB * LM_NB * 8) +
                       16384;
   int rc = ztm_ws_reserve(c, need);
@@ -1238,7 +1250,7 @@ extern "C" int ztm_lm_steps(ztm_ctx* c, const double* J, int nrows, int ncols, c
   double* part = wc.take<double>((size_t)s.slices * n * n);
   double* S = wc.take<double>((size_t)nd * (n + 1) * ld);
   unsigned char* digits = wc.take<unsigned char>(dig);
-  int* pex = wc.take<int>((size_t)nd * prb * OZ_M);
+  int* pex = wc.take<int>(2 * (size_t)nd * prb * OZ_M);
   int* piv = wc.take<int>((size_t)nd * n);
   int* state = wc.take<int>(2 * (size_t)nd + 1);  // bad, singular, the barrier
   if (wc.off > need) return ztm_fail(c, ZTM_ERR_ALLOC, "normal equations: workspace");
@@ -1286,10 +1298,8 @@ extern "C" int ztm_lm_steps(ztm_ctx* c, const double* J, int nrows, int ncols, c
         ncols, ld, oJJ, g, (const double*)ps, (const double*)pd, S);
     launches += 3;
     OzArgs u = {};
-    u.dig = digits;
     u.nkc = 2;
     u.per = 2;
-    u.exps = pex;
     u.err = c->d_err;
     u.dig_stride = dig_stride;
     u.exp_stride = (int)(prb * OZ_M);
@@ -1297,22 +1307,41 @@ extern "C" int ztm_lm_steps(ztm_ctx* c, const double* J, int nrows, int ncols, c
     u.s_stride = (n + 1) * (size_t)ld;
     u.ld = ld;
     u.bad = bad;
-    for (int k0 = 0; k0 < ncols; k0 += LM_NB) {
+    // A panel is two latency chains on few SMs (diagonal block 73 us, rows 35), so
+    // the update of the columns beyond the next panel runs beside the next
+    // panel's kernels on the side stream, leaving them some SMs; it reads the
+    // panel's digits while the next panel writes the other set.  (One update after
+    // the panel: 10.3 ms a call for 12000 x 2700; beside it, with two SMs left free
+    // 9.0, with 8 9.1, with 24 9.3, with 48 9.6.)
+    const int rest_grid = std::max(1, c->num_sms - std::max(nd, 2));
+    for (int k0 = 0, set = 0; k0 < ncols; k0 += LM_NB, set ^= 1) {
       const int nb = std::min(LM_NB, ncols - k0);
+      unsigned char* dset = digits + set * (size_t)nd * dig_stride;
+      int* eset = pex + set * (size_t)nd * u.exp_stride;
       lm_potrf<<<nd, PF_T, 0, c->stream>>>(ncols, k0, nb, ld, S, dinv, LT, bad);
       const int rows = ncols + 1 - (k0 + nb), rb = (rows + OZ_M - 1) / OZ_M;
       // whole row blocks of digits: the rows past the last are zeros
       lm_trsm<<<dim3(rb * (OZ_M / TR_R), nd), TR_T, 0, c->stream>>>(
-          ncols, k0, nb, ld, S, dinv, LT, digits, dig_stride, pex, u.exp_stride, bad);
+          ncols, k0, nb, ld, S, dinv, LT, dset, dig_stride, eset, u.exp_stride, bad);
       launches += 2;
-      if (rows > 1) {
-        u.n = rows;
-        u.r0 = k0 + nb;
-        u.tiles = rb * (rb + 1);
-        u.work = u.tiles * nd;
-        oz_kernel<1><<<std::min(u.work, std::max(c->num_sms, 1)), OZ_T, OZ_SMEM, c->stream>>>(u);
-        launches++;
-      }
+      if (k0) ztm_join(c);  // the update by the last panel
+      if (rows <= 1) continue;
+      u.dig = dset;
+      u.exps = eset;
+      u.n = rows;
+      u.r0 = k0 + nb;
+      u.part = OZ_NEXT;
+      u.tiles = rb;
+      u.work = rb * nd;
+      oz_kernel<1><<<std::min(u.work, std::max(c->num_sms, 1)), OZ_T, OZ_SMEM, c->stream>>>(u);
+      launches++;
+      ztm_fork(c);
+      if (rows <= OZ_N) continue;
+      u.part = OZ_REST;
+      u.tiles = rb * rb;
+      u.work = u.tiles * nd;
+      oz_kernel<1><<<std::min(u.work, rest_grid), OZ_T, OZ_SMEM, c->aux>>>(u);
+      launches++;
     }
     for (int b0 = ((ncols - 1) / LM_NB) * LM_NB; b0 >= 0; b0 -= LM_NB) {
       lm_backstep<<<dim3(std::max(1, b0 / 64), nd), BK_T, 0, c->stream>>>(
