@@ -43,7 +43,7 @@ constexpr int IF_NEAR_WPB = 4;
 // took 1.75 ms at 8 (under one wave), 1.6 at 24, 1.55 at 48
 constexpr int IF_FWD_PER_SM = 48;
 constexpr int IF_SUB = 32;       // columns per second-order test in the forward
-constexpr float IF_FAR = 1.0e6f; // -index of a padding column, height of a padding station
+constexpr float IF_FAR = 1.0e6f; // -index of a padding column (far away)
 constexpr int IF_ROWS = 3;       // rows of the adjoint's table of Y terms
 // the forward's tile load: each warp loads whole blocks of IF_SUB columns
 static_assert(IF_SUB == 32 && IF_TILE % IF_TS == 0 && IF_TS % 32 == 0, "tile load layout");
@@ -459,35 +459,41 @@ struct IfMisfit {
   double* r;
   IStation* sf;      // null: no float copy
   double* misfit;
-  double* part;      // [blocks] sums of r^2
-  unsigned* ticket;  // zeroed before: the block that takes the last one adds the parts
+  unsigned* ticket;  // zeroed before: the block that takes the last one adds up
 };
 
 // gz[s] = G5 * (far_scale * sum_c partial[c][s] + near[s]): 32 stations per
-// block, FIN_Y threads each over the chunks, summed in a fixed order (a thread
-// per station over all chunks is one chain of dependent loads: 11.5 us at 64
-// chunks, 5 now).  MISFIT: the residual and the misfit too (a kernel of one block
-// for them took 9 us for 4,096 stations and 17 us for 16,384).
-constexpr int FIN_Y = 16;
+// block, whose threads fetch FIN_C chunks at a time for one of them to add in
+// order (a thread per station over all chunks waited for every load: 11.5 us at
+// 64 chunks, 6 now).  MISFIT: the residual, and by the last block the misfit, in
+// the order of IF_SUMS strided sums and a tree over them (as a kernel of its own
+// 9 us for 4,096 stations and 17 us for 16,384).  The orders are fixed: an
+// inversion's iterations can turn a last bit of a sum into 1e-8 of its result.
+constexpr int FIN_Y = 16, FIN_C = 64, IF_SUMS = 1024;
 template <bool MISFIT>
 __global__ void __launch_bounds__(32 * FIN_Y)
     iface_finalize(int ns, int nchunks, const double* __restrict__ partial, double far_scale,
                    const double* __restrict__ near, double G5, double* __restrict__ gz,
                    IfMisfit mf) {
-  __shared__ double sm[FIN_Y][33];
+  __shared__ double sm[FIN_C * 32];
   __shared__ bool last;
+  static_assert(IF_SUMS <= FIN_C * 32, "the misfit's sums fit");
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const int s = blockIdx.x * 32 + x;
   double f = 0.0;
-  if (s < ns) {
-#pragma unroll 4
-    for (int c = y; c < nchunks; c += FIN_Y) f += partial[(size_t)c * ns + s];
+  for (int c0 = 0; c0 < nchunks; c0 += FIN_C) {
+    const int cnt = min(FIN_C, nchunks - c0);
+    if (s < ns) {
+#pragma unroll
+      for (int c = y; c < FIN_C; c += FIN_Y)
+        if (c < cnt) sm[c * 32 + x] = partial[(size_t)(c0 + c) * ns + s];
+    }
+    __syncthreads();
+    if (y == 0 && s < ns)
+      for (int c = 0; c < cnt; c++) f += sm[c * 32 + x];
+    __syncthreads();
   }
-  sm[y][x] = f;
-  __syncthreads();
   if (y == 0) {
-    for (int q = 1; q < FIN_Y; q++) f += sm[q][x];
-    double r2 = 0.0;
     if (s < ns) {
       double g = far_scale * f;
       if (near) g += near[s];
@@ -497,30 +503,32 @@ __global__ void __launch_bounds__(32 * FIN_Y)
         const double r = v - mf.data[s];
         mf.r[s] = r;
         if (mf.sf) mf.sf[s].r = (float)r;
-        r2 = r * r;
       }
     }
     if (MISFIT) {
-      r2 = warp_sum_d(r2);
-      if (x == 0) {
-        mf.part[blockIdx.x] = r2;
-        __threadfence();
-        last = atomicAdd(mf.ticket, 1u) == gridDim.x - 1;
-      }
+      __threadfence();
+      __syncwarp();
+      if (x == 0) last = atomicAdd(mf.ticket, 1u) == gridDim.x - 1;
     }
   }
   if (!MISFIT) return;
   __syncthreads();
   if (!last) return;
   __threadfence();
-  double a = 0.0;
-  for (unsigned q = threadIdx.x; q < gridDim.x; q += 32 * FIN_Y) a += __ldcg(mf.part + q);
-  a = warp_sum_d(a);
-  if (x == 0) sm[y][0] = a;
+  for (int q = threadIdx.x; q < IF_SUMS; q += 32 * FIN_Y) {
+    double a = 0.0;
+    for (int i = q; i < ns; i += IF_SUMS) {
+      const double v = __ldcg(mf.r + i);
+      a += v * v;
+    }
+    sm[q] = a;
+  }
   __syncthreads();
-  if (threadIdx.x) return;
-  for (int q = 1; q < FIN_Y; q++) a += sm[q][0];
-  *mf.misfit = 0.5 * a;
+  for (int o = IF_SUMS / 2; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *mf.misfit = 0.5 * sm[0];
 }
 
 // ---- forward, plain double --------------------------------------------------
@@ -554,7 +562,7 @@ __global__ void __launch_bounds__(64)
 // are formed once per row and block, in shared memory (with fewer columns in x a
 // block has too many rows for that to pay, and each pair forms them).  Bound by
 // the FMA pipe, as the forward: 128x128 columns, 64x64 stations 155 -> 124 us;
-// with 256x256 columns and 128x128 stations both directions 3.47 -> 2.82 ms.
+// with 256x256 columns and 128x128 stations both directions 3.47 -> 2.81 ms.
 // RHO: the density gradient too (without it, as in an inversion for the depths, a
 // pair is its face term alone: 124 -> 70 us at 128x128 columns, 64x64 stations).
 template <bool ROWS, bool RHO>
@@ -590,9 +598,7 @@ __global__ void __launch_bounds__(IF_TS, 5)
     int nf = 0;
     for (int q = threadIdx.x; q < IF_TILE + 2; q += IF_TS) {
       const bool ok = t0 + q < s1;
-      // a padding station has no residual and lies far above: its terms are
-      // finite and add zero
-      IStation z = {0.f, 0.f, IF_FAR, 0.f};
+      IStation z = {0.f, 0.f, 0.f, 0.f};
       const IStation f = ok ? sf[t0 + q] : z;
       const int2 h = ok ? si[t0 + q] : make_int2(0, 0);
       s_ex[q] = f.ex;
@@ -619,9 +625,9 @@ __global__ void __launch_bounds__(IF_TS, 5)
     if (!active) continue;
     const int cnt = min(IF_TILE, s1 - t0);
     float2 gr = make_float2(0.f, 0.f), gd = make_float2(0.f, 0.f);  // 32 stations, Kahan across
-#pragma unroll 4
-    for (int q = 0; q < cnt; q += 2) {
-      // stations q and q+1 (past the end of the tile: a padding station)
+    // stations q and q+1 (TAIL: the second is a padding station, dropped)
+    auto pair = [&](int q, auto tail) {
+      constexpr bool TAIL = decltype(tail)::value;
       const float2 hx = *reinterpret_cast<const float2*>(s_hx + q);
       const float2 X = __ffma2_rn(__fadd2_rn(hx, nix2), dxn2,
                                   *reinterpret_cast<const float2*>(s_ex + q));
@@ -658,8 +664,9 @@ __global__ void __launch_bounds__(IF_TS, 5)
       if (tile_near && (s_nf[q] | s_nf[q + 1])) {
         const int2 ha = s_i[q], hb = s_i[q + 1];
         if (is_near(mask, t0 + q, ha.x, ha.y, ix, iy, k)) vr.x = vd.x = 0.f;
-        if (q + 1 < cnt && is_near(mask, t0 + q + 1, hb.x, hb.y, ix, iy, k)) vr.y = vd.y = 0.f;
+        if (!TAIL && is_near(mask, t0 + q + 1, hb.x, hb.y, ix, iy, k)) vr.y = vd.y = 0.f;
       }
+      if (TAIL) vr.y = vd.y = 0.f;
       gr = __fadd2_rn(gr, vr);
       gd = __fadd2_rn(gd, vd);
       if ((q & 30) == 30) {
@@ -667,7 +674,10 @@ __global__ void __launch_bounds__(IF_TS, 5)
         ad.add(gd.x + gd.y);
         gr = gd = make_float2(0.f, 0.f);
       }
-    }
+    };
+#pragma unroll 4
+    for (int q = 0; q + 1 < cnt; q += 2) pair(q, std::false_type{});
+    if (cnt & 1) pair(cnt - 1, std::true_type{});
     ar.add(gr.x + gr.y);
     ad.add(gd.x + gd.y);
   }
@@ -1036,7 +1046,7 @@ extern "C" int ztm_gfm_interface_misfit(ztm_ctx* c, const ztm_imesh* mesh, const
     }
   } restore{prev, c->device};
   size_t need = 2 * WsCarver::need(nc * 8) + WsCarver::need((size_t)ns * 24) +
-                5 * WsCarver::need((size_t)ns * 8) + 2 * WsCarver::need(nc * 8) + 512 +
+                4 * WsCarver::need((size_t)ns * 8) + 2 * WsCarver::need(nc * 8) + 512 +
                 ztm_iface_ws(m, ns, prec, c->num_sms) + 4096;
   int rc = ztm_ws_reserve(c, need);
   if (rc) return rc;
@@ -1048,7 +1058,6 @@ extern "C" int ztm_gfm_interface_misfit(ztm_ctx* c, const ztm_imesh* mesh, const
   double* s_gz = wc.take<double>(ns);
   double* s_r = wc.take<double>(ns);
   double* s_mis = wc.take<double>(1);
-  double* s_part = wc.take<double>((ns + 31) / 32);
   unsigned* s_ticket = wc.take<unsigned>(1);
   double* s_gr = wc.take<double>(nc);
   double* s_gd = wc.take<double>(nc);
@@ -1060,7 +1069,7 @@ extern "C" int ztm_gfm_interface_misfit(ztm_ctx* c, const ztm_imesh* mesh, const
   double* ogz = (dev && gz) ? gz : s_gz;
   // the residual and misfit come out of the forward's last kernel; the mixed
   // adjoint takes over what the forward prepared
-  IfMisfit mf{(const double*)pdat, s_r, nullptr, dev ? misfit : s_mis, s_part, s_ticket};
+  IfMisfit mf{(const double*)pdat, s_r, nullptr, dev ? misfit : s_mis, s_ticket};
   IfPrep prep;
   rc = iface_forward_impl<false>(c, m, (const double*)pd, (const double*)pr, nullptr, ns,
                                  (const double*)px, ogz, G, prec, o, wc, &mf, &prep);
@@ -1172,8 +1181,7 @@ int ztm_iface_host_begin(ztm_ctx* c, const ztm_imesh* mesh, const double* rho, i
   return ztm_cuda_check(c, cudaGetLastError(), "copy the inversion's arrays to the device");
 }
 
-int ztm_iface_host_misfit(ztm_ctx* c, const ztm_imesh* mesh, int ns, const ztm_opts* o,
-                          double* misfit) {
+int ztm_iface_host_start(ztm_ctx* c, const ztm_imesh* mesh, int ns, const ztm_opts* o) {
   const long long nc = (long long)mesh->nx * mesh->ny;
   OnDevice guard(c->device);
   const HostDevice d(c->inv, nc, ns);
@@ -1181,9 +1189,15 @@ int ztm_iface_host_misfit(ztm_ctx* c, const ztm_imesh* mesh, int ns, const ztm_o
   ztm_opts od = *o;
   od.flags |= ZTM_FLAG_DEVICE_PTRS;
   cudaMemcpyAsync(d.depth, h.depth, nc * 8, cudaMemcpyHostToDevice, c->stream);
-  int rc = ztm_gfm_interface_misfit(c, mesh, d.depth, d.rho, ns, d.xyz, d.data, d.mis, nullptr,
-                                    nullptr, d.g, &od);
-  if (rc || (rc = host_result(c, d, h, nc))) return rc;
+  return ztm_gfm_interface_misfit(c, mesh, d.depth, d.rho, ns, d.xyz, d.data, d.mis, nullptr,
+                                  nullptr, d.g, &od);
+}
+
+int ztm_iface_host_wait(ztm_ctx* c, const ztm_imesh* mesh, int ns, double* misfit) {
+  const long long nc = (long long)mesh->nx * mesh->ny;
+  OnDevice guard(c->device);
+  const IfaceHost h = host_arrays(c, nc);
+  if (int rc = host_result(c, HostDevice(c->inv, nc, ns), h, nc)) return rc;
   *misfit = h.g[nc];
   return ZTM_OK;
 }

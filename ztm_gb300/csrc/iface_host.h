@@ -16,8 +16,8 @@ struct IfaceHost {  // host arrays of one entry per column, owned by the context
 // begin on this context).
 int ztm_iface_host_begin(ztm_ctx* c, const ztm_imesh* mesh, const double* rho, int ns,
                          const double* sxyz, const double* data, IfaceHost* h);
-// Misfit of `depth`, its depth gradient in `g`.
-int ztm_iface_host_misfit(ztm_ctx* c, const ztm_imesh* mesh, int ns, const ztm_opts* o,
-                          double* misfit);
+// Misfit of `depth` and its depth gradient: started, and waited for (in `g`).
+int ztm_iface_host_start(ztm_ctx* c, const ztm_imesh* mesh, int ns, const ztm_opts* o);
+int ztm_iface_host_wait(ztm_ctx* c, const ztm_imesh* mesh, int ns, double* misfit);
 // J^T J `v` at `depth` in `g`, J the depth derivative of the forward.
 int ztm_iface_host_product(ztm_ctx* c, const ztm_imesh* mesh, int ns, const ztm_opts* o);

@@ -37,48 +37,23 @@ struct Problem {
   IfaceHost io;
 };
 
-// Sums in eight partial sums (a chain of dependent adds over 128 x 128 columns
-// took 20 us, a dozen times an iteration).
-constexpr size_t LANES = 8;
-double total(const double* s) {
-  return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
-}
+// Sums run in index order: the iterations can turn a last bit into 1e-8 of the
+// result, and runs are to repeat those of earlier versions.
 double dot(const double* a, const double* b, size_t n) {
-  double s[LANES] = {};
-  size_t i = 0;
-  for (; i + LANES <= n; i += LANES)
-    for (size_t j = 0; j < LANES; j++) s[j] += a[i + j] * b[i + j];
-  for (size_t j = 0; i < n; i++, j++) s[j] += a[i] * b[i];
-  return total(s);
+  double s = 0.0;
+  for (size_t i = 0; i < n; i++) s += a[i] * b[i];
+  return s;
 }
-// sum of (a - b)^2
-double dist2(const double* a, const double* b, size_t n) {
-  double s[LANES] = {};
-  size_t i = 0;
-  for (; i + LANES <= n; i += LANES)
-    for (size_t j = 0; j < LANES; j++) {
-      const double d = a[i + j] - b[i + j];
-      s[j] += d * d;
-    }
-  for (size_t j = 0; i < n; i++, j++) s[j] += (a[i] - b[i]) * (a[i] - b[i]);
-  return total(s);
-}
-// d = (d - a y) scale, and the new d . z
+// d = (d - a y) scale, and the new d . z (the sum's chain of adds hides the rest)
 double step_dot(size_t n, double* __restrict d, double a, const double* __restrict y, double scale,
                 const double* __restrict z) {
-  double s[LANES] = {};
-  size_t i = 0;
-  for (; i + LANES <= n; i += LANES)
-    for (size_t j = 0; j < LANES; j++) {
-      const double v = (d[i + j] - a * y[i + j]) * scale;
-      d[i + j] = v;
-      s[j] += v * z[i + j];
-    }
-  for (size_t j = 0; i < n; i++, j++) {
-    d[i] = (d[i] - a * y[i]) * scale;
-    s[j] += d[i] * z[i];
+  double s = 0.0;
+  for (size_t i = 0; i < n; i++) {
+    const double v = (d[i] - a * y[i]) * scale;
+    d[i] = v;
+    s += v * z[i];
   }
-  return total(s);
+  return s;
 }
 double dot(const std::vector<double>& a, const std::vector<double>& b) {
   return dot(a.data(), b.data(), a.size());
@@ -109,15 +84,21 @@ int evaluate(Problem& P, const std::vector<double>& m, double* f, std::vector<do
              double* data_misfit) {
   const size_t nc = m.size();
   for (size_t c = 0; c < nc; c++) P.io.depth[c] = 1000.0 * m[c];
-  double mis = 0.0;
-  if (int rc = ztm_iface_host_misfit(P.ctx, P.mesh, P.ns, &P.opts, &mis)) return rc;
-  add_smoothing(P, m.data(), P.io.g, g.data());  // d/dm (km) = 1000 d/ddepth (m)
+  if (int rc = ztm_iface_host_start(P.ctx, P.mesh, P.ns, &P.opts)) return rc;
+  // the smoothing term meanwhile
   double reg = 0.0;
   for (int iy = 0; iy < P.ny; iy++) {
     const double* r = m.data() + (size_t)P.nx * iy;
-    reg += dist2(r, r + 1, P.nx - 1);
-    if (iy + 1 < P.ny) reg += dist2(r, r + P.nx, P.nx);
+    const double* q = r + P.nx;
+    const bool down = iy + 1 < P.ny;
+    for (int ix = 0; ix < P.nx; ix++) {
+      if (ix + 1 < P.nx) reg += (r[ix] - r[ix + 1]) * (r[ix] - r[ix + 1]);
+      if (down) reg += (r[ix] - q[ix]) * (r[ix] - q[ix]);
+    }
   }
+  double mis = 0.0;
+  if (int rc = ztm_iface_host_wait(P.ctx, P.mesh, P.ns, &mis)) return rc;
+  add_smoothing(P, m.data(), P.io.g, g.data());  // d/dm (km) = 1000 d/ddepth (m)
   *f = mis + 0.5 * P.lambda * reg;
   if (data_misfit) *data_misfit = mis;
   return ZTM_OK;
@@ -169,7 +150,7 @@ extern "C" int ztm_invert_interface(ztm_ctx* ctx, const ztm_imesh* mesh, double*
   // steps and gradient changes: S[p], Y[p] for p = kept.front() .. kept.back()
   std::vector<std::vector<double>> S(H), Y(H);
   std::vector<int> kept;
-  double rhoh[H], alpha[H], yy[H];
+  double rhoh[H], alpha[H], sy[H], yy[H];
   std::vector<double> spare_s, spare_y;
   int it = 0;
   for (; it < iterations; it++) {
@@ -179,7 +160,7 @@ extern "C" int ztm_invert_interface(ztm_ctx* ctx, const ztm_imesh* mesh, double*
     const int n = (int)kept.size();
     if (n) {
       d = g;
-      const double gamma = 1.0 / (rhoh[kept[n - 1]] * yy[kept[n - 1]]);
+      const double gamma = sy[kept[n - 1]] / yy[kept[n - 1]];
       double sd = dot(S[kept[n - 1]], d);
       for (int k = n - 1; k >= 0; k--) {
         const int q = kept[k];
@@ -228,12 +209,17 @@ extern "C" int ztm_invert_interface(ztm_ctx* ctx, const ztm_imesh* mesh, double*
     double *s = spare_s.data(), *y = spare_y.data();
     for (size_t i = 0; i < nc; i++) s[i] = mt[i] - m[i];
     for (size_t i = 0; i < nc; i++) y[i] = gt[i] - g[i];
-    const double sy = dot(s, y, nc);
-    const double ss = dot(s, s, nc), y2 = dot(y, y, nc);
-    if (sy > 1e-12 * sqrt(ss * y2)) {
+    double s_y = 0.0, ss = 0.0, y2 = 0.0;
+    for (size_t i = 0; i < nc; i++) {
+      s_y += s[i] * y[i];
+      ss += s[i] * s[i];
+      y2 += y[i] * y[i];
+    }
+    if (s_y > 1e-12 * sqrt(ss * y2)) {
       S[p].swap(spare_s);
       Y[p].swap(spare_y);
-      rhoh[p] = 1.0 / sy;
+      rhoh[p] = 1.0 / s_y;
+      sy[p] = s_y;
       yy[p] = y2;
       if (kept.size() == (size_t)H) kept.erase(kept.begin());
       kept.push_back(p);
