@@ -404,7 +404,7 @@ def extras(ctx, mesh, rho, st, d_rho, d_st, gz_mixed, fwd_ms):
     out["forward_plus_adjoint_vs_plain_fp64"] = {
         "mixed_s": tmx, "fp64_s_at_measured_rates": t64, "speedup": t64 / tmx,
         "what": "mixed forward (the timed step) + mixed adjoint against the plain double forward "
-                "+ adjoint of the same pairs at their measured rates (vertex-shared double kernels)"}
+                "+ adjoint of the same pairs at their measured rates (double kernels)"}
     # the reference's own point-mass model on the same geometry (its grid,
     # every node as a station): our float and double gathers and adjoints
     g, drho, surf = synth.pointmass_grid_of_mesh(mesh, rho, st)
@@ -678,7 +678,7 @@ def run_workload(args, local_rank):
         sub = st[np.arange(0, len(st), len(st) // 64)[:64]]
         dr, ds = d(rho), d(sub)
         units = mesh.nx * mesh.ny * mesh.nz * len(sub)
-        what = ("plain double prism forward (vertex-shared) of the 256x256x64 draped mesh at 64 of "
+        what = ("double prism forward of the 256x256x64 draped mesh at 64 of "
                 "its stations")
         step = lambda: ctx.prism(mesh, dr, ds, precision="fp64")
     elif args.workload in ("pointmass_small", "pointmass64_small", "pointmass_adjoint_small",
@@ -708,10 +708,10 @@ def run_workload(args, local_rank):
         dsig = d(rng.uniform(0.05, 2.0, ncols))
         dm = d(np.array([[0.0, 0.0], [1e-3, 1e-4], [0.1, 1e-2], [1.0, 1.0]]))
         # units: the multiply-adds of J^T J (full) and of a Gauss-Jordan inversion
-        # per pair (the reference's work); the library factorises by blocked LU
+        # per pair (the reference's work); the library factorises by Cholesky
         units = nrows * ncols * ncols + nd * ncols ** 3
         what = ("damped Gauss-Newton trials (TFM.cpp:159-160): J 12000 x 2700, 4 damping pairs "
-                "(J^T J + 4 solves by blocked LU; units: the multiply-adds of J^T J and of the "
+                "(J^T J + 4 solves; units: the multiply-adds of J^T J and of the "
                 "reference's Gauss-Jordan inversions)")
         step = lambda: ctx.lm_steps(dJ, dr_, db, dsig, dm)
     elif args.workload == "inversion":

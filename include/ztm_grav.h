@@ -42,7 +42,11 @@ enum {
 
 /* ---- precision / method ----------------------------------------------- */
 enum {
-  ZTM_PREC_FP64 = 0,  /* plain: every pair in double (closed form / pow) */
+  ZTM_PREC_FP64 = 0,  /* double accuracy for every pair: prisms near a
+                         station by the closed form, the others by a
+                         twelfth-order expansion in pairs of floats
+                         (closer to the exact field than the closed form
+                         there); point masses in double */
   ZTM_PREC_FP32 = 1,  /* every pair in float with compensated sums */
   ZTM_PREC_MIXED = 2  /* prism modes: far pairs in float (moment expansion
                          to sixth order on 3-D meshes, horizontal expansion
