@@ -29,3 +29,20 @@ def test_bits_of_the_persistent_kernel(nx, ny, nz, ns, precision):
         b.count_forms(True)
         assert np.array_equal(a.prism(mesh, rho, st, precision=precision),
                               b.prism(mesh, rho, st, precision=precision))
+
+
+@pytest.mark.parametrize("ns", [1, 2, 33, 511, 512, 513])
+def test_station_order_by_counting(ctx, ns):
+    """Up to 512 stations are ordered by counting, more by the library's sort:
+    stations that share cells, lie outside the mesh or twice in the list.
+    TOLERANCE: 1e-6 of the largest value against double, that of the mixed
+    method."""
+    rng = np.random.default_rng(ns)
+    mesh = ztm_gb300.make_mesh(23, 31, 12, 900.0, 1100.0, 500.0, z_top=50.0)
+    rho = rng.normal(0.0, 300.0, 23 * 31 * 12)
+    st = np.stack([rng.uniform(-0.5, 1.5, ns) * 23 * 900.0, rng.uniform(-0.5, 1.5, ns) * 31 * 1100.0,
+                   rng.uniform(60.0, 3000.0, ns)], axis=1)
+    st[ns // 2:][: ns // 4] = st[: ns // 4]
+    a = ctx.prism(mesh, rho, st, precision="mixed")
+    b = ctx.prism(mesh, rho, st, precision="fp64")
+    assert np.max(np.abs(a - b)) <= 1e-6 * np.max(np.abs(b))

@@ -18,25 +18,12 @@
 
 namespace {
 
-__device__ __forceinline__ uint32_t spread16(uint32_t v) {
-  v &= 0xffffu;
-  v = (v | (v << 8)) & 0x00ff00ffu;
-  v = (v | (v << 4)) & 0x0f0f0f0fu;
-  v = (v | (v << 2)) & 0x33333333u;
-  v = (v | (v << 1)) & 0x55555555u;
-  return v;
-}
-
-// key = interleaved bits of the home cell (x, y), clamped to 16 bits each
-// (si: the home cell's x, y as the first two of `stride` ints per station;
-// cells outside the mesh sort with the nearest edge cell)
+// si: the home cell's x, y as the first two of `stride` ints per station
 __global__ void station_key_kernel(int ns, const int* __restrict__ si, int stride, int nx, int ny,
                                    uint32_t* __restrict__ key, int* __restrict__ idx) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= ns) return;
-  const uint32_t x = (uint32_t)min(max(si[(size_t)s * stride], 0), nx - 1);
-  const uint32_t y = (uint32_t)min(max(si[(size_t)s * stride + 1], 0), ny - 1);
-  key[s] = spread16(x) | (spread16(y) << 1);
+  key[s] = ztm_station_key(si[(size_t)s * stride], si[(size_t)s * stride + 1], nx, ny);
   idx[s] = s;
 }
 

@@ -269,6 +269,21 @@ __device__ __forceinline__ double ztm_face_unit(double xa, double xb,
 }
 
 // Compensated (Kahan) accumulation in float.  The true sum is s - c.
+// Z-order key of a station's home cell: interleaved bits of (x, y), clamped to
+// 16 bits each (cells outside the mesh sort with the nearest edge cell).
+__device__ __forceinline__ uint32_t ztm_spread16(uint32_t v) {
+  v &= 0xffffu;
+  v = (v | (v << 8)) & 0x00ff00ffu;
+  v = (v | (v << 4)) & 0x0f0f0f0fu;
+  v = (v | (v << 2)) & 0x33333333u;
+  v = (v | (v << 1)) & 0x55555555u;
+  return v;
+}
+__device__ __forceinline__ uint32_t ztm_station_key(int x, int y, int nx, int ny) {
+  return ztm_spread16((uint32_t)min(max(x, 0), nx - 1)) |
+         (ztm_spread16((uint32_t)min(max(y, 0), ny - 1)) << 1);
+}
+
 struct Kahan {
   float s = 0.f, c = 0.f;
   __device__ __forceinline__ void add(float x) {
