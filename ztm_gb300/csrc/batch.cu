@@ -333,7 +333,7 @@ __device__ bool far_item_cc(const BJob& J, int tile, int chunk, int mg, uint64_t
     const int ncol = min(J.sc, c1 - cs);
     if (one) {  // every lane (inactive ones on dummy data) for the warp votes
       unsigned cnt[3];
-      meshfar::far_stage<false>(J.iv, k, fc, t, s, Lm, rs, cs, ncol, acc1, cnt);
+      meshfar::far_stage<false, false, false>(J.iv, k, fc, t, s, Lm, rs, cs, ncol, acc1, cnt);
     } else if constexpr (MG > 1) {
       if (active) {
         int ix = cs % k.nx, iy = cs / k.nx;

@@ -57,7 +57,10 @@ __device__ __forceinline__ float2 far_group(const float* col, int l0, float fl,
 // All layers of one column: groups [0, lmask) with the near mask, full
 // groups up to nz8 without, a masked tail group if nz is not a multiple of 8.
 // Plain float sums over 32 layers (two lanes of 16), compensated across.
-template <bool T2, class ACC>
+// BIG: 64 layers unrolled, here and in the pairs (the forward's kernel, 256x256x64
+// prisms, 128x128 stations: 21.0 ms against 21.4); the batch, whose kernel is
+// larger than the instruction cache, takes the small loops (96.2 -> 95.4 ms).
+template <bool T2, bool BIG, class ACC>
 __device__ __forceinline__ void far_column(const float* col, int lmask, int nz8, int nz,
                                            const float2 (&Zb)[4], float2 zstep,
                                            const ColPoly2& cp2, float2 c2t, int elo,
@@ -82,7 +85,7 @@ __device__ __forceinline__ void far_column(const float* col, int lmask, int nz8,
       g = make_float2(0.f, 0.f);
     }
   }
-  for (; l0 + 64 <= nz8; l0 += 64, fl += 64.f) {
+  for (; BIG && l0 + 64 <= nz8; l0 += 64, fl += 64.f) {
     g = far_group<T2, false>(col, l0, fl, Zb, zstep, cp2, c2t, elo, espan, nz, g);
     g = far_group<T2, false>(col, l0 + 8, fl + 8.f, Zb, zstep, cp2, c2t, elo, espan, nz, g);
     g = far_group<T2, false>(col, l0 + 16, fl + 16.f, Zb, zstep, cp2, c2t, elo, espan, nz, g);
@@ -146,7 +149,7 @@ __device__ __forceinline__ float2 far_group_pair(const float* colA, const float*
 // Layers 0 .. nl - 1 of two columns (nl a multiple of 8: nz, or the padded
 // nzp where the padding layers' K is finite): plain float sums over 16
 // layers of both (32 terms), compensated across.
-template <class ACC>
+template <bool BIG, class ACC>
 __device__ __forceinline__ void far_column_pair(const float* colA, const float* colB, int nl,
                                                 const float2 (&Zb)[4], float2 zstep,
                                                 const ColPoly2& cpA, float2 c2tA,
@@ -155,7 +158,7 @@ __device__ __forceinline__ void far_column_pair(const float* colA, const float* 
   float fl = 0.f;
   const float2 z0 = make_float2(0.f, 0.f);
   for (; l0 + 64 <= nl; l0 += 64, fl += 64.f) {
-#pragma unroll
+#pragma unroll(BIG ? 4 : 1)
     for (int h = 0; h < 4; h++) {
       float2 g = far_group_pair(colA, colB, l0 + 16 * h, fl + 16.f * h, Zb, zstep, cpA, c2tA,
                                 cpB, c2tB, z0);
@@ -183,7 +186,7 @@ __device__ __forceinline__ void far_column_pair(const float* colA, const float* 
 // PART: only the columns and column pairs that start in [qa, qb) are evaluated;
 // which columns form pairs is found from the stage's first column on, so that the
 // parts together make the same sequence of acc.add.
-template <bool COUNT, bool PART = false, class ACC = Kahan>
+template <bool COUNT, bool PART = false, bool BIG = true, class ACC = Kahan>
 __device__ __forceinline__ void far_stage(const short2* __restrict__ ivs, const MeshConst& k,
                                           const FarCoef& fc, const FarStation& t, int s, int Lm,
                                           const float* rs, int cs, int ncol, ACC& acc,
@@ -239,7 +242,7 @@ __device__ __forceinline__ void far_stage(const short2* __restrict__ ivs, const 
         cpA.a1 = cpB.a1 = make_float2(fc.a1, fc.a1);
         cpA.C2 = cpA.C3 = cpA.C4 = cpA.C5 = cpA.C6 = make_float2(0.f, 0.f);
         cpB.C2 = cpB.C3 = cpB.C4 = cpB.C5 = cpB.C6 = make_float2(0.f, 0.f);
-        far_column_pair(rs + q * k.nzp, rs + (q + 1) * k.nzp, k.nzp, Zb, zstep, cpA,
+        far_column_pair<BIG>(rs + q * k.nzp, rs + (q + 1) * k.nzp, k.nzp, Zb, zstep, cpA,
                         make_float2(cA, cA), cpB, make_float2(cB, cB), acc);
         if (COUNT) cnt[2] += 2 * k.nzp;
         q++;
@@ -284,12 +287,12 @@ __device__ __forceinline__ void far_stage(const short2* __restrict__ ivs, const 
       cp2.rh = make_float2(rh, rh);
       cp2.a1 = make_float2(fc.a1, fc.a1);
       cp2.C2 = cp2.C3 = cp2.C4 = cp2.C5 = cp2.C6 = make_float2(0.f, 0.f);  // unused by the form
-      far_column<true>(col, lmask, nz8, k.nz, Zb, zstep, cp2, make_float2(c2t, c2t), elo, espan,
+      far_column<true, BIG>(col, lmask, nz8, k.nz, Zb, zstep, cp2, make_float2(c2t, c2t), elo, espan,
                        acc);
       if (COUNT) cnt[1] += k.nzp;
     } else {
       const ColPoly2 cp2 = col_poly2(col_poly(X, Y, fc), fc.a1);
-      far_column<false>(col, lmask, nz8, k.nz, Zb, zstep, cp2, make_float2(0.f, 0.f), elo, espan,
+      far_column<false, BIG>(col, lmask, nz8, k.nz, Zb, zstep, cp2, make_float2(0.f, 0.f), elo, espan,
                         acc);
       if (COUNT) cnt[0] += k.nzp;
     }
